@@ -4,8 +4,8 @@
 //   host    per-instance element builds (the reference's geometry arithmetic, lib/element.cpp and
 //           the GeometryDataST constructors, exactly as the single-scene path does it), in
 //           parallel threads, written into one pinned staging image of the device arena
-//   device  one CUDA graph: upload the image, zero the flux maps and counters, refit every
-//           instance's BVH (refit_kernel), compute every instance's sun plane
+//   device  one CUDA graph: upload the image, zero the flux maps and counters, refit the BVH of
+//           the instances that traverse one (refit_kernel), compute every instance's sun plane
 //           (prepare_sun_batch_kernel) and sun-ray candidate grid (csp_sungrid.cu), trace the
 //           small-scene, BVH and grid instances (one persistent batch_kernel launch per group),
 //           copy flux maps, counters and sun frames back
@@ -288,9 +288,10 @@ int Batch::layout(int si) {
     const size_t n = inst.size();
     place.assign(n, Place{});
     for (int g = 0; g < kBatchGroups; ++g) n_group[g] = 0;
+    n_refit = 0;
     max_nodes = 0;
     n_sg = 0;
-    max_sg_n = 0;
+    max_n = 0;
     size_t off = 0;
     for (size_t i = 0; i < n; ++i) {
         const BScene& s = scenes[inst[i].scene];
@@ -315,11 +316,14 @@ int Batch::layout(int si) {
             p.global = off;
             off += align16(std::max<size_t>(1, hg.global.size()) * sizeof(Aabb));
         }
-        max_nodes = std::max(max_nodes, (int)s.base.nodes.size());
+        if (p.group != kAccelGrid) {
+            p.rf_slot = n_refit++;
+            max_nodes = std::max(max_nodes, (int)s.base.nodes.size());
+        }
         if (p.group != kAccelFlat) {
             p.sg_slot = n_sg++;
-            max_sg_n = std::max(max_sg_n, (int)ne);
         }
+        max_n = std::max(max_n, (int)ne);
     }
     for (int g = 0; g < kBatchGroups; ++g) {
         desc_off[g] = off;
@@ -330,15 +334,17 @@ int Batch::layout(int si) {
         off += align16((n_group[g] + 1) * sizeof(uint64_t));
     }
     refit_off = off;
-    off += align16(n * sizeof(RefitJob));
+    off += align16((size_t)n_refit * sizeof(RefitJob));
     sunjob_off = off;
     off += align16(n * sizeof(SunJob));
     sgjob_off = off;
     off += align16((size_t)n_sg * sizeof(SunGridJob));
     up_bytes = off;
     for (size_t i = 0; i < n; ++i) {
-        place[i].nodes = off;
-        off += align16(scenes[inst[i].scene].base.nodes.size() * sizeof(Node));
+        if (place[i].rf_slot >= 0) {
+            place[i].nodes = off;
+            off += align16(scenes[inst[i].scene].base.nodes.size() * sizeof(Node));
+        }
         if (place[i].sg_slot >= 0) {
             place[i].sgrid = off;
             off += align16(sungrid_bytes(count_of(i)));
@@ -462,18 +468,20 @@ void Batch::fill_instance(size_t i) {
         std::memcpy(h_stage + p.items, hg.items.data(), hg.items.size() * sizeof(Aabb));
         if (!hg.global.empty()) std::memcpy(h_stage + p.global, hg.global.data(), hg.global.size() * sizeof(Aabb));
     }
-    RefitJob rj;
-    rj.topo = s.d_topo;
-    rj.aabbs = reinterpret_cast<const Aabb*>(dev(p.aabbs));
-    rj.prune = reinterpret_cast<const Aabb*>(dev(p.prune));
-    rj.out = reinterpret_cast<Node*>(dev(p.nodes));
-    rj.n_nodes = (int)s.base.nodes.size();
-    rj.pad = 0;
-    std::memcpy(h_stage + refit_off + i * sizeof(RefitJob), &rj, sizeof rj);
+    if (p.rf_slot >= 0) {
+        RefitJob rj;
+        rj.topo = s.d_topo;
+        rj.aabbs = reinterpret_cast<const Aabb*>(dev(p.aabbs));
+        rj.prune = reinterpret_cast<const Aabb*>(dev(p.prune));
+        rj.out = reinterpret_cast<Node*>(dev(p.nodes));
+        rj.n_nodes = (int)s.base.nodes.size();
+        rj.pad = 0;
+        std::memcpy(h_stage + refit_off + (size_t)p.rf_slot * sizeof(RefitJob), &rj, sizeof rj);
+    }
     float sv[3];
     sun_vector_f(b.sun, sv);
     SunJob sj;
-    sj.aabbs = rj.aabbs;
+    sj.aabbs = reinterpret_cast<const Aabb*>(dev(p.aabbs));
     sj.n = (int)ne;
     sj.sx = sv[0];
     sj.sy = sv[1];
@@ -487,7 +495,7 @@ void Batch::fill_instance(size_t i) {
         SunGridJob gj;
         sungrid_place(dev(p.sgrid), ne, gj);
         gj.sun = sj.out;
-        gj.aabbs = rj.aabbs;
+        gj.aabbs = sj.aabbs;
         std::memcpy(h_stage + sgjob_off + (size_t)p.sg_slot * sizeof(SunGridJob), &gj, sizeof gj);
     }
 }
@@ -509,7 +517,7 @@ void Batch::fill_descs(const int* block, const std::vector<bool>* sample, std::v
         uint64_t rays = b.rays;
         if (sample && !(*sample)[i]) rays = 0;
         InstanceDesc& d = out_desc[g][p.slot];
-        d.args.nodes = reinterpret_cast<const Node*>(dev(p.nodes));
+        d.args.nodes = p.rf_slot >= 0 ? reinterpret_cast<const Node*>(dev(p.nodes)) : nullptr;
         d.args.prims = reinterpret_cast<const Prim*>(dev(p.prims));
         d.args.optics = reinterpret_cast<const Optics*>(dev(p.optics));
         d.args.sun = reinterpret_cast<const SunFrame*>(dev(p.sun));
@@ -578,15 +586,15 @@ int Batch::enqueue_zero(cudaStream_t st) {
 
 int Batch::enqueue_scene_setup(cudaStream_t st) {
     int rc;
-    if ((rc = cuda_status(launch_refit(reinterpret_cast<const RefitJob*>(dev(refit_off)), (int)inst.size(),
+    if ((rc = cuda_status(launch_refit(reinterpret_cast<const RefitJob*>(dev(refit_off)), n_refit,
                                        max_nodes, st),
                           "refit_kernel")))
         return rc;
     if ((rc = cuda_status(launch_prepare_sun_batch(reinterpret_cast<const SunJob*>(dev(sunjob_off)),
-                                                   (int)inst.size(), st),
+                                                   (int)inst.size(), max_n, st),
                           "prepare_sun_batch_kernel")))
         return rc;
-    return cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(dev(sgjob_off)), n_sg, max_sg_n, st),
+    return cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(dev(sgjob_off)), n_sg, max_n, st),
                        "sun grid build");
 }
 

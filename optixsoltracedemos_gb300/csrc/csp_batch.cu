@@ -17,7 +17,6 @@ namespace csp {
 namespace {
 
 constexpr int kRefitBlock = 256;  // 8 warps, one node per warp
-constexpr int kPrepBlock = 512;
 
 __global__ void __launch_bounds__(kRefitBlock) refit_kernel(const RefitJob* __restrict__ jobs) {
     const RefitJob J = jobs[blockIdx.y];
@@ -70,10 +69,12 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(const RefitJob* __re
     }
 }
 
-__global__ void __launch_bounds__(kPrepBlock) prepare_sun_batch_kernel(const SunJob* __restrict__ jobs) {
-    __shared__ float scratch[kPrepBlock / 32];
-    const SunJob J = jobs[blockIdx.x];
-    sun_frame_block(J.aabbs, J.n, make_float3(J.sx, J.sy, J.sz), J.tan_pad, J.shape, J.param, J.out, scratch);
+template <int kCluster>
+__global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kCluster)
+    prepare_sun_batch_kernel(const SunJob* __restrict__ jobs) {
+    __shared__ StateSmem sm;
+    const SunJob J = jobs[blockIdx.x / kCluster];
+    sun_frame_state<kCluster>(J.aabbs, J.n, make_float3(J.sx, J.sy, J.sz), J.tan_pad, J.shape, J.param, J.out, sm);
 }
 
 template <int kB, int kAccel>
@@ -223,9 +224,13 @@ cudaError_t launch_refit(const RefitJob* jobs, int n_jobs, int max_nodes, cudaSt
     return cudaGetLastError();
 }
 
-cudaError_t launch_prepare_sun_batch(const SunJob* jobs, int n_jobs, cudaStream_t stream) {
+cudaError_t launch_prepare_sun_batch(const SunJob* jobs, int n_jobs, int max_n, cudaStream_t stream) {
     if (n_jobs <= 0) return cudaSuccess;
-    prepare_sun_batch_kernel<<<(unsigned)n_jobs, kPrepBlock, 0, stream>>>(jobs);
+    if (max_n >= kStateClusterMin)
+        prepare_sun_batch_kernel<kStateCluster>
+            <<<(unsigned)n_jobs * kStateCluster, kStateBlock, 0, stream>>>(jobs);
+    else
+        prepare_sun_batch_kernel<1><<<(unsigned)n_jobs, kStateBlock, 0, stream>>>(jobs);
     return cudaGetLastError();
 }
 

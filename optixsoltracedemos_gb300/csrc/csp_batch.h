@@ -47,6 +47,7 @@ struct Place {
     size_t cells = 0, items = 0, global = 0;  // own grid arrays (instances with poses in the grid group)
     size_t sgrid = 0;  // sun-ray candidate grid (BVH and grid groups), built on the device
     int sg_slot = -1;  // index of its build job
+    int rf_slot = -1;  // index of its refit job (grid instances have no nodes)
     int group = 0;  // kAccelFlat, kAccelBvh or kAccelGrid: the kernel that traces the instance
     int slot = 0;   // index within the group
 };
@@ -105,9 +106,9 @@ struct Batch {
     size_t desc_off[kBatchGroups] = {}, tb_off[kBatchGroups] = {}, refit_off = 0, sunjob_off = 0, counter_off = 0;
     size_t sgjob_off = 0;
     int n_group[kBatchGroups] = {};
-    int n_sg = 0, max_sg_n = 0;  // sun grid build jobs and their largest element count
+    int n_sg = 0, max_n = 0;  // sun grid build jobs; largest element count of the instances
     std::vector<InstBuild> builds;  // per instance, during a run (instances with poses)
-    int max_nodes = 0;
+    int n_refit = 0, max_nodes = 0;  // refit jobs and their largest node count
 
     double time_setup = 0.0, time_trace = 0.0;  // of the last completed run
     size_t last_up = 0, last_res = 0;            // its transfer sizes

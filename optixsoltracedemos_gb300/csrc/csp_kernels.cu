@@ -25,14 +25,14 @@ namespace csp {
 namespace {
 
 constexpr int kTraceBlock = 256;
-constexpr int kPrepBlock = 512;
 constexpr int kFluxBlock = 256;
 
-__global__ void __launch_bounds__(kPrepBlock) prepare_sun_kernel(const Aabb* __restrict__ aabbs, int n, float3 s,
-                                                                   float tan_pad, int shape, float param,
-                                                                   SunFrame* __restrict__ out) {
-    __shared__ float scratch[kPrepBlock / 32];
-    sun_frame_block(aabbs, n, s, tan_pad, shape, param, out, scratch);
+template <int kCluster>
+__global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kCluster)
+    prepare_sun_kernel(const Aabb* __restrict__ aabbs, int n, float3 s, float tan_pad, int shape, float param,
+                       SunFrame* __restrict__ out) {
+    __shared__ StateSmem sm;
+    sun_frame_state<kCluster>(aabbs, n, s, tan_pad, shape, param, out, sm);
 }
 
 template <int kAccel>
@@ -278,7 +278,12 @@ const float* halton3_table() {
 
 cudaError_t launch_prepare_sun(const Aabb* aabbs, int n, float sx, float sy, float sz, float tan_pad, int shape,
                                float param, SunFrame* out, cudaStream_t stream) {
-    prepare_sun_kernel<<<1, kPrepBlock, 0, stream>>>(aabbs, n, make_float3(sx, sy, sz), tan_pad, shape, param, out);
+    const float3 s = make_float3(sx, sy, sz);
+    if (n >= kStateClusterMin)
+        prepare_sun_kernel<kStateCluster>
+            <<<kStateCluster, kStateBlock, 0, stream>>>(aabbs, n, s, tan_pad, shape, param, out);
+    else
+        prepare_sun_kernel<1><<<1, kStateBlock, 0, stream>>>(aabbs, n, s, tan_pad, shape, param, out);
     return cudaGetLastError();
 }
 

@@ -72,12 +72,14 @@ struct SunGridJob {
     const SunFrame* sun;      // sun frame of the state (prepare_sun output)
     const Aabb* aabbs;        // [n] exact boxes, lo.w = element | type << kTypeShift
     int n;
-    int cap_cells;            // cell_start holds cap_cells + 1 entries, cursor cap_cells
+    int cap_cells;
     uint32_t cap_items;
     int pad;
-    uint32_t* cell_start;
-    uint32_t* cursor;
-    float4* rect;             // [n]
+    uint2* cells;             // [cap_cells]
+    uint32_t* alloc;          // items handed out to cells so far
+    float4* rect;             // [n] candidate rectangles
+    float4* reach_rect;       // [n] reach rectangles
+    uint32_t* reach;          // [kReachRaster^2 / 32]
     float4* item_rect;        // [cap_items]
     Aabb* item_box;           // [cap_items]
     uint32_t* global_id;      // [n]
@@ -95,8 +97,8 @@ size_t sungrid_bytes(uint32_t n);
 // aligned); fills every SunGridJob field except sun and aabbs.
 void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job);
 
-// Build the sun grids of n_jobs scene states (jobs: device array) on `stream`: reach rectangles and
-// grid size, counts, prefix sums, fill.  max_n = the largest element count among the jobs.
+// Build the sun grids of n_jobs scene states (jobs: device array) on `stream`; max_n =
+// the largest element count among the jobs.
 cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, cudaStream_t stream);
 
 // Trace rays [ray_begin, ray_begin + count): generation, closest-hit search, shading, the dense
@@ -168,7 +170,8 @@ struct SunJob {
 };
 
 cudaError_t launch_refit(const RefitJob* jobs, int n_jobs, int max_nodes, cudaStream_t stream);
-cudaError_t launch_prepare_sun_batch(const SunJob* jobs, int n_jobs, cudaStream_t stream);
+// max_n: the largest element count among the jobs
+cudaError_t launch_prepare_sun_batch(const SunJob* jobs, int n_jobs, int max_n, cudaStream_t stream);
 // Closest-hit search of a batch group: 0 element list (<= 8 elements), 1 BVH, 2 field grid.
 constexpr int kBatchGroups = 3;
 // Occupancy limit of the multi-instance kernel for (accel, block); 0 if unsupported.

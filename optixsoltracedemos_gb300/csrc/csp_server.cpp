@@ -590,7 +590,7 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
     RefitJob* refits = reinterpret_cast<RefitJob*>(h_adm + refit_at);
     SunJob* suns = reinterpret_cast<SunJob*>(h_adm + sun_at);
     SunGridJob* sgs = reinterpret_cast<SunGridJob*>(h_adm + sg_at);
-    int n_refit = 0, n_sun = 0, max_nodes = 0, n_sg = 0, max_sg_n = 0;
+    int n_refit = 0, n_sun = 0, max_nodes = 0, n_sg = 0, max_n = 0;
     for (size_t i = 0; i < admitted.size(); ++i) {
         SRequest& r = *admitted[i];
         const SScene& s = *r.sc;
@@ -654,8 +654,8 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
             sungrid_place(d_arena + r.o_sgrid, n, gj);
             gj.sun = sj.out;
             gj.aabbs = d_aabbs;
-            max_sg_n = std::max(max_sg_n, (int)n);
         }
+        max_n = std::max(max_n, (int)n);
         r.t_admit = Clock::now();
     }
     if (n_sun == 0) return CSP_OK;
@@ -669,11 +669,12 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
                          "refit_kernel");
     if (!rc)
         rc = cuda_status(
-            launch_prepare_sun_batch(reinterpret_cast<const SunJob*>(d_jobs + (sun_at - refit_at)), n_sun, adm_stream),
+            launch_prepare_sun_batch(reinterpret_cast<const SunJob*>(d_jobs + (sun_at - refit_at)), n_sun, max_n,
+                                     adm_stream),
             "prepare_sun_batch_kernel");
     if (!rc && n_sg)
         rc = cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(d_jobs + (sg_at - refit_at)), n_sg,
-                                              max_sg_n, adm_stream),
+                                              max_n, adm_stream),
                          "sun grid build");
     return rc;
 }

@@ -3,21 +3,27 @@
 //
 // The reference has no counterpart: OptiX traverses its GAS from the sun plane for every ray
 // (cuda/sun.cu:119-133).  Here the sun rays of scenes above 8 elements find their candidates in one
-// cell of a grid over the sun plane's Halton coordinates, binned from the elements' reach
-// rectangles (reach_rect, csp_trace.cuh), and rays outside every rectangle skip the direction and
-// the search altogether.  Which elements a ray tests changes, never which hit it finds: the reach
-// rectangles bound every ray that can meet an element's AABB, and the closest hit keeps the lower
-// element index on equal t whatever the order of the candidates.
+// cell of a grid over the sun plane's Halton coordinates, binned from the elements' candidate
+// rectangles (cross_rect, csp_trace.cuh), and rays in a clear cell of the reach raster (reach_rect)
+// skip the direction and the search altogether.  Which elements a ray tests changes, never which hit
+// it finds: the rectangles bound every ray that can meet an element's AABB, and the closest hit keeps
+// the lower element index on equal t whatever the order of the candidates.
 //
-// Four launches per set of states (blockIdx.y or blockIdx.x = the state):
-//   size   one block per state: every element's rectangle, the grid size from their mean extent
-//          (shrunk until the registered items fit the capacity), the descriptor, zeroed counts
-//   count  one thread per element: per-cell counts, or a place in the global list for rectangles of
-//          more than kSunGridMaxCells cells
-//   scan   one block per state: exclusive prefix sums of the counts (cell_start) and fill cursors
-//   fill   one thread per element: rectangles and exact boxes into their cells
-// The order of the items within a cell and of the global list follows the atomics; nothing that a
-// ray records depends on it.
+// Four launches per set of states:
+//   size    a cluster of kStateCluster blocks per state (dependent reductions over the elements: the
+//           middle of the field and with it the reference plane; every element's rectangles; the grid
+//           size from the candidate rectangles' mean extent, shrunk until the registered items fit
+//           the capacity), the descriptor, zeroed counts and raster
+//   count   kElemLanes threads per element: raster bits, per-cell counts, or a place in the global
+//           list for rectangles of more than kSunGridMaxCells cells
+//   ranges  one thread per four cells: a warp takes the sum of its cells' counts from the state's
+//           item counter
+//   fill    kElemLanes threads per element: rectangles and exact boxes into their cells
+// Each is a chain of memory latencies, so the wide ones take the whole device rather than one block
+// or cluster per state: 16 + 7 + 4.5 + 6 us for 10,001 elements, against 98 us with the count per
+// element and the scan in one block, and 96 us with all phases in one cluster.
+// The order of the cells' ranges, of the items within a cell and of the global list follows the
+// atomics; nothing that a ray records depends on it.
 #include <algorithm>
 
 #include "csp_kernels.cuh"
@@ -26,188 +32,214 @@
 namespace csp {
 namespace {
 
-constexpr int kSizeBlock = 512;
-constexpr int kElemBlock = 256;
-constexpr int kScanBlock = 1024;
 constexpr int kMaxAxisCells = 4096;
 constexpr float kCellScale = 0.5f;  // cell width / mean rectangle width
 constexpr int kMaxJobsPerLaunch = 65535;  // gridDim.y limit
+constexpr int kElemBlock = 256;
+constexpr int kElemLanes = 8;  // lanes that share an element's cells and raster words
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Cells covered by rectangle r in an nu x nv grid; false when r holds no point of [0, 1]^2.
-__device__ __forceinline__ bool sg_range(float4 r, float fnu, float fnv, int nu, int nv, int& iu0, int& iu1, int& iv0,
+// Cells covered by rectangle r, clamped to [0, 1]^2, in an nu x nv grid: a candidate point in r,
+// clamped the same way by the lookup, lies in one of them.
+__device__ __forceinline__ void sg_range(float4 r, float fnu, float fnv, int nu, int nv, int& iu0, int& iu1, int& iv0,
                                          int& iv1) {
-    if (!(r.y >= 0.0f && r.x <= 1.0f && r.w >= 0.0f && r.z <= 1.0f)) return false;
-    iu0 = sg_cell(fmaxf(r.x, 0.0f), fnu, nu);
-    iu1 = sg_cell(fminf(r.y, 1.0f), fnu, nu);
-    iv0 = sg_cell(fmaxf(r.z, 0.0f), fnv, nv);
-    iv1 = sg_cell(fminf(r.w, 1.0f), fnv, nv);
-    return true;
+    iu0 = sg_cell(__saturatef(r.x), fnu, nu);
+    iu1 = sg_cell(__saturatef(r.y), fnu, nu);
+    iv0 = sg_cell(__saturatef(r.z), fnv, nv);
+    iv1 = sg_cell(__saturatef(r.w), fnv, nv);
 }
 
-// Block-wide sum in a fixed order (the same result on every run).
-template <class T>
-__device__ T block_sum(T v, T* scratch) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    T s = scratch[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) s += scratch[i];
-    return s;
+// Set the raster bits of reach rectangle r (words w = lane of `lanes`, lane + lanes, ...).
+__device__ __forceinline__ void set_reach(uint32_t* __restrict__ raster, float4 r, int lane, int lanes) {
+    if (!(r.y >= 0.0f && r.x <= 1.0f && r.w >= 0.0f && r.z <= 1.0f)) return;  // holds no ray
+    int iu0, iu1, iv0, iv1;
+    sg_range(r, (float)kReachRaster, (float)kReachRaster, kReachRaster, kReachRaster, iu0, iu1, iv0, iv1);
+    const int w0 = iu0 >> 5, nw = (iu1 >> 5) - w0 + 1;
+    for (int k = lane; k < nw * (iv1 - iv0 + 1); k += lanes) {
+        const int row = iv0 + k / nw, word = w0 + k % nw;
+        const int b0 = max(iu0 - 32 * word, 0), b1 = min(iu1 - 32 * word, 31);
+        const uint32_t bits = (0xFFFFFFFFu >> (31 - b1)) & (0xFFFFFFFFu << b0);
+        uint32_t* p = raster + row * (kReachRaster / 32) + word;
+        if ((*reinterpret_cast<volatile uint32_t*>(p) & bits) != bits) atomicOr(p, bits);
+    }
 }
 
-__global__ void __launch_bounds__(kSizeBlock) sungrid_size_kernel(const SunGridJob* __restrict__ jobs) {
-    const SunGridJob J = jobs[blockIdx.x];
+__global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
+    sungrid_size_kernel(const SunGridJob* __restrict__ jobs) {
+    const SunGridJob& J = jobs[blockIdx.x / kStateCluster];
+    const int n = J.n;
+    constexpr int kThreads = kStateCluster * kStateBlock;
+    const int tid = (int)(blockIdx.x % kStateCluster) * kStateBlock + (int)threadIdx.x;
     __shared__ SunFrame S;
-    __shared__ float fs[kSizeBlock / 32];
-    __shared__ unsigned long long us[kSizeBlock / 32];
-    __shared__ int s_nu, s_nv;
+    __shared__ StateSmem sm;
+    __shared__ unsigned long long upart[kStateBlock / 32], uslot;
     if (threadIdx.x < sizeof(SunFrame) / 4)
         reinterpret_cast<uint32_t*>(&S)[threadIdx.x] = reinterpret_cast<const uint32_t*>(J.sun)[threadIdx.x];
+    for (int c = tid; c < kReachRaster * kReachRaster / 128; c += kThreads)
+        reinterpret_cast<uint4*>(J.reach)[c] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) *J.alloc = 0u;
     __syncthreads();
-    // reach rectangles; mean extent of the ordinary ones (not the whole-plane or oversized ones)
-    float su = 0.0f, sv = 0.0f;
-    unsigned long long cnt = 0;
-    for (int e = threadIdx.x; e < J.n; e += kSizeBlock) {
+    const float inf = __int_as_float(0x7f800000);
+    const float tan_a = cone_tan(S);
+    // the reference plane, horizontal or across the sun, through the middle of the elements before
+    // the receiver (the last one), whichever the cone can move less from
+    float zlo = inf, zhi = -inf, hlo = inf, hhi = -inf;
+    for (int e = tid; e + 1 < n; e += kThreads) {
         const Aabb b = J.aabbs[e];
-        const float4 r = reach_rect(S, b.lo, b.hi);
+        zlo = fminf(zlo, b.lo.z);
+        zhi = fmaxf(zhi, b.hi.z);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float h = dot(corner(b, k), xyz(S.w));
+            hlo = fminf(hlo, h);
+            hhi = fmaxf(hhi, h);
+        }
+    }
+    const float4 mid = state_reduce<kStateCluster>(make_float4(zlo, -zhi, hlo, -hhi), sm.part, &sm.slot, Min4());
+    const float dz = fabsf(S.w.z) - tan_a * sqrtf(fmaxf(0.0f, 1.0f - S.w.z * S.w.z));
+    const bool level = dz > 0.02f && (-mid.y - mid.x) < dz * (-mid.w - mid.z);
+    const float4 plane = level ? make_float4(0.0f, 0.0f, 1.0f, 0.5f * (mid.x - mid.y))
+                               : make_float4(S.w.x, S.w.y, S.w.z, 0.5f * (mid.z - mid.w));
+    const float den = level ? dz : dot(xyz(S.w), xyz(S.w)) - 1e-3f * tan_a;
+    // rectangles; mean extent of the ordinary candidate ones (not whole-plane or oversized)
+    float4 ext = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int e = tid; e < n; e += kThreads) {
+        const Aabb b = J.aabbs[e];
+        const BoxSpan span = box_span(S, plane, b.lo, b.hi);
+        J.reach_rect[e] = reach_rect(S, tan_a, span);
+        const float4 r = cross_rect(S, tan_a, den, span);
         J.rect[e] = r;
-        if (r.y >= 0.0f && r.x <= 1.0f && r.w >= 0.0f && r.z <= 1.0f) {
-            const float wu = fminf(r.y, 1.0f) - fmaxf(r.x, 0.0f), wv = fminf(r.w, 1.0f) - fmaxf(r.z, 0.0f);
-            if (wu < 0.25f && wv < 0.25f) {
-                su += wu;
-                sv += wv;
-                ++cnt;
-            }
-        }
+        const float wu = __saturatef(r.y) - __saturatef(r.x), wv = __saturatef(r.w) - __saturatef(r.z);
+        if (wu < 0.25f && wv < 0.25f) ext = Sum()(ext, make_float4(wu, wv, 1.0f, 0.0f));
     }
-    su = block_sum(su, fs);
-    sv = block_sum(sv, fs);
-    cnt = block_sum(cnt, us);
-    if (threadIdx.x == 0) {
-        // cells half as wide as the mean rectangle: a rectangle covers about 3 x 3 cells, and a ray
-        // scans the items of its cell -- on the 256-instance field batch 13 per generated ray with
-        // cells as wide as the mean rectangle (3.5 of them holding the ray), and 5 % less batch time
-        // with half-width cells than with those (no gain from a third)
-        int nu = 1, nv = 1;
-        if (cnt > 0) {
-            const float mu = fmaxf(su / (float)cnt, 1.0f / kMaxAxisCells), mv = fmaxf(sv / (float)cnt, 1.0f / kMaxAxisCells);
-            nu = min(kMaxAxisCells, max(1, (int)ceilf(1.0f / (mu * kCellScale))));
-            nv = min(kMaxAxisCells, max(1, (int)ceilf(1.0f / (mv * kCellScale))));
-        }
-        while ((long long)nu * nv > (long long)J.cap_cells) {
-            nu = max(1, nu * 3 / 4);
-            nv = max(1, nv * 3 / 4);
-        }
-        s_nu = nu;
-        s_nv = nv;
+    ext = state_reduce<kStateCluster>(ext, sm.part, &sm.slot, Sum());
+    // cells half as wide as the mean rectangle: a rectangle covers about 3 x 3 cells
+    int nu = 1, nv = 1;
+    if (ext.z > 0.0f) {
+        const float mu = fmaxf(ext.x / ext.z, 1.0f / kMaxAxisCells), mv = fmaxf(ext.y / ext.z, 1.0f / kMaxAxisCells);
+        nu = min(kMaxAxisCells, max(1, (int)ceilf(1.0f / (mu * kCellScale))));
+        nv = min(kMaxAxisCells, max(1, (int)ceilf(1.0f / (mv * kCellScale))));
     }
-    __syncthreads();
-    // shrink until the registered items fit (at 1 x 1 every element holds at most one item)
+    while ((long long)nu * nv > (long long)J.cap_cells) {
+        nu = max(1, nu * 3 / 4);
+        nv = max(1, nv * 3 / 4);
+    }
+    // shrink until the registered items fit (at 1 x 1 every element holds one item)
+    unsigned long long total;
     for (;;) {
-        const int nu = s_nu, nv = s_nv;
-        const float fnu = (float)nu, fnv = (float)nv;
         unsigned long long items = 0;
-        for (int e = threadIdx.x; e < J.n; e += kSizeBlock) {
+        for (int e = tid; e < n; e += kThreads) {
             int iu0, iu1, iv0, iv1;
-            if (!sg_range(J.rect[e], fnu, fnv, nu, nv, iu0, iu1, iv0, iv1)) continue;
+            sg_range(J.rect[e], (float)nu, (float)nv, nu, nv, iu0, iu1, iv0, iv1);
             const long long cells = (long long)(iu1 - iu0 + 1) * (iv1 - iv0 + 1);
             if (cells <= kSunGridMaxCells) items += (unsigned long long)cells;
         }
-        items = block_sum(items, us);
-        if (items <= J.cap_items || (nu == 1 && nv == 1)) break;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_nu = max(1, nu * 3 / 4);
-            s_nv = max(1, nv * 3 / 4);
-        }
-        __syncthreads();
+        total = state_reduce<kStateCluster>(items, upart, &uslot, Sum());
+        if (total <= J.cap_items || (nu == 1 && nv == 1)) break;
+        nu = max(1, nu * 3 / 4);
+        nv = max(1, nv * 3 / 4);
     }
-    const int nu = s_nu, nv = s_nv;
-    for (int c = threadIdx.x; c <= nu * nv; c += kSizeBlock) J.cell_start[c] = 0;
-    if (threadIdx.x == 0) {
+    for (int c = tid; c < nu * nv; c += kThreads) J.cells[c] = make_uint2(0u, 0u);
+    if (tid == 0) {
         SunGrid d;
         d.nu = nu;
         d.nv = nv;
         d.n_global = 0;
-        d.n = J.n;
+        d.n = n;
         d.fnu = (float)nu;
         d.fnv = (float)nv;
-        d.pad0 = d.pad1 = 0.0f;
-        d.cell_start = J.cell_start;
+        d.n_items = (int)total;
+        d.pad = 0;
+        d.plane = plane;
+        const float l1 = dot(xyz(S.e1), xyz(S.e1)), l2 = dot(xyz(S.e2), xyz(S.e2));
+        const bool ok = l1 > 0.0f && l2 > 0.0f;  // else every rectangle is the whole plane
+        d.e1 = ok ? make_float4(S.e1.x / l1, S.e1.y / l1, S.e1.z / l1, 0.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        d.e2 = ok ? make_float4(S.e2.x / l2, S.e2.y / l2, S.e2.z / l2, 0.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        d.cells = J.cells;
         d.item_rect = J.item_rect;
         d.item_box = J.item_box;
         d.global_id = J.global_id;
         d.rect = J.rect;
+        d.reach = J.reach;
         d.aabbs = J.aabbs;
         *J.desc = d;
     }
+    cooperative_groups::this_cluster().sync();  // the slots are read
 }
+
+// Cells of element e's candidate rectangle, k-th of `cells`.
+struct ElemCells {
+    int iu0, iv0, w, nu;
+    long long cells;
+    __device__ ElemCells(float4 r, int nu, int nv) : nu(nu) {
+        int iu1, iv1;
+        sg_range(r, (float)nu, (float)nv, nu, nv, iu0, iu1, iv0, iv1);
+        w = iu1 - iu0 + 1;
+        cells = (long long)w * (iv1 - iv0 + 1);
+    }
+    __device__ int at(int k) const { return (iv0 + k / w) * nu + iu0 + k % w; }
+};
 
 __global__ void __launch_bounds__(kElemBlock) sungrid_count_kernel(const SunGridJob* __restrict__ jobs) {
     const SunGridJob& J = jobs[blockIdx.y];
-    const int e = blockIdx.x * kElemBlock + threadIdx.x;
+    const int e = (int)(blockIdx.x * kElemBlock + threadIdx.x) / kElemLanes;
+    const int lane = threadIdx.x & (kElemLanes - 1);
     if (e >= J.n) return;
-    const int nu = J.desc->nu, nv = J.desc->nv;
-    int iu0, iu1, iv0, iv1;
-    if (!sg_range(J.rect[e], (float)nu, (float)nv, nu, nv, iu0, iu1, iv0, iv1)) return;
-    if ((long long)(iu1 - iu0 + 1) * (iv1 - iv0 + 1) > kSunGridMaxCells) {
-        const int k = atomicAdd(&J.desc->n_global, 1);
-        if (CSP_BOUNDS(6, k < J.n)) J.global_id[k] = (uint32_t)e;
+    set_reach(J.reach, J.reach_rect[e], lane, kElemLanes);
+    const ElemCells E(J.rect[e], J.desc->nu, J.desc->nv);
+    if (E.cells > kSunGridMaxCells) {
+        if (lane == 0) {
+            const int k = atomicAdd(&J.desc->n_global, 1);
+            if (CSP_BOUNDS(6, k < J.n)) J.global_id[k] = (uint32_t)e;
+        }
         return;
     }
-    for (int iv = iv0; iv <= iv1; ++iv)
-        for (int iu = iu0; iu <= iu1; ++iu)
-            if (CSP_BOUNDS(6, iv * nu + iu < J.cap_cells)) atomicAdd(J.cell_start + iv * nu + iu, 1u);
+    for (int k = lane; k < (int)E.cells; k += kElemLanes)
+        if (CSP_BOUNDS(6, E.at(k) < J.cap_cells)) atomicAdd(&J.cells[E.at(k)].y, 1u);
 }
 
-__global__ void __launch_bounds__(kScanBlock) sungrid_scan_kernel(const SunGridJob* __restrict__ jobs) {
-    const SunGridJob& J = jobs[blockIdx.x];
-    __shared__ uint32_t part[kScanBlock];
+__global__ void __launch_bounds__(kElemBlock) sungrid_ranges_kernel(const SunGridJob* __restrict__ jobs) {
+    const SunGridJob& J = jobs[blockIdx.y];
     const int nc = J.desc->nu * J.desc->nv;
-    const int chunk = (nc + kScanBlock - 1) / kScanBlock;
-    const int c0 = min(nc, (int)threadIdx.x * chunk), c1 = min(nc, c0 + chunk);
-    uint32_t s = 0;
-    for (int c = c0; c < c1; ++c) s += J.cell_start[c];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    // inclusive scan of the per-thread sums (Hillis-Steele)
-    for (int o = 1; o < kScanBlock; o <<= 1) {
-        const uint32_t v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
+    const int c = 4 * (int)(blockIdx.x * kElemBlock + threadIdx.x), lane = threadIdx.x & 31;
+    if (c - 4 * lane >= nc) return;  // whole warps
+    uint32_t k[4], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        k[i] = c + i < nc ? J.cells[c + i].y : 0u;
+        sum += k[i];
     }
-    uint32_t run = part[threadIdx.x] - s;
-    for (int c = c0; c < c1; ++c) {
-        const uint32_t k = J.cell_start[c];
-        J.cell_start[c] = run;
-        J.cursor[c] = run;
-        run += k;
+    uint32_t incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
-    if (threadIdx.x == kScanBlock - 1) J.cell_start[nc] = part[kScanBlock - 1];
+    uint32_t base = 0;
+    if (lane == 31 && incl) base = atomicAdd(J.alloc, incl);
+    base = __shfl_sync(0xffffffffu, base, 31) + incl - sum;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (c + i < nc) J.cells[c + i] = make_uint2(base, base);
+        base += k[i];
+    }
 }
 
 __global__ void __launch_bounds__(kElemBlock) sungrid_fill_kernel(const SunGridJob* __restrict__ jobs) {
     const SunGridJob& J = jobs[blockIdx.y];
-    const int e = blockIdx.x * kElemBlock + threadIdx.x;
+    const int e = (int)(blockIdx.x * kElemBlock + threadIdx.x) / kElemLanes;
     if (e >= J.n) return;
-    const int nu = J.desc->nu, nv = J.desc->nv;
     const float4 r = J.rect[e];
-    int iu0, iu1, iv0, iv1;
-    if (!sg_range(r, (float)nu, (float)nv, nu, nv, iu0, iu1, iv0, iv1)) return;
-    if ((long long)(iu1 - iu0 + 1) * (iv1 - iv0 + 1) > kSunGridMaxCells) return;
-    for (int iv = iv0; iv <= iv1; ++iv)
-        for (int iu = iu0; iu <= iu1; ++iu) {
-            if (!CSP_BOUNDS(6, iv * nu + iu < J.cap_cells)) continue;
-            const uint32_t k = atomicAdd(J.cursor + iv * nu + iu, 1u);
-            if (!CSP_BOUNDS(6, k < J.cap_items)) continue;
-            J.item_rect[k] = r;
-            J.item_box[k] = J.aabbs[e];
-        }
+    const ElemCells E(r, J.desc->nu, J.desc->nv);
+    if (E.cells > kSunGridMaxCells) return;
+    const Aabb b = J.aabbs[e];
+    for (int k = threadIdx.x & (kElemLanes - 1); k < (int)E.cells; k += kElemLanes) {
+        if (!CSP_BOUNDS(6, E.at(k) < J.cap_cells)) continue;
+        const uint32_t at = atomicAdd(&J.cells[E.at(k)].y, 1u);
+        if (!CSP_BOUNDS(6, at < J.cap_items)) continue;
+        J.item_rect[at] = r;
+        J.item_box[at] = b;
+    }
 }
 
 }  // namespace
@@ -223,8 +255,8 @@ SunGridCaps sungrid_caps(uint32_t n) {
 
 size_t sungrid_bytes(uint32_t n) {
     const SunGridCaps c = sungrid_caps(n);
-    return a256(sizeof(SunGrid)) + a256(((size_t)c.cap_cells + 1) * sizeof(uint32_t)) +
-           a256((size_t)c.cap_cells * sizeof(uint32_t)) + a256((size_t)n * sizeof(float4)) +
+    return a256(sizeof(SunGrid)) + a256((size_t)c.cap_cells * sizeof(uint2)) + a256(sizeof(uint32_t)) +
+           2 * a256((size_t)n * sizeof(float4)) + a256(kReachRaster * kReachRaster / 8) +
            a256((size_t)c.cap_items * sizeof(float4)) + a256((size_t)c.cap_items * sizeof(Aabb)) +
            a256((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t));
 }
@@ -238,9 +270,11 @@ void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job) {
         return p;
     };
     job.desc = reinterpret_cast<SunGrid*>(take(sizeof(SunGrid)));
-    job.cell_start = reinterpret_cast<uint32_t*>(take(((size_t)c.cap_cells + 1) * sizeof(uint32_t)));
-    job.cursor = reinterpret_cast<uint32_t*>(take((size_t)c.cap_cells * sizeof(uint32_t)));
+    job.cells = reinterpret_cast<uint2*>(take((size_t)c.cap_cells * sizeof(uint2)));
+    job.alloc = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t)));
     job.rect = reinterpret_cast<float4*>(take((size_t)n * sizeof(float4)));
+    job.reach_rect = reinterpret_cast<float4*>(take((size_t)n * sizeof(float4)));
+    job.reach = reinterpret_cast<uint32_t*>(take(kReachRaster * kReachRaster / 8));
     job.item_rect = reinterpret_cast<float4*>(take((size_t)c.cap_items * sizeof(float4)));
     job.item_box = reinterpret_cast<Aabb*>(take((size_t)c.cap_items * sizeof(Aabb)));
     job.global_id = reinterpret_cast<uint32_t*>(take((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t)));
@@ -252,14 +286,15 @@ void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job) {
 
 cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, cudaStream_t stream) {
     if (n_jobs <= 0 || max_n <= 0) return cudaSuccess;
+    const unsigned elem_blocks = (unsigned)(((uint64_t)max_n * kElemLanes + kElemBlock - 1) / kElemBlock);
+    const unsigned cell_blocks = (unsigned)((sungrid_caps((uint32_t)max_n).cap_cells / 4 + kElemBlock) / kElemBlock);
     for (int j0 = 0; j0 < n_jobs; j0 += kMaxJobsPerLaunch) {
-        const int nj = std::min(kMaxJobsPerLaunch, n_jobs - j0);
+        const unsigned nj = (unsigned)std::min(kMaxJobsPerLaunch, n_jobs - j0);
         const SunGridJob* J = jobs + j0;
-        const dim3 eg((unsigned)((max_n + kElemBlock - 1) / kElemBlock), (unsigned)nj);
-        sungrid_size_kernel<<<nj, kSizeBlock, 0, stream>>>(J);
-        sungrid_count_kernel<<<eg, kElemBlock, 0, stream>>>(J);
-        sungrid_scan_kernel<<<nj, kScanBlock, 0, stream>>>(J);
-        sungrid_fill_kernel<<<eg, kElemBlock, 0, stream>>>(J);
+        sungrid_size_kernel<<<nj * kStateCluster, kStateBlock, 0, stream>>>(J);
+        sungrid_count_kernel<<<dim3(elem_blocks, nj), kElemBlock, 0, stream>>>(J);
+        sungrid_ranges_kernel<<<dim3(cell_blocks, nj), kElemBlock, 0, stream>>>(J);
+        sungrid_fill_kernel<<<dim3(elem_blocks, nj), kElemBlock, 0, stream>>>(J);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

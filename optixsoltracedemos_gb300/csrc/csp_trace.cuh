@@ -33,6 +33,7 @@
 #pragma once
 
 #include <cfloat>
+#include <cooperative_groups.h>
 #include <type_traits>
 
 #include "csp_kernels.cuh"
@@ -166,33 +167,72 @@ __device__ __forceinline__ float3 corner(const Aabb& b, int k) {
     return make_float3((k & 1) ? b.hi.x : b.lo.x, (k & 2) ? b.hi.y : b.lo.y, (k & 4) ? b.hi.z : b.lo.z);
 }
 
-template <bool kMax>
-__device__ float block_reduce(float v, float* scratch) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const float w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = kMax ? fmaxf(v, w) : fminf(v, w);
+__device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ unsigned long long shfl_xor(unsigned long long v, int o) {
+    return __shfl_xor_sync(0xffffffffu, v, o);
+}
+__device__ __forceinline__ float4 shfl_xor(float4 v, int o) {
+    return make_float4(shfl_xor(v.x, o), shfl_xor(v.y, o), shfl_xor(v.z, o), shfl_xor(v.w, o));
+}
+// Reductions over the threads of one scene state: a block (kCluster = 1) or a thread-block cluster
+// of kCluster blocks, whose blocks exchange their partial results through distributed shared memory.
+// `part` holds a value per warp, `slot` the block's result; both may be reused after the call (the
+// cluster meets before the slot is written again), and a cluster meets once more before it exits.
+template <int kCluster, class T, class Op>
+__device__ T state_reduce(T v, T* part, T* slot, Op op) {
+    for (int o = 16; o > 0; o >>= 1) v = op(v, shfl_xor(v, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = part[0];
+    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) v = op(v, part[i]);
+    if constexpr (kCluster > 1) {
+        namespace cg = cooperative_groups;
+        const cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        if (threadIdx.x == 0) *slot = v;
+        cl.sync();
+        v = *cl.map_shared_rank(slot, 0);
+        for (int i = 1; i < kCluster; ++i) v = op(v, *cl.map_shared_rank(slot, i));
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    v = scratch[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) v = kMax ? fmaxf(v, scratch[i]) : fminf(v, scratch[i]);
     return v;
 }
+struct Min4 {
+    __device__ float4 operator()(float4 a, float4 b) const {
+        return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
+    }
+};
+struct Sum {
+    __device__ float4 operator()(float4 a, float4 b) const {
+        return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    }
+    __device__ unsigned long long operator()(unsigned long long a, unsigned long long b) const { return a + b; }
+};
 
-// One block computes the sun frame of one scene: plane distance, u/v bounds, parallelogram
-// (lib/sun_utils.cu:53-179, lib/geometry_manager.cpp:97-148) and cone frame (cuda/sun.cu:76-79).
-// `scratch` holds blockDim.x / 32 floats.
-__device__ void sun_frame_block(const Aabb* __restrict__ aabbs, int n, float3 s, float tan_pad, int shape,
-                                float param, SunFrame* __restrict__ out, float* scratch) {
+constexpr int kStateBlock = 512;    // threads of a state's block
+constexpr int kStateCluster = 8;    // blocks of a large state
+constexpr int kStateClusterMin = 1024;  // elements from which the sun frame takes a cluster
+struct StateSmem {
+    float4 part[kStateBlock / 32], slot;
+};
+
+// One block, or one cluster of kCluster blocks, computes the sun frame of one scene: plane distance,
+// u/v bounds, parallelogram (lib/sun_utils.cu:53-179, lib/geometry_manager.cpp:97-148) and cone frame
+// (cuda/sun.cu:76-79).  Two passes over the element boxes, the second after the first's result:
+// latency-bound, so large scenes spread them over a cluster (10,001 elements: 28.4 us in one block).
+template <int kCluster>
+__device__ void sun_frame_state(const Aabb* __restrict__ aabbs, int n, float3 s, float tan_pad, int shape,
+                                float param, SunFrame* __restrict__ out, StateSmem& sm) {
+    const int rank = kCluster > 1 ? (int)(blockIdx.x % kCluster) : 0;
+    const int first = rank * (int)blockDim.x + (int)threadIdx.x, step = kCluster * (int)blockDim.x;
+    const float inf = __int_as_float(0x7f800000);
     // plane distance: max over every AABB corner of |c . s| (and 0), lib/sun_utils.cu:53-104
     float md = 0.0f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = first; i < n; i += step) {
         const Aabb b = aabbs[i];
         for (int k = 0; k < 8; ++k) md = fmaxf(md, fabsf(dot(corner(b, k), s)));
     }
-    const float d = block_reduce<true>(md, scratch);
+    const float d = -state_reduce<kCluster>(make_float4(-md, inf, inf, inf), sm.part, &sm.slot, Min4()).x;
 
     const float3 axis = (fabsf(s.x) < 0.9f) ? f3(1.0f, 0.0f, 0.0f) : f3(0.0f, 1.0f, 0.0f);
     const float3 su = normalize(cross(axis, s));
@@ -200,7 +240,7 @@ __device__ void sun_frame_block(const Aabb* __restrict__ aabbs, int n, float3 s,
     const float3 pc = scale(d, s);
     // u/v bounds padded by |c . s| tan(angle), lib/sun_utils.cu:106-179
     float umin = FLT_MAX, umax = -FLT_MAX, vmin = FLT_MAX, vmax = -FLT_MAX;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = first; i < n; i += step) {
         const Aabb b = aabbs[i];
         for (int k = 0; k < 8; ++k) {
             const float3 pt = corner(b, k);
@@ -213,11 +253,14 @@ __device__ void sun_frame_block(const Aabb* __restrict__ aabbs, int n, float3 s,
             vmax = fmaxf(vmax, v + buf);
         }
     }
-    umin = block_reduce<false>(umin, scratch);
-    umax = block_reduce<true>(umax, scratch);
-    vmin = block_reduce<false>(vmin, scratch);
-    vmax = block_reduce<true>(vmax, scratch);
-    if (threadIdx.x != 0) return;
+    // the maxima as minima of the negated values
+    const float4 m = state_reduce<kCluster>(make_float4(umin, -umax, vmin, -vmax), sm.part, &sm.slot, Min4());
+    umin = m.x;
+    umax = -m.y;
+    vmin = m.z;
+    vmax = -m.w;
+    if constexpr (kCluster > 1) cooperative_groups::this_cluster().sync();  // the slots are read
+    if (rank != 0 || threadIdx.x != 0) return;
     const float3 ds = scale(d, s);
     const float3 v0 = add(add(scale(umin, su), scale(vmin, sv)), ds);
     const float3 v1 = add(add(scale(umax, su), scale(vmin, sv)), ds);
@@ -636,36 +679,39 @@ __device__ __forceinline__ bool in_rect(float4 r, float u, float v) {
     return (u >= r.x) & (u <= r.y) & (v >= r.z) & (v <= r.w);
 }
 
-// Whether some element's reach rectangle holds the sun-plane point (u, v): only then can the ray
-// meet an element box (otherwise its record is the sun-plane point alone).
+// dot product with fused steps: candidate selection only, never a recorded value
+__device__ __forceinline__ float fdot(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+
+// Whether the reach raster leaves it open that a sun ray from (u, v) meets an element box
+// (otherwise its record is the sun-plane point alone).
 __device__ __forceinline__ bool sun_reach_any(const SunGrid& G, float u, float v) {
-    const int c = sg_cell(v, G.fnv, G.nv) * G.nu + sg_cell(u, G.fnu, G.nu);
-    if (!CSP_BOUNDS(5, c >= 0 && c < G.nu * G.nv)) return true;
-    uint32_t j = __ldg(G.cell_start + c);
-    const uint32_t e = __ldg(G.cell_start + c + 1);
-    if (!CSP_BOUNDS(5, j <= e && e <= __ldg(G.cell_start + G.nu * G.nv))) return true;
-    for (; j < e; ++j)
-        if (in_rect(__ldg(G.item_rect + j), u, v)) return true;
-    for (int k = 0; k < G.n_global; ++k)
-        if (in_rect(__ldg(G.rect + __ldg(G.global_id + k)), u, v)) return true;
-    return false;
+    const int c = sg_cell(v, (float)kReachRaster, kReachRaster) * kReachRaster +
+                  sg_cell(u, (float)kReachRaster, kReachRaster);
+    if (!CSP_BOUNDS(5, c >= 0 && c < kReachRaster * kReachRaster)) return true;
+    return (__ldg(G.reach + (c >> 5)) >> (c & 31)) & 1u;
 }
 
 // Closest hit of the sun ray leaving the plane at (u, v) = o with direction d: the elements of its
-// cell and of the global list whose reach rectangles hold (u, v), each through the exact AABB test
-// and its intersection program (test_box).  Every element whose box the ray meets is among them,
-// so this is the closest hit over all elements (equal t keeps the lower element index).
+// candidate point's cell and of the global list whose candidate rectangles hold the point, each
+// through the exact AABB test and its intersection program (test_box).  Every element whose box the
+// ray meets is among them, so this is the closest hit over all elements (equal t keeps the lower
+// element index).  The candidate point only has to be right to the rectangles' margins, so its
+// division is the approximate one and its products may fuse.
 __device__ __forceinline__ int sun_closest(const SunGrid& G, const Prim* __restrict__ prims, float u, float v,
                                            float3 o, float3 d, bool acc, float& best_t, uint32_t& best_type) {
+    const float s = __fdividef(G.plane.w - fdot(xyz(G.plane), o), fdot(xyz(G.plane), d));
+    u = fmaf(s, fdot(xyz(G.e1), d), u);
+    v = fmaf(s, fdot(xyz(G.e2), d), v);
     const float3 inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
     int best = -1;
     best_t = __int_as_float(0x7f800000);
     float prune = kTmax;
-    const int c = sg_cell(v, G.fnv, G.nv) * G.nu + sg_cell(u, G.fnu, G.nu);
+    const int c = sg_cell(__saturatef(v), G.fnv, G.nv) * G.nu + sg_cell(__saturatef(u), G.fnu, G.nu);
     if (!CSP_BOUNDS(5, c >= 0 && c < G.nu * G.nv)) return best;
-    uint32_t j = __ldg(G.cell_start + c);
-    const uint32_t e = __ldg(G.cell_start + c + 1);
-    if (!CSP_BOUNDS(5, j <= e && e <= __ldg(G.cell_start + G.nu * G.nv))) return best;
+    const uint2 range = __ldg(G.cells + c);
+    uint32_t j = range.x;
+    const uint32_t e = range.y;
+    if (!CSP_BOUNDS(5, j <= e && e <= (uint32_t)G.n_items)) return best;
     for (; j < e; ++j) {
         if (!in_rect(__ldg(G.item_rect + j), u, v)) continue;
         const float4* q = reinterpret_cast<const float4*>(G.item_box + j);
@@ -863,6 +909,53 @@ __device__ __forceinline__ float3 sun_direction(const typename C::Args& A, const
     return dir;
 }
 
+// Tangent of the largest angle between a sun ray and the cone axis, 1 % (and 1e-6) high.
+__device__ __forceinline__ float cone_tan(const SunFrame& S) {
+    float tan_a;
+    if (S.shape & 1) {
+        tan_a = 5.8f * S.sigma;
+    } else if (S.shape & 2) {
+        const float c = S.cos_theta;
+        tan_a = c > 0.2f ? sqrtf(S.omc * (2.0f - S.omc)) / c : __int_as_float(0x7f800000);
+    } else {
+        const float c = S.cos_theta;
+        tan_a = c > 0.2f ? sqrtf(fmaxf(0.0f, 1.0f - c * c)) / c : __int_as_float(0x7f800000);
+    }
+    return tan_a * 1.01f + 1e-6f;
+}
+
+// An element box over the sun plane: the range of its corners' Halton coordinates, its depth below
+// the plane and its largest distance from the reference plane.
+struct BoxSpan {
+    float umin, umax, vmin, vmax, hmax, off;
+};
+
+__device__ __forceinline__ BoxSpan box_span(const SunFrame& S, float4 plane, float4 lo, float4 hi) {
+    const float3 v0 = xyz(S.v0), e1 = xyz(S.e1), e2 = xyz(S.e2), w = xyz(S.w);
+    const float i1 = 1.0f / dot(e1, e1), i2 = 1.0f / dot(e2, e2), inf = __int_as_float(0x7f800000);
+    BoxSpan s{inf, -inf, inf, -inf, 0.0f, 0.0f};
+    const Aabb b{lo, hi};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float3 c = corner(b, k), r = sub(c, v0);
+        const float du = dot(r, e1) * i1, dv = dot(r, e2) * i2;
+        s.umin = fminf(s.umin, du);
+        s.umax = fmaxf(s.umax, du);
+        s.vmin = fminf(s.vmin, dv);
+        s.vmax = fmaxf(s.vmax, dv);
+        s.hmax = fmaxf(s.hmax, dot(r, w));
+        s.off = fmaxf(s.off, fabsf(dot(xyz(plane), c) - plane.w));
+    }
+    return s;
+}
+
+// The span widened by (ru, rv); degenerate frames (a zero or overflowing axis) give the whole plane.
+__device__ __forceinline__ float4 widened(const BoxSpan& s, float ru, float rv) {
+    const float inf = __int_as_float(0x7f800000);
+    const float4 r = make_float4(s.umin - ru, s.umax + ru, s.vmin - rv, s.vmax + rv);
+    return r.x <= r.y && r.z <= r.w ? r : make_float4(-inf, inf, -inf, inf);
+}
+
 // Reach rectangle of one element box: Halton coordinates (u in [x, y], v in [z, w]) outside which
 // no sun ray can meet the box.  A ray leaves the sun plane at o = v0 + u e1 + v e2 with a direction
 // at most a from the cone axis w; at depth h below the plane it has moved at most h tan a across
@@ -874,41 +967,24 @@ __device__ __forceinline__ float3 sun_direction(const typename C::Args& A, const
 // 1 mm on the distance, 1e-5 in Halton units, far above the float rounding of the ray's origin,
 // direction and box test, so a ray outside every rectangle fails the exact box test of every
 // element.  Degenerate frames give the whole plane.
-__device__ __forceinline__ float4 reach_rect(const SunFrame& S, float4 lo, float4 hi) {
-    const float3 v0 = xyz(S.v0), e1 = xyz(S.e1), e2 = xyz(S.e2), w = xyz(S.w);
-    const float l1 = dot(e1, e1), l2 = dot(e2, e2);
-    float tan_a;
-    if (S.shape & 1) {
-        tan_a = 5.8f * S.sigma;
-    } else if (S.shape & 2) {
-        const float c = S.cos_theta;
-        tan_a = c > 0.2f ? sqrtf(S.omc * (2.0f - S.omc)) / c : __int_as_float(0x7f800000);
-    } else {
-        const float c = S.cos_theta;
-        tan_a = c > 0.2f ? sqrtf(fmaxf(0.0f, 1.0f - c * c)) / c : __int_as_float(0x7f800000);
-    }
-    tan_a = tan_a * 1.01f + 1e-6f;
-    float umin = __int_as_float(0x7f800000), umax = -umin, vmin = umin, vmax = -umin, hmax = 0.0f;
-    const Aabb b{lo, hi};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float3 r = sub(corner(b, k), v0);
-        const float du = dot(r, e1) / l1, dv = dot(r, e2) / l2;
-        umin = fminf(umin, du);
-        umax = fmaxf(umax, du);
-        vmin = fminf(vmin, dv);
-        vmax = fmaxf(vmax, dv);
-        hmax = fmaxf(hmax, dot(r, w));
-    }
-    const float n1 = sqrtf(l1), n2 = sqrtf(l2);
-    const float rad = hmax * tan_a + 1e-4f * (length(v0) + n1 + n2 + hmax) + 1e-3f;
-    const float ru = rad / n1 + 1e-5f, rv = rad / n2 + 1e-5f;
-    float4 r = make_float4(umin - ru, umax + ru, vmin - rv, vmax + rv);
-    if (!(l1 > 0.0f && l2 > 0.0f && r.x <= r.y && r.z <= r.w)) {
-        const float inf = __int_as_float(0x7f800000);
-        r = make_float4(-inf, inf, -inf, inf);
-    }
-    return r;
+__device__ __forceinline__ float4 reach_rect(const SunFrame& S, float tan_a, const BoxSpan& b) {
+    const float n1 = length(xyz(S.e1)), n2 = length(xyz(S.e2));
+    const float rad = b.hmax * tan_a + 1e-4f * (length(xyz(S.v0)) + n1 + n2 + b.hmax) + 1e-3f;
+    return widened(b, rad / n1 + 1e-5f, rad / n2 + 1e-5f);
+}
+
+// Candidate rectangle of one element box: the (u', v') outside which no sun ray can meet it.  A ray
+// o + h (w + t), t across the axis with |t| <= tan a, meets the plane n.P = c at depth h_P and a point
+// Q of the box at depth h_Q: |h_Q - h_P| = |n.Q - c| / |n.(w + t)|, and |n.(w + t)| is at least den =
+// |n.w| - tan a sqrt(1 - (n.w)^2).  Projected along w, the two lie |h_Q - h_P| |t| apart, so the
+// ray's candidate point -- its crossing of the plane, projected -- lies within max |n.Q - c| tan a /
+// den of the box's projection.  Margins: 1 % on tan a, 5e-6 of the scene's extent plus 1 mm (the
+// rounding of the ray's origin, direction and crossing moves the point by about 1e-6 of it), 2e-6 in
+// Halton units.
+__device__ __forceinline__ float4 cross_rect(const SunFrame& S, float tan_a, float den, const BoxSpan& b) {
+    const float n1 = length(xyz(S.e1)), n2 = length(xyz(S.e2));
+    const float rad = (b.off / den) * tan_a + 5e-6f * (length(xyz(S.v0)) + n1 + n2 + fabsf(b.hmax)) + 1e-3f;
+    return widened(b, rad / n1 + 2e-6f, rad / n2 + 2e-6f);
 }
 
 // Queue entries of BVH/grid launches carry the depth of their pending mirror hit in the top bits of
@@ -1227,7 +1303,7 @@ __device__ __forceinline__ void load_instance_smem(const typename C::Args& A, ty
             sm.flat.box[k].lo = nd.lo;
             sm.flat.box[k].hi = nd.hi;
             sm.flat.type[k] = (__float_as_uint(nd.lo.w) >> kTypeShift) & 7u;
-            sm.reach[k] = reach_rect(*A.sun, nd.lo, nd.hi);
+            sm.reach[k] = reach_rect(*A.sun, cone_tan(*A.sun), box_span(*A.sun, make_float4(0.f, 0.f, 0.f, 0.f), nd.lo, nd.hi));
         }
         if (k == 0) sm.flat.n = min(nprim, kFlatMax);
     }

@@ -94,25 +94,39 @@ struct alignas(16) GridDesc {
 };
 
 // Candidate grid of the sun rays of one scene state and sun frame (scenes of more than 8
-// elements), built on the device after the sun plane.  Every element has a reach rectangle in the
-// Halton coordinates (u, v) of the sun plane, outside which no sun ray can meet its AABB (rect[e],
-// see reach_rect in csp_trace.cuh).  [0, 1]^2 is cut into nu x nv cells; cell (iu, iv) lists
-// (items[cell_start[iv nu + iu] .. cell_start[iv nu + iu + 1])) every element whose rectangle overlaps
-// it, with the rectangle (item_rect) and the element's exact box (item_box, lo.w = element | type
-// << kTypeShift) inline, so that a candidate's box test does not wait for an index.  Elements whose
-// rectangle covers more than kSunGridMaxCells cells are in the global list instead, tested by every
-// ray.  A sun ray at (u, v) can only meet the elements of its cell and the global list whose
-// rectangles hold (u, v); a ray that lies in none meets no element box at all.
+// elements), built on the device after the sun plane.  Two tests, both in the Halton coordinates
+// (u, v) of the sun plane:
+//   before the direction is drawn: bit (u, v) of the reach raster (kReachRaster^2 bits), set where
+//     the reach rectangle of some element (reach_rect in csp_trace.cuh: the element's box widened by
+//     what any direction of the cone can move over the whole depth of the scene) overlaps the raster
+//     cell.  A ray in a clear cell meets no element box at all.
+//   with the direction: the point where the ray crosses the reference plane (a plane through the
+//     middle of the field), projected back along the cone axis, is its candidate point (u', v').  An
+//     element's candidate rectangle rect[e] (cross_rect) is its box's projection widened only by what
+//     the cone can move between that plane and the box -- centimetres for a heliostat in the layer of
+//     its field, where the reach rectangle of a field 1 km below the sun plane is wider than the
+//     mirror.  A ray meets no box whose candidate rectangle does not hold (u', v').
+// [0, 1]^2 is cut into nu x nv cells; cell (iu, iv) lists (items [x, y) of cells[iv nu + iu]) every
+// element whose candidate rectangle overlaps it (both clamped to
+// [0, 1]), with the rectangle (item_rect) and the element's exact box (item_box, lo.w = element |
+// type << kTypeShift) inline, so that a candidate's box test does not wait for an index.  Elements
+// whose rectangle covers more than kSunGridMaxCells cells are in the global list instead, tested by
+// every ray.
 constexpr int kSunGridMaxCells = 64;     // cells of one element's rectangle before it goes global
+constexpr int kReachRaster = 512;        // raster cells per axis: 32 KB, resident in L1
 constexpr int kSunGridItemsPerElem = 12;  // item capacity per element (the sizing keeps the total below)
 struct alignas(16) SunGrid {
     int nu, nv, n_global, n;
-    float fnu, fnv, pad0, pad1;
-    const uint32_t* cell_start;  // [nu nv + 1]
+    float fnu, fnv;
+    int n_items, pad;
+    float4 plane;                // reference plane: xyz . P = w
+    float4 e1, e2;               // SunFrame e1 / |e1|^2, e2 / |e2|^2: metres across the plane -> (u, v)
+    const uint2* cells;          // [nu nv], item range of each cell
     const float4* item_rect;
     const Aabb* item_box;
     const uint32_t* global_id;   // [n_global]
-    const float4* rect;          // [n], every element's reach rectangle
+    const float4* rect;          // [n], every element's candidate rectangle
+    const uint32_t* reach;       // reach raster, row v of kReachRaster / 32 words
     const Aabb* aabbs;           // exact element boxes, lo.w = element | type << kTypeShift (bits)
 };
 
