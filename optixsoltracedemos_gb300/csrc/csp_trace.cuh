@@ -94,9 +94,9 @@ struct Cfg {
     // arguments from shared memory)
     static constexpr bool kSched = kAccel_ == kAccelFlat && kDense_;
     using Args = std::conditional_t<kSched, TraceArgsK, TraceArgs>;
-    // every launch defers the direction of the sun rays whose sun-plane point may reach an element
-    // box to full batches (the generation queue); the other rays provably miss.  Element-list
-    // launches test the reach rectangles of their elements, the others the sun grid (SunGrid).
+    // element-list launches defer the direction of the sun rays whose sun-plane point may reach an
+    // element box to full batches (the generation queue), the other rays provably miss; BVH and grid
+    // launches trace the first segment in place (first_segment)
     using Core = CoreSmem<kB_, kFlat>;
     // phase A record staging of dense element-list launches
     using Stage = FlatStageSmem<kB_>;
@@ -993,17 +993,16 @@ constexpr int kDepthShift = 56;
 constexpr uint64_t kRayMask = (1ull << kDepthShift) - 1u;
 static_assert((1ull << kDepthShift) == kRayIndexLimit, "the host ray-window check must match the packing");
 
-// Shared memory of one CTA: the bounce queue, the generation queue (sun rays waiting for their
-// direction: kFlat launches keep the sun-plane point, the others its Halton coordinates), the
-// Halton table, the sun frame, and the kFlat scene with its elements' reach rectangles or the
-// descriptors of the grids of the other launches.
+// Shared memory of one CTA: the bounce queue, the generation queue of kFlat launches (sun-plane points
+// of the rays waiting for their direction), the Halton table, the sun frame, and the kFlat scene with
+// its elements' reach rectangles or the descriptors of the grids of the other launches.
 template <int kB, bool kFlat>
 struct CoreSmem {
     float qo[3][2 * kB], qd[3][2 * kB], qt[2 * kB];
     uint32_t qw[2 * kB];  // kFlat: candidate mask; BVH: element | type << 28 of the pending mirror hit
     uint64_t qray[2 * kB];
-    float go[3][2 * kB];
-    uint64_t gray[2 * kB];
+    float go[3][kFlat ? 2 * kB : 1];
+    uint64_t gray[kFlat ? 2 * kB : 1];
     float4 reach[kFlat ? kFlatMax : 1];
     float t6[kH3Tab];
     FlatScene flat;
@@ -1216,12 +1215,10 @@ __device__ __forceinline__ int bounce_batch(const typename C::Args& A, const Sin
     }
 }
 
-// One batch of up to kB rays from the top of the generation queue (gs entries): sun direction and
-// the closest-hit search of the first segment, on full warps.  Element-list launches run the box
-// tests and queue the rays that meet a box with their candidate mask; the others find the closest
-// hit among the sun-grid candidates, emit its record and queue mirror hits for shading.  Both append
-// to the bounce queue (qs entries, fewer than kB on entry).  Updates gs and qs, the same in every
-// thread (the closing barrier counts the rays queued).
+// One batch of up to kB rays from the top of the generation queue (element-list launches; gs
+// entries): sun direction and the box tests of the first segment, on full warps; rays that meet a box
+// go to the bounce queue (qs entries, fewer than kB on entry) with their candidate mask.  Updates gs
+// and qs, the same in every thread (the closing barrier counts the rays queued).
 template <class C>
 __device__ __forceinline__ void gen_batch(const typename C::Args& A, const Sink& k, typename C::Core& sm, int& gs,
                                           int& qs) {
@@ -1239,36 +1236,15 @@ __device__ __forceinline__ void gen_batch(const typename C::Args& A, const Sink&
     }
     __syncthreads();
     if (threadIdx.x == 0) sm.gsize = base;
-    if constexpr (C::kFlat) {
-        const float3 o = f3(a, b, c);
-        float3 d = f3(0.f, 0.f, 1.f);
-        uint32_t m = 0;
-        if (have) {
-            d = sun_direction<C>(A, sm.sun, ray);
-            m = candidates(sm.flat, o, d, kTminSun);
-        }
-        push(sm, m != 0u, ray, o, d, 0.0f, m);
-        qs += __syncthreads_count(m != 0u);
-    } else {
-        // (a, b) = the Halton coordinates of the ray's sun-plane point
-        bool again = false;
-        Segment g{f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 1.f), kTminSun, 0};
-        Hit h{-1, 0.f, 0u};
-        if (have) {
-            g.o = sun_point(sm.sun, a, b);
-            g.d = sun_direction<C>(A, sm.sun, ray);
-            h.best = sun_closest(sm.sg, A.prims, a, b, g.o, g.d, (sm.sun.shape & 2) != 0, h.t, h.type);
-            if (h.best >= 0) {
-                const Prim p = load_prim(A.prims, (uint32_t)h.best);
-                float4 rec;
-                int s;
-                again = classify(p, g, h, rec, s);
-                if (s >= 0) emit<C>(A, k, ray, s, rec, (uint32_t)h.best);
-            }
-        }
-        push(sm, again, ray, g.o, g.d, h.t, (uint32_t)h.best | (h.type << kTypeShift));
-        qs += __syncthreads_count(again);
+    const float3 o = f3(a, b, c);
+    float3 d = f3(0.f, 0.f, 1.f);
+    uint32_t m = 0;
+    if (have) {
+        d = sun_direction<C>(A, sm.sun, ray);
+        m = candidates(sm.flat, o, d, kTminSun);
     }
+    push(sm, m != 0u, ray, o, d, 0.0f, m);
+    qs += __syncthreads_count(m != 0u);
     gs = base;
 }
 
@@ -1279,9 +1255,17 @@ __device__ __forceinline__ void gen_batch(const typename C::Args& A, const Sink&
 template <class C>
 __device__ void drain(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool all, int& qs, int& gs) {
     for (;;) {
-        if (qs >= C::kB || (all && qs > 0 && gs == 0)) qs = bounce_batch<C>(A, k, sm, qs);
-        else if (gs >= C::kB || (all && gs > 0)) gen_batch<C>(A, k, sm, gs, qs);
-        else break;
+        if (qs >= C::kB || (all && qs > 0 && gs == 0)) {
+            qs = bounce_batch<C>(A, k, sm, qs);
+            continue;
+        }
+        if constexpr (C::kFlat) {
+            if (gs >= C::kB || (all && gs > 0)) {
+                gen_batch<C>(A, k, sm, gs, qs);
+                continue;
+            }
+        }
+        break;
     }
 }
 
@@ -1314,6 +1298,60 @@ __device__ __forceinline__ void load_instance_smem(const typename C::Args& A, ty
             reinterpret_cast<const uint32_t*>(A.sgrid)[threadIdx.x - 64];
 }
 
+// Phase A of one tile of a BVH or grid launch, one ray per thread: the sun-plane point, and unless
+// the reach raster rules every element out, the direction, the closest hit among the sun-grid
+// candidates and its record; mirror hits are queued for the bounce batches.  The coherent ray order
+// gives a warp neighbouring points, so its lanes mostly agree on the raster and on the candidates,
+// and the first segment needs no queue of its own: against a generation queue like the element
+// lists' (two CTA barriers per batch of directions, 10 KB of shared memory, the record's slot 1
+// stored a second time) 64M rays over 10,000 heliostats went from 6249 to 5855 us, 1.2M rays over a
+// hillside of 600 from 118 to 107 us.
+template <class C>
+__device__ __forceinline__ void first_segment(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool have,
+                                              uint64_t pos, uint64_t ray, int& qs) {
+    Segment g{f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 1.f), kTminSun, 0};
+    Hit h{-1, 0.f, 0u};
+    bool again = false;
+    int slot = -1;
+    float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (have) {
+        const float hu = halton2(ray), hv = halton3_tab(ray, sm.t6, A.h3t12);
+        g.o = sun_point(sm.sun, hu, hv);
+        if (sun_reach_any(sm.sg, hu, hv)) {
+            g.d = sun_direction<C>(A, sm.sun, ray);
+            h.best = sun_closest(sm.sg, A.prims, hu, hv, g.o, g.d, (sm.sun.shape & 2) != 0, h.t, h.type);
+            if (h.best >= 0) {
+                const Prim p = load_prim(A.prims, (uint32_t)h.best);
+                again = classify(p, g, h, rec, slot);
+                if constexpr (C::kFlux) {
+                    if (slot >= 0) flux_record(k, rec, slot);
+                }
+            }
+        }
+    }
+    push(sm, again, ray, g.o, g.d, h.t, (uint32_t)h.best | (h.type << kTypeShift));
+    if constexpr (C::kDense) {
+        // each lane writes its own ray's 80 B row: the sun-plane record, the first hit's, empty slots
+        // (the bounce batches overwrite the slots they fill, after the barriers between)
+        if (have && CSP_BOUNDS(2, pos < A.count)) {
+            if (slot < 0) rec = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4* gh = A.hits + pos * kMaxDepth;
+            gh[0] = make_float4(0.0f, g.o.x, g.o.y, g.o.z);
+            gh[1] = rec;
+#pragma unroll
+            for (int s = 2; s < kMaxDepth; ++s) gh[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (A.ids) {
+                uint32_t* gi = A.ids + pos * kMaxDepth;
+#pragma unroll
+                for (int s = 0; s < kMaxDepth; ++s) gi[s] = s == 1 && slot == 1 ? (uint32_t)h.best : kNoElement;
+            }
+        }
+    }
+    // the barrier before the bounce batches counts this tile's appends
+    qs += __syncthreads_count(again);
+    while (qs >= C::kB) qs = bounce_batch<C>(A, k, sm, qs);
+}
+
 // Phase A of one tile (rays A.ray_begin + tile * kB ...) followed by phase B on full batches.
 // `stage` is the kDense staging area of element-list launches (unused otherwise); qs, gs: the queue
 // sizes (see drain).
@@ -1327,6 +1365,10 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
     // shared cells save
     if constexpr (C::kCoherent) pos = coherent_order<!C::kDense, C::kDense ? 2 : C::kB / 32>(kk, A.count);
     const uint64_t ray = A.ray_begin + pos;
+    if constexpr (!C::kFlat) {
+        first_segment<C>(A, k, sm, kk < A.count, pos, ray, qs);
+        return;
+    }
     // sun-plane point; the direction waits in the generation queue unless the point lies outside
     // every reach rectangle (then the ray meets no element box and its record is the point alone)
     bool want = false;
@@ -1336,37 +1378,16 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
         hu = halton2(ray);
         hv = halton3_tab(ray, sm.t6, A.h3t12);
         o = sun_point(sm.sun, hu, hv);
-        if constexpr (C::kFlat) {
-            const int nr = sm.flat.n;
+        const int nr = sm.flat.n;
 #pragma unroll
-            for (int e = 0; e < kFlatMax; ++e) {
-                if (e >= nr) break;
-                want |= in_rect(sm.reach[e], hu, hv);
-            }
-        } else {
-            want = sun_reach_any(sm.sg, hu, hv);
+        for (int e = 0; e < kFlatMax; ++e) {
+            if (e >= nr) break;
+            want |= in_rect(sm.reach[e], hu, hv);
         }
     }
     __syncwarp();
-    // element-list launches queue the point, the others its Halton coordinates (their batch looks
-    // up the cell again)
-    if constexpr (C::kFlat) push_gen(sm, want, ray, o);
-    else push_gen(sm, want, ray, f3(hu, hv, 0.f));
-    if constexpr (C::kDense && C::kCoherent) {
-        // each lane writes its own ray's 80 B row: the sun-plane record, then empty slots (the
-        // generation and bounce batches overwrite the slots they fill, after the barriers between)
-        if (kk < A.count && CSP_BOUNDS(2, pos < A.count)) {
-            float4* gh = A.hits + pos * kMaxDepth;
-            gh[0] = make_float4(0.0f, o.x, o.y, o.z);
-#pragma unroll
-            for (int s = 1; s < kMaxDepth; ++s) gh[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (A.ids) {
-                uint32_t* gi = A.ids + pos * kMaxDepth;
-#pragma unroll
-                for (int s = 0; s < kMaxDepth; ++s) gi[s] = kNoElement;
-            }
-        }
-    } else if constexpr (C::kDense) {
+    push_gen(sm, want, ray, o);
+    if constexpr (C::kDense) {
         // the warp's 32 x 80 B of records leave as 5 fully coalesced 512-byte rows: record e of the
         // warp is slot e mod 5 of ray e / 5, the staged sun-plane record for slot 0, else empty
         float4* wh = stage->rec0 + warp * 32;
