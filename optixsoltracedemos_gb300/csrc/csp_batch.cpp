@@ -14,7 +14,7 @@
 // result buffers, graph, events): run_async builds the next run on the host while the previous one
 // executes, wait completes the oldest run in flight.
 //
-// Device layout (offsets 16-byte aligned):
+// Device layout (offsets 32-byte aligned):
 //   upload  [per instance: prims | optics | aabbs | prune (| own field grid)] [descs per group]
 //           [tile_begin per group] [refit jobs] [sun jobs] [sun grid jobs]
 //   nodes   per-instance refitted BVH nodes and sun grid (written on the device)
@@ -44,7 +44,8 @@
 namespace csp {
 namespace {
 
-size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
+// offsets 32-byte aligned: the kernels read records and boxes 32 bytes at a time
+size_t align32(size_t x) { return (x + 31) & ~(size_t)31; }
 
 // Tuned launch parameters per (device model, kernel build, kernel group, ray-count class), shared
 // by every batch of the process and, when a cache file is set (csp_set_tune_cache, or the
@@ -300,21 +301,21 @@ int Batch::layout(int si) {
         p.group = s.flat ? kAccelFlat : (grid_of(i).valid ? kAccelGrid : kAccelBvh);
         p.slot = n_group[p.group]++;
         p.prims = off;
-        off += align16(ne * sizeof(Prim));
+        off += align32(ne * sizeof(Prim));
         p.optics = off;
-        off += align16(ne * sizeof(Optics));
+        off += align32(ne * sizeof(Optics));
         p.aabbs = off;
-        off += align16(ne * sizeof(Aabb));
+        off += align32(ne * sizeof(Aabb));
         p.prune = off;
-        off += align16(ne * sizeof(Aabb));
+        off += align32(ne * sizeof(Aabb));
         if (p.group == kAccelGrid && !inst[i].poses.empty()) {
             const HostGrid& hg = builds[i].grid;
             p.cells = off;
-            off += align16(hg.cell_start.size() * sizeof(uint32_t));
+            off += align32(hg.cell_start.size() * sizeof(uint32_t));
             p.items = off;
-            off += align16(hg.items.size() * sizeof(Aabb));
+            off += align32(hg.items.size() * sizeof(Aabb));
             p.global = off;
-            off += align16(std::max<size_t>(1, hg.global.size()) * sizeof(Aabb));
+            off += align32(std::max<size_t>(1, hg.global.size()) * sizeof(Aabb));
         }
         if (p.group != kAccelGrid) {
             p.rf_slot = n_refit++;
@@ -327,32 +328,32 @@ int Batch::layout(int si) {
     }
     for (int g = 0; g < kBatchGroups; ++g) {
         desc_off[g] = off;
-        off += align16(n_group[g] * sizeof(InstanceDesc));
+        off += align32(n_group[g] * sizeof(InstanceDesc));
     }
     for (int g = 0; g < kBatchGroups; ++g) {
         tb_off[g] = off;
-        off += align16((n_group[g] + 1) * sizeof(uint64_t));
+        off += align32((n_group[g] + 1) * sizeof(uint64_t));
     }
     refit_off = off;
-    off += align16((size_t)n_refit * sizeof(RefitJob));
+    off += align32((size_t)n_refit * sizeof(RefitJob));
     sunjob_off = off;
-    off += align16(n * sizeof(SunJob));
+    off += align32(n * sizeof(SunJob));
     sgjob_off = off;
-    off += align16((size_t)n_sg * sizeof(SunGridJob));
+    off += align32((size_t)n_sg * sizeof(SunGridJob));
     up_bytes = off;
     for (size_t i = 0; i < n; ++i) {
         if (place[i].rf_slot >= 0) {
             place[i].nodes = off;
-            off += align16(scenes[inst[i].scene].base.nodes.size() * sizeof(Node));
+            off += align32(scenes[inst[i].scene].base.nodes.size() * sizeof(Node));
         }
         if (place[i].sg_slot >= 0) {
             place[i].sgrid = off;
-            off += align16(sungrid_bytes(count_of(i)));
+            off += align32(sungrid_bytes(count_of(i)));
         }
     }
     zero_off = off;
     counter_off = off;
-    off += align16(kBatchGroups * sizeof(unsigned long long));
+    off += align32(kBatchGroups * sizeof(unsigned long long));
     res_off = off;
     for (size_t i = 0; i < n; ++i) {
         place[i].stats = off;
@@ -361,12 +362,12 @@ int Batch::layout(int si) {
     const size_t nb = (size_t)nx * ny;
     for (size_t i = 0; i < n; ++i) {
         place[i].counts = off;
-        off += align16(nb * sizeof(uint32_t));
+        off += align32(nb * sizeof(uint32_t));
     }
     zero_bytes = off - zero_off;
     for (size_t i = 0; i < n; ++i) {
         place[i].sun = off;
-        off += align16(sizeof(SunFrame));
+        off += align32(sizeof(SunFrame));
     }
     res_bytes = off - res_off;
     const size_t comp = std::max<size_t>(off - up_bytes, 16);

@@ -47,7 +47,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 
 // The packed records travel to the device as a kernel parameter (no staging copy) and this kernel,
 // which names the array directly, stores them.
-struct alignas(16) RecordBlock {
+struct alignas(32) RecordBlock {
     unsigned char bytes[kOffSun];
 };
 static_assert(sizeof(RecordBlock) % 16 == 0 && sizeof(RecordBlock) <= 4096, "record block must fit a parameter");

@@ -1,6 +1,6 @@
 // csp_types.cuh -- device data layout shared by the host scene builder and the CUDA kernels.
 //
-// Layout in HBM (all arrays 16-byte aligned, read through the read-only path):
+// Layout in HBM (records and boxes 32-byte aligned, read through the read-only path):
 //   Prim   [n]      64 B  geometry of one element in the form its intersection test consumes
 //   Optics [n]      16 B  reflectivity, slope error, specularity error (extension)
 //   Aabb   [n]      32 B  element AABB exactly as the reference hands it to OptiX (float)
@@ -38,7 +38,7 @@ constexpr uint64_t kRayIndexLimit = 1ull << 56;
 //    a = (e1, L1/2)   b = (e2, L2/2)   c = (n = normalize(e2 x e1), curv_x)   d = (rect center, curv_y)
 //  cylinder receiver (Cylinder_Y, cuda/GeometryDataST.h:60-77, cuda/intersection.cu:188-194):
 //    a = (center, radius)   b = (local x, half height)   c = (local y = z x x, radius^2)   d = (local z, 0)
-struct alignas(16) Prim {
+struct alignas(32) Prim {
     float4 a, b, c, d;
 };
 
@@ -46,7 +46,7 @@ struct alignas(16) Optics {
     float reflectivity, slope, spec, pad;
 };
 
-struct alignas(16) Aabb {
+struct alignas(32) Aabb {
     float4 lo;  // xyz, w unused
     float4 hi;
 };
@@ -57,7 +57,7 @@ struct alignas(16) Aabb {
 //   leaf:     hit = kLeafFlag | type << kTypeShift | element index; miss as above.
 // Internal boxes bound every surface below them (sag-inflated for paraboloids); a leaf box is the
 // element's exact AABB, the box whose overlap decides whether the element is tested at all.
-struct alignas(16) Node {
+struct alignas(32) Node {
     float4 lo;
     float4 hi;
 };
