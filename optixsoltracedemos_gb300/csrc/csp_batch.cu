@@ -87,19 +87,6 @@ struct BatchSmem {
     unsigned long long want;
 };
 
-// Drain the queues of the current instance and add its record counters to the instance's totals.
-template <class C>
-__device__ __forceinline__ void finish_instance(BatchSmem<C::kB, C::kAccel>& sm, const Sink& k, int& qs, int& gs) {
-    drain<C>(sm.A, k, sm.core, true, qs, gs);
-    __syncthreads();
-    if (threadIdx.x > 0 && threadIdx.x < 4) {
-        const unsigned long long v = sm.stat[threadIdx.x];
-        if (v) atomicAdd(sm.F.stats + threadIdx.x, v);
-        sm.stat[threadIdx.x] = 0;
-    }
-    __syncthreads();
-}
-
 // Resident threads per SM the register budget is cut for: 1024 for the field kernels (64
 // registers: more warps to hide the grid walk's load latency), 1152 for the element-list kernel
 // (nine 128-thread CTAs, 56 registers: its phases are short latency chains, and it measured 3.5 %
@@ -122,55 +109,78 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
         sm.grab = 0;
     }
     const Sink k{&sm.F, sm.stat};
-    bool have = false;
+    bool have = false;        // an instance is loaded
+    bool flush = false;       // its remaining queued rays first, then its counters
+    bool done = false;        // no tiles left
     uint64_t t0 = 0, t1 = 0;  // tile range of the current instance
-    int qs = 0, gs = 0;       // queue sizes (see drain)
+    uint64_t g = 0, g1 = 0;   // tiles of this CTA's current grab not yet traced
+    int qs = 0, gs = 0;       // queue sizes (see phase_b)
+    __syncthreads();
     for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            // guided grabs: a quarter of an even share of the tiles left (as this CTA last saw
-            // them), at most L.chunk and at least one, so grabs shrink towards single tiles at the
-            // end (a large grab taken last would otherwise run alone).  Large grabs early keep a CTA
-            // on one instance across consecutive grabs: each switch drains its queues in partial
-            // batches.
-            const unsigned long long left = L.total_tiles > sm.grab ? L.total_tiles - sm.grab : 0;
-            const unsigned long long want =
-                max(1ull, min((unsigned long long)L.chunk, left / ((unsigned long long)gridDim.x * 4)));
-            sm.grab = atomicAdd(L.next_tile, want);
-            sm.want = want;
-        }
-        __syncthreads();
-        const uint64_t g0 = sm.grab;
-        if (g0 >= L.total_tiles) break;
-        const uint64_t g1 = min(g0 + (uint64_t)sm.want, L.total_tiles);
-        for (uint64_t g = g0; g < g1; ++g) {
-            if (!have || g < t0 || g >= t1) {
-                // instance of tile g: the last i with tile_begin[i] <= g (empty instances skipped)
-                int lo = 0, hi = L.n_inst - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (__ldg(L.tile_begin + mid) <= g) lo = mid;
-                    else hi = mid - 1;
-                }
-                if (have) finish_instance<C>(sm, k, qs, gs);
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(L.inst + lo);
-                constexpr int kWordsA = sizeof(TraceArgs) / 4, kWordsF = sizeof(FluxTarget) / 4;
-                for (int w = threadIdx.x; w < kWordsA + kWordsF; w += kB) {
-                    if (w < kWordsA) reinterpret_cast<uint32_t*>(&sm.A)[w] = __ldg(src + w);
-                    else reinterpret_cast<uint32_t*>(&sm.F)[w - kWordsA] =
-                        __ldg(src + offsetof(InstanceDesc, flux) / 4 + (w - kWordsA));
-                }
-                __syncthreads();
-                load_instance_smem<C>(sm.A, sm.core);
-                __syncthreads();
-                have = true;
-                t0 = __ldg(L.tile_begin + lo);
-                t1 = __ldg(L.tile_begin + lo + 1);
+        if (phase_b<C>(sm.A, k, sm.core, flush, qs, gs)) continue;
+        if (flush) {
+            // every ray of the instance is through: its record counters to the instance's totals
+            __syncthreads();
+            if (threadIdx.x > 0 && threadIdx.x < 4) {
+                const unsigned long long v = sm.stat[threadIdx.x];
+                if (v) atomicAdd(sm.F.stats + threadIdx.x, v);
+                sm.stat[threadIdx.x] = 0;
             }
-            trace_tile<C>(sm.A, k, sm.core, nullptr, g - t0, qs, gs);
+            if (done) break;
+            flush = have = false;
+            __syncthreads();
         }
+        if (g == g1) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                // guided grabs: a quarter of an even share of the tiles left (as this CTA last saw
+                // them), at most L.chunk and at least one, so grabs shrink towards single tiles at the
+                // end (a large grab taken last would otherwise run alone).  Large grabs early keep a CTA
+                // on one instance across consecutive grabs: each switch drains its queues in partial
+                // batches.
+                const unsigned long long left = L.total_tiles > sm.grab ? L.total_tiles - sm.grab : 0;
+                const unsigned long long want =
+                    max(1ull, min((unsigned long long)L.chunk, left / ((unsigned long long)gridDim.x * 4)));
+                sm.grab = atomicAdd(L.next_tile, want);
+                sm.want = want;
+            }
+            __syncthreads();
+            g = sm.grab;
+            g1 = min(g + (uint64_t)sm.want, L.total_tiles);
+            if (g >= L.total_tiles) {
+                if (!have) break;
+                done = flush = true;
+                continue;
+            }
+        }
+        if (!have || g < t0 || g >= t1) {
+            if (have) {
+                flush = true;
+                continue;
+            }
+            // instance of tile g: the last i with tile_begin[i] <= g (empty instances skipped)
+            int lo = 0, hi = L.n_inst - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(L.tile_begin + mid) <= g) lo = mid;
+                else hi = mid - 1;
+            }
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(L.inst + lo);
+            constexpr int kWordsA = sizeof(TraceArgs) / 4, kWordsF = sizeof(FluxTarget) / 4;
+            for (int w = threadIdx.x; w < kWordsA + kWordsF; w += kB) {
+                if (w < kWordsA) reinterpret_cast<uint32_t*>(&sm.A)[w] = __ldg(src + w);
+                else reinterpret_cast<uint32_t*>(&sm.F)[w - kWordsA] =
+                    __ldg(src + offsetof(InstanceDesc, flux) / 4 + (w - kWordsA));
+            }
+            __syncthreads();
+            load_instance_smem<C>(sm.A, sm.core);
+            __syncthreads();
+            have = true;
+            t0 = __ldg(L.tile_begin + lo);
+            t1 = __ldg(L.tile_begin + lo + 1);
+        }
+        trace_tile<C>(sm.A, k, sm.core, nullptr, g++ - t0, qs, gs);
     }
-    if (have) finish_instance<C>(sm, k, qs, gs);
 }
 
 template <int kB, int kAccel>

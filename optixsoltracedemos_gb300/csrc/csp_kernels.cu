@@ -61,7 +61,7 @@ constexpr int trace_min_blocks() {
 // a tile.  Guided grabs measured 27.5 ms per 268M rays of the 10,000-heliostat field against
 // 30.3 ms round robin (a CTA's tiles differ much in work, so round robin ends in a long tail), and
 // 0.325 against 0.328 ms per 16M rays of the single parabolic heliostat.
-constexpr unsigned long long kTraceGrab = 64;
+constexpr uint32_t kTraceGrab = 64;
 
 template <int kAccel>
 __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace_kernel(
@@ -79,32 +79,40 @@ __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace
     }
     __syncthreads();
     const Sink none{nullptr, nullptr};
-    const uint64_t tiles = (A.count + kTraceBlock - 1) / kTraceBlock;
+    // 32-bit tile indices: launch_trace_t takes fewer than 2^31 tiles
+    const uint32_t tiles = (uint32_t)((A.count + kTraceBlock - 1) / kTraceBlock);
+    __shared__ unsigned long long s_grab;
+    __shared__ uint32_t s_want;
+    const bool guided = A.tile_counter != nullptr;
+    // this CTA's tiles: [g, g1) of its current grab, or g, g + gridDim.x, ... below g1
+    uint32_t g = guided ? 0u : blockIdx.x, g1 = guided ? 0u : tiles;
+    bool flush = false;  // no tiles left: the remaining queued rays
     int qs = 0, gs = 0;
-    if (A.tile_counter) {
-        __shared__ unsigned long long s_grab, s_want;
-        unsigned long long seen = 0;  // end of this CTA's last grab (thread 0's estimate of the rest)
-        for (;;) {
-            if (threadIdx.x == 0) {
-                const unsigned long long left = tiles > seen ? tiles - seen : 0;
-                const unsigned long long want =
-                    max(1ull, min(kTraceGrab, left / ((unsigned long long)gridDim.x * 4)));
-                s_grab = atomicAdd(A.tile_counter, want);
-                s_want = want;
+    for (;;) {
+        if (phase_b<C>(A, none, sm.core, flush, qs, gs)) continue;
+        if (flush) break;
+        if (g >= g1) {
+            if (guided && g1 < tiles) {
+                if (threadIdx.x == 0) {
+                    // the rest as of this CTA's last grab
+                    const uint32_t want = max(1u, min(kTraceGrab, (tiles - g1) / (gridDim.x * 4)));
+                    s_grab = atomicAdd(A.tile_counter, (unsigned long long)want);
+                    s_want = want;
+                }
+                __syncthreads();
+                // every thread reads the grab before thread 0 can write the next one: each tile has
+                // CTA barriers, and a grab past the end is the last
+                g = (uint32_t)min(s_grab, (unsigned long long)tiles);
+                g1 = min(g + min(s_want, tiles - g), tiles);
             }
-            __syncthreads();
-            // every thread reads the grab before thread 0 can write the next one: trace_tile has
-            // CTA barriers, and a grab past the end ends the loop in every thread
-            const uint64_t g0 = s_grab, g1 = min((uint64_t)(g0 + s_want), tiles);
-            if (g0 >= tiles) break;
-            seen = g1;
-            for (uint64_t tile = g0; tile < g1; ++tile) trace_tile<C>(A, none, sm.core, &sm.stage, tile, qs, gs);
+            if (g >= g1) {
+                flush = true;
+                continue;
+            }
         }
-    } else {
-        for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-            trace_tile<C>(A, none, sm.core, &sm.stage, tile, qs, gs);
+        trace_tile<C>(A, none, sm.core, &sm.stage, g, qs, gs);
+        g += guided ? 1u : gridDim.x;
     }
-    drain<C>(A, none, sm.core, true, qs, gs);
 }
 
 template <int kAccel>
@@ -126,6 +134,7 @@ cudaError_t launch_trace_t(const TraceArgs& args, cudaStream_t stream) {
                                                           sizeof(TraceSmem<kAccel>));
     if (e != cudaSuccess) return e;
     const uint64_t tiles = (args.count + kTraceBlock - 1) / kTraceBlock;  // CTAs that have work
+    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // 44 TB of records
     const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)std::max(1, sms * std::max(1, per_sm)));
     typename PlainCfg<kAccel>::Args a;
     static_cast<TraceArgs&>(a) = args;

@@ -155,11 +155,16 @@ __device__ __forceinline__ U coherent_order_t(U kk, U count) {
 }
 
 // Launches of fewer than 2^32 rays (all but the largest) take the 32-bit form: the same
-// arithmetic, without the cost of 64-bit division by the block sizes.
+// arithmetic, without the cost of 64-bit division by the block sizes, whose code stays out of line.
+template <bool kFine, int G>
+__device__ __noinline__ uint64_t coherent_order_far(uint64_t kk, uint64_t count) {
+    return coherent_order_t<kFine, G, uint64_t>(kk, count);
+}
+
 template <bool kFine, int G>
 __device__ __forceinline__ uint64_t coherent_order(uint64_t kk, uint64_t count) {
     if (count <= 0xFFFFFFFFull) return coherent_order_t<kFine, G, uint32_t>((uint32_t)kk, (uint32_t)count);
-    return coherent_order_t<kFine, G, uint64_t>(kk, count);
+    return coherent_order_far<kFine, G>(kk, count);
 }
 
 // ------------------------------------------------------------------------------ sun plane -----
@@ -324,7 +329,7 @@ __device__ __forceinline__ float halton2(uint64_t i) {
     return r;
 }
 
-__device__ __forceinline__ float halton3(uint64_t i) {
+__device__ __noinline__ float halton3(uint64_t i) {
     float r = 0.0f;
     int k = 0;
     while (i >= (1ull << 32)) {
@@ -728,17 +733,23 @@ __device__ __forceinline__ int sun_closest(const SunGrid& G, const Prim* __restr
     uint32_t j = range.x;
     const uint32_t e = range.y;
     if (!CSP_BOUNDS(5, j <= e && e <= (uint32_t)G.n_items)) return best;
-    for (; j < e; ++j) {
-        if (!in_rect(__ldg(G.item_rect + j), u, v)) continue;
+    // the cell's items, then the global list (one test site)
+    for (int k = 0;;) {
+        float4 r;
+        const Aabb* box;
+        if (j < e) {
+            r = __ldg(G.item_rect + j);
+            box = G.item_box + j++;
+        } else if (k < G.n_global) {
+            const uint32_t id = __ldg(G.global_id + k++);
+            r = __ldg(G.rect + id);
+            box = G.aabbs + id;
+        } else {
+            break;
+        }
+        if (!in_rect(r, u, v)) continue;
         float4 lo, hi;
-        ldg32(G.item_box + j, lo, hi);
-        test_box(lo, hi, prims, o, d, inv, kTminSun, acc, best, best_t, best_type, prune);
-    }
-    for (int k = 0; k < G.n_global; ++k) {
-        const uint32_t id = __ldg(G.global_id + k);
-        if (!in_rect(__ldg(G.rect + id), u, v)) continue;
-        float4 lo, hi;
-        ldg32(G.aabbs + id, lo, hi);
+        ldg32(box, lo, hi);
         test_box(lo, hi, prims, o, d, inv, kTminSun, acc, best, best_t, best_type, prune);
     }
     return best;
@@ -1134,33 +1145,29 @@ __device__ __forceinline__ void push(Core& sm, bool want, uint64_t ray, float3 o
     }
 }
 
-// Remainder of a path in phase B, from the closest hit `h` of segment `g`: record, shade, next
-// segment, until the ray misses, is absorbed, ends on the receiver or reaches the depth limit.
-// pending: `h` is a mirror hit whose record was already emitted (phase A), shading comes next.
+// A queued path of an element-list launch, from its first segment `g` with candidate mask `m`: closest
+// hit, record, shade, next segment, until the ray misses, is absorbed, ends on the receiver or reaches
+// the depth limit.
 template <class C>
-__device__ void finish_path(const typename C::Args& A, const Sink& k, const typename C::Core& sm, uint64_t ray, Segment g,
-                            Hit h, bool pending) {
+__device__ __forceinline__ void flat_path(const typename C::Args& A, const Sink& k, const typename C::Core& sm,
+                                          uint64_t ray, Segment g, uint32_t m) {
+    // the first segment's search on its own: in one copy inside the loop the kernel spills (16 M rays
+    // of the single parabolic heliostat: 381 us against 313)
+    Hit h;
+    h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
     for (;;) {
         if (h.best < 0) return;  // __miss__ms, cuda/materials.cu:236-253
-        const Prim p = C::kFlat ? sm.flat.prim[h.best] : load_prim(A.prims, (uint32_t)h.best);
-        if (!pending) {
-            float4 rec;
-            int slot;
-            const bool mirror = classify(p, g, h, rec, slot);
-            if (slot >= 0) emit<C>(A, k, ray, slot, rec, (uint32_t)h.best);
-            if (!mirror) return;
-        }
-        pending = false;
-        const Optics op = C::kFlat ? sm.flat.optics[h.best] : A.optics[h.best];
+        const Prim p = sm.flat.prim[h.best];
+        float4 rec;
+        int slot;
+        const bool mirror = classify(p, g, h, rec, slot);
+        if (slot >= 0) emit<C>(A, k, ray, slot, rec, (uint32_t)h.best);
+        if (!mirror) return;
         Segment next;
-        if (!shade_mirror<C>(A, ray, p, op, g, h, next)) return;
+        if (!shade_mirror<C>(A, ray, p, sm.flat.optics[h.best], g, h, next)) return;
         g = next;
-        if (C::kFlat) {
-            const uint32_t m = candidates(sm.flat, g.o, g.d, g.tmin);
-            h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
-        } else {
-            h.best = find_closest<C>(A, sm, g.o, g.d, g.tmin, kNoElement, h.t, h.type);
-        }
+        m = candidates(sm.flat, g.o, g.d, g.tmin);
+        h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
     }
 }
 
@@ -1208,15 +1215,9 @@ __device__ __forceinline__ int bounce_batch(const typename C::Args& A, const Sin
         if (threadIdx.x == 0) sm.qsize = base;
         __syncthreads();
         if (have) {
-            if (C::kFlat) {
-                // first segment from the sun: intersection programs of the candidate elements
-                const Segment g{o, d, kTminSun, 0};
-                Hit h;
-                h.best = closest_in(sm.flat, w, o, d, kTminSun, (sm.sun.shape & 2) != 0, h.t, h.type);
-                finish_path<C>(A, k, sm, ray, g, h, false);
-            }
+            if constexpr (C::kFlat) flat_path<C>(A, k, sm, ray, Segment{o, d, kTminSun, 0}, w);
         }
-        if (!C::kFlat) {
+        if constexpr (!C::kFlat) {
             // one bounce per batch: shade the pending mirror hit (its record is out), find the next
             // hit, record it, and queue it again when it is another mirror below the depth limit
             bool again = false;
@@ -1281,25 +1282,28 @@ __device__ __forceinline__ void gen_batch(const typename C::Args& A, const Sink&
     gs = base;
 }
 
-// Phase B: run full batches of queued rays (all = also the remainders).  The bounce queue is below
-// kB before each generation batch (a bounce batch never grows it), so neither queue exceeds 2 kB.  qs and gs
-// are the sizes of the bounce and generation queues, carried in registers by every thread of the
-// CTA (equal in all of them); the caller has passed a barrier since the last append.
+// Phase B: one full batch of queued rays, or with `flush` one of what remains; false when there is
+// none.  The bounce queue is below kB before each generation batch (a bounce batch never grows it), so
+// neither queue exceeds 2 kB.  qs and gs are the sizes of the bounce and generation queues, carried in
+// registers by every thread of the CTA (equal in all of them); the caller has passed a barrier since
+// the last append.
+// The kernels call this and trace_tile from one place each, in one loop: with a copy of the batches
+// behind every tile loop and every drain the field kernel was 163 KB of code, and its warps waited
+// for instructions wherever they left each other's phase.
 template <class C>
-__device__ void drain(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool all, int& qs, int& gs) {
-    for (;;) {
-        if (qs >= C::kB || (all && qs > 0 && gs == 0)) {
-            qs = bounce_batch<C>(A, k, sm, qs);
-            continue;
-        }
-        if constexpr (C::kFlat) {
-            if (gs >= C::kB || (all && gs > 0)) {
-                gen_batch<C>(A, k, sm, gs, qs);
-                continue;
-            }
-        }
-        break;
+__device__ __forceinline__ bool phase_b(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool flush,
+                                        int& qs, int& gs) {
+    if (qs >= C::kB || (flush && qs > 0 && gs == 0)) {
+        qs = bounce_batch<C>(A, k, sm, qs);
+        return true;
     }
+    if constexpr (C::kFlat) {
+        if (gs >= C::kB || (flush && gs > 0)) {
+            gen_batch<C>(A, k, sm, gs, qs);
+            return true;
+        }
+    }
+    return false;
 }
 
 // Per-CTA setup of an instance: sun frame and the kFlat element list or the grid descriptors into
@@ -1390,12 +1394,11 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
     }
     // the barrier before the bounce batches counts this tile's appends
     qs += __syncthreads_count(again);
-    while (qs >= C::kB) qs = bounce_batch<C>(A, k, sm, qs);
 }
 
-// Phase A of one tile (rays A.ray_begin + tile * kB ...) followed by phase B on full batches.
+// Phase A of one tile (rays A.ray_begin + tile * kB ...); phase_b runs its full batches.
 // `stage` is the kDense staging area of element-list launches (unused otherwise); qs, gs: the queue
-// sizes (see drain).
+// sizes (see phase_b).
 template <class C>
 __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink& k, typename C::Core& sm,
                                            typename C::Stage* stage, uint64_t tile, int& qs, int& gs) {
@@ -1456,7 +1459,6 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
     }
     // the barrier before phase B counts this tile's appends to the generation queue
     gs += __syncthreads_count(want);
-    drain<C>(A, k, sm, false, qs, gs);
 }
 
 }  // namespace
