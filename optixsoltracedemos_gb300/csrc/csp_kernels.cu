@@ -257,6 +257,15 @@ __global__ void __launch_bounds__(kCompactBlock) compact_write_kernel(const floa
 __global__ void __launch_bounds__(256) halton3_table_kernel(float* __restrict__ t) {
     const uint32_t m = blockIdx.x * 256u + threadIdx.x;
     if (m < kH3T12) t[m] = halton3(m);
+    if (m < kH3Tail) {
+        uint32_t j = m;
+        for (uint32_t k = 0; k < 8; ++k) {
+            const uint32_t q = j / 3u;
+            t[kH3TailAt + 8 * m + k] =
+                k < kH3TailDigits ? c_halton3_f[kH3T12Digits + k] * (float)(j - 3u * q) : 0.0f;
+            j = q;
+        }
+    }
 }
 
 }  // namespace
@@ -275,7 +284,7 @@ const float* halton3_table() {
     if (!tried[dev]) {
         tried[dev] = true;
         float* t = nullptr;
-        if (dev_alloc((void**)&t, kH3T12 * sizeof(float)) == cudaSuccess) {
+        if (dev_alloc((void**)&t, (kH3TailAt + 8 * kH3Tail) * sizeof(float)) == cudaSuccess) {
             halton3_table_kernel<<<(kH3T12 + 255) / 256, 256>>>(t);
             if (cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess) tables[dev] = t;
             else cudaFree(t);

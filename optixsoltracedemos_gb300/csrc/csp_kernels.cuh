@@ -55,8 +55,9 @@ struct TraceArgsK : TraceArgs {
     uint32_t keys[20];
 };
 
-// Device table of the base-3 Halton fold after its first 12 digits, t[m] = the reference loop's
-// sum for m < 3^12 (2.1 MB, filled once per device by the same loop), or nullptr if it could not be
+// Device table of the base-3 Halton fold: its sums after 12 digits, t[m] = the reference loop's sum
+// for m < 3^12, and the addends of the next six (2.1 MB, filled once per device by the same loop), or
+// nullptr if it could not be
 // made.  Thread-safe; the calling thread's current device.
 const float* halton3_table();
 

@@ -312,6 +312,21 @@ __device__ void sun_frame_state(const Aabb* __restrict__ aabbs, int n, float3 s,
     *out = f;
 }
 
+// 32-byte accesses (p 32-byte aligned).  Lanes on different records of a scene, or on different
+// rows of the hit buffer, touch a cache line per access and lane: half as many accesses is half the
+// time in the L1 pipe, which was 56 % busy in the field kernel with 16-byte ones (64M rays over 10,000
+// heliostats 5855 -> 5461 us, 3M rays over 1,000 focused ones with ids 256 -> 230 us).
+__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+__device__ __forceinline__ void stg32(void* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 // ------------------------------------------------------------------------------ sampling ------
 // Halton radical inverse, cuda/sun.cu:16-24: f /= b; r += f * (i mod b); i /= b, in float.
 // The loop's partial sum after its first 24 digits (the low 24 bits of i) is a dyadic fraction of
@@ -346,23 +361,37 @@ __device__ __noinline__ float halton3(uint64_t i) {
     return r;
 }
 
-// Same fold with its first steps looked up: t6[m] = halton3(m) for m < 3^6 (shared memory) or
-// t12[m] = halton3(m) for m < 3^12 (global table, when present).  The partial sum of the reference
-// loop after k digits depends only on i mod 3^k and equals halton3(i mod 3^k) (a zero digit adds +0,
-// which leaves the sum unchanged); for larger i the loop continues from exactly that sum with digit
-// k + 1, so the result is identical bit for bit.
+// Same fold with its steps looked up: t6[m] = halton3(m) for m < 3^6 (shared memory) or, when the
+// device table is present, t12[m] = halton3(m) for m < 3^12 followed by the next six digits' addends.
+// The partial sum of the reference loop after k digits depends only on i mod 3^k and equals
+// halton3(i mod 3^k) (a zero digit adds +0, which leaves the sum unchanged); for larger i the loop
+// continues from exactly that sum with digit k + 1, so the result is identical bit for bit.  The
+// addends of digits 13 to 18 are the loop's products f_k digit, one 32-byte entry per value of those
+// digits (23 KB, in L1): the loop's division, conversion and multiplication per digit left every ray
+// of 16 M ray runs about 35 instructions.
 constexpr uint32_t kH3T12Digits = 12, kH3T12 = 531441;
+constexpr uint32_t kH3TailDigits = 6, kH3Tail = 729;
+constexpr uint32_t kH3TailAt = (kH3T12 + 7) / 8 * 8;  // the addends' place behind t12, 8 floats each
 __device__ __forceinline__ float halton3_tab(uint64_t i, const float* __restrict__ t6, const float* __restrict__ t12) {
     if (i >= (1ull << 32)) return halton3(i);
     uint32_t j = (uint32_t)i;
     float r;
     int k;
     if (t12) {
-        const uint32_t q = j / kH3T12;
+        uint32_t q = j / kH3T12;
         if (!CSP_BOUNDS(7, j - kH3T12 * q < kH3T12)) return 0.0f;
         r = __ldg(t12 + (j - kH3T12 * q));
-        k = kH3T12Digits;
-        j = q;
+        if (q == 0) return r;
+        j = q / kH3Tail;
+        float4 a, b;
+        ldg32(t12 + kH3TailAt + 8 * (q - kH3Tail * j), a, b);
+        r = r + a.x;
+        r = r + a.y;
+        r = r + a.z;
+        r = r + a.w;
+        r = r + b.x;
+        r = r + b.y;
+        k = kH3T12Digits + kH3TailDigits;
     } else {
         const uint32_t q = j / kH3Tab;
         r = t6[j - kH3Tab * q];
@@ -519,21 +548,6 @@ __device__ __forceinline__ bool hit_prim(uint32_t type, const Prim& p, float3 o,
     if (type == kParabolicMirror) return hit_parab(p, o, d, tmin, t);
     if (type == kCylReceiver) return hit_cyl(p, o, d, tmin, acc, t);
     return hit_flat(p, o, d, tmin, t);
-}
-
-// 32-byte accesses (p 32-byte aligned).  Lanes on different records of a scene, or on different
-// rows of the hit buffer, touch a cache line per access and lane: half as many accesses is half the
-// time in the L1 pipe, which was 56 % busy in the field kernel with 16-byte ones (64M rays over 10,000
-// heliostats 5855 -> 5461 us, 3M rays over 1,000 focused ones with ids 256 -> 230 us).
-__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
-}
-__device__ __forceinline__ void stg32(void* p, float4 a, float4 b) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
-                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-                 : "memory");
 }
 
 __device__ __forceinline__ Prim load_prim(const Prim* prims, uint32_t i) {
