@@ -528,7 +528,7 @@ void Batch::fill_descs(const int* block, const std::vector<bool>* sample, std::v
         d.args.count = rays;
         d.args.seed = b.seed;
         d.args.instance = b.instance;
-        d.args.pad = 0;
+        d.args.n_prims = (int)count_of(i);
         d.args.grid = nullptr;
         d.args.h3t12 = h3t12;
         d.args.sgrid = nullptr;

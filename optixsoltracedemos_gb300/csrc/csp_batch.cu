@@ -114,10 +114,10 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
     bool done = false;        // no tiles left
     uint64_t t0 = 0, t1 = 0;  // tile range of the current instance
     uint64_t g = 0, g1 = 0;   // tiles of this CTA's current grab not yet traced
-    int qs = 0, gs = 0;       // queue sizes (see phase_b)
+    int qs = 0;               // queue size (see phase_b)
     __syncthreads();
     for (;;) {
-        if (phase_b<C>(sm.A, k, sm.core, flush, qs, gs)) continue;
+        if (phase_b<C>(sm.A, k, sm.core, flush, qs)) continue;
         if (flush) {
             // every ray of the instance is through: its record counters to the instance's totals
             __syncthreads();
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
             t0 = __ldg(L.tile_begin + lo);
             t1 = __ldg(L.tile_begin + lo + 1);
         }
-        trace_tile<C>(sm.A, k, sm.core, nullptr, g++ - t0, qs, gs);
+        trace_tile<C>(sm.A, k, sm.core, nullptr, g++ - t0, qs);
     }
 }
 

@@ -250,9 +250,12 @@ int System::initialize() {
     const auto t0 = std::chrono::steady_clock::now();
     int rc = ensure_streams();
     if (rc) return rc;
-    if (!d_tile_counter &&
-        (rc = cuda_status(dev_alloc((void**)&d_tile_counter, sizeof(unsigned long long)), "cudaMalloc tile counter")))
-        return rc;
+    if (!d_tile_counter) {
+        if ((rc = cuda_status(dev_alloc((void**)&d_tile_counter, 2 * sizeof(unsigned int)), "cudaMalloc tile counter")))
+            return rc;
+        // zero before the first launch; every launch leaves it so
+        if ((rc = cuda_status(cudaMemsetAsync(d_tile_counter, 0, 2 * sizeof(unsigned int), stream), "memset"))) return rc;
+    }
     h3t12 = halton3_table();
     std::string err;
     if ((rc = build_elements(elements.data(), (uint32_t)elements.size(), scene, err))) return fail(rc, err);
@@ -306,7 +309,7 @@ TraceArgs System::args(uint64_t begin, uint64_t count) const {
     a.count = count;
     a.seed = seed;
     a.instance = instance;
-    a.pad = 0;
+    a.n_prims = (int)scene.prims.size();
     a.grid = grid.valid ? d_grid : nullptr;
     a.h3t12 = h3t12;
     a.sgrid = scene.prims.size() > kFlatListMax && d_sgrid ? sgjob_host.desc : nullptr;
@@ -320,7 +323,7 @@ int System::trace_async(cudaStream_t st) {
     if (rc) return rc;
     // it writes the hit buffer: it never overlaps the handle's other launches, so the tile counter
     // serves it on any stream
-    return cuda_status(launch_trace(args(0, num_rays), (int)scene.prims.size(), st ? st : stream), "trace_kernel");
+    return cuda_status(launch_trace(args(0, num_rays), st ? st : stream), "trace_kernel");
 }
 
 int System::run() {
@@ -329,7 +332,7 @@ int System::run() {
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     if ((rc = cuda_status(cudaEventRecord(ev0, stream), "cudaEventRecord"))) return rc;
-    if ((rc = cuda_status(launch_trace(args(0, num_rays), (int)scene.prims.size(), stream), "trace_kernel"))) return rc;
+    if ((rc = cuda_status(launch_trace(args(0, num_rays), stream), "trace_kernel"))) return rc;
     if ((rc = cuda_status(cudaEventRecord(ev1, stream), "cudaEventRecord"))) return rc;
     if ((rc = cuda_status(cudaEventSynchronize(ev1), "trace"))) return rc;
     float ms = 0.f;
@@ -348,7 +351,7 @@ int System::run_to_host(float* dst, uint32_t* ids_dst) {
     const auto t0 = std::chrono::steady_clock::now();
     for (uint64_t b = 0; b < num_rays; b += chunk) {
         const uint64_t c = std::min(chunk, num_rays - b);
-        if ((rc = cuda_status(launch_trace(args(b, c), (int)scene.prims.size(), stream), "trace_kernel"))) break;
+        if ((rc = cuda_status(launch_trace(args(b, c), stream), "trace_kernel"))) break;
         cudaEvent_t ev;
         if ((rc = cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate"))) break;
         done.push_back(ev);
@@ -402,7 +405,7 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
         cap_compact_rays = n;
     }
     const auto t0 = std::chrono::steady_clock::now();
-    if ((rc = cuda_status(launch_trace(args(0, n), (int)scene.prims.size(), stream), "trace_kernel"))) return rc;
+    if ((rc = cuda_status(launch_trace(args(0, n), stream), "trace_kernel"))) return rc;
     if ((rc = cuda_status(launch_compact_count(d_hits, n, d_ccounts, d_csums, stream), "compact_count_kernel")))
         return rc;
     unsigned long long total = 0;
@@ -690,7 +693,7 @@ int csp_trace_into(csp_handle h, void* hits, void* ids, uint64_t first, uint64_t
     a.count = count;
     cudaStream_t st = stream ? reinterpret_cast<cudaStream_t>(stream) : s->stream;
     if (st != s->stream) a.tile_counter = nullptr;  // may overlap the launches on the handle's stream
-    return csp::cuda_status(csp::launch_trace(a, (int)s->scene.prims.size(), st), "trace_kernel");
+    return csp::cuda_status(csp::launch_trace(a, st), "trace_kernel");
 }
 
 int csp_run_to_host_compact(csp_handle h, float* points, uint8_t* counts, float* records, uint64_t capacity,

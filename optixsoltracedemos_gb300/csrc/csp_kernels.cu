@@ -24,7 +24,7 @@
 namespace csp {
 namespace {
 
-constexpr int kTraceBlock = 256;
+constexpr int kTraceBlock = 128;
 constexpr int kFluxBlock = 256;
 
 template <int kCluster>
@@ -44,32 +44,39 @@ struct TraceSmem {
     typename PlainCfg<kAccel>::Core core;
 };
 
-// Resident 256-thread CTAs per SM the register budget is cut for: four (64 registers, 1,024
-// threads) -- more warps to cover the record stream of the element-list kernel and the dependent
-// loads of the candidate and cell lists of the others (64 registers measured faster than 72 or 77
-// for every kernel); 256-thread CTAs instead of eight of 128: the 10,000-heliostat field 32.05 ->
-// 30.23 ms per 268M rays, the single parabolic heliostat 0.3305 -> 0.3283 ms per 16M (two of 512:
-// 30.4 and 0.347 ms).
+// Resident CTAs per SM the register budget is cut for: eight of 128 threads (64 registers, 1,024
+// threads), more warps to cover the record stream of the element-list kernel and the dependent loads
+// of the candidate and cell lists of the others.  Four of 256 threads, with the barriers of a tile over
+// twice the warps: the 10,000-heliostat field 5170 against 5069 us per 64M rays, the single parabolic
+// heliostat 302 against 287 us per 16M; ten of 128 (48 registers, spills) 299 us, two of 512 322 us.
 template <int kAccel>
 constexpr int trace_min_blocks() {
-    return 4;
+    return 1024 / kTraceBlock;
 }
 
-// Persistent kernel over the tiles of one launch; dense records out.  With a tile counter the CTAs
-// take guided grabs (a quarter of an even share of the tiles left, at most kTraceGrab, shrinking to
-// single tiles at the end), else static round robin.  The records do not depend on which CTA traces
-// a tile.  Guided grabs measured 27.5 ms per 268M rays of the 10,000-heliostat field against
-// 30.3 ms round robin (a CTA's tiles differ much in work, so round robin ends in a long tail), and
-// 0.325 against 0.328 ms per 16M rays of the single parabolic heliostat.
-constexpr uint32_t kTraceGrab = 64;
+// Persistent kernel over the tiles of one launch; dense records out.  With a tile counter every CTA
+// starts on a share of its own (half of an even share for element lists, a quarter for fields, whose
+// tiles differ much in work) and then takes guided grabs (a quarter of an even share of the tiles
+// left, shrinking to single tiles at the end), each requested while the last tile of the one before is
+// traced; grabs and shares are at most kTraceGrab tiles, so that the CTAs work on the same stretch of
+// the sun plane and share its scene data in L2 (the field at caps of 2 / 4 / 8 / 16 / 32 / 64 tiles:
+// 4887 / 4855 / 4857 / 4893 / 4992 / 5070 us per 64M rays).  Without a counter: one contiguous even share
+// (element lists: the next tile's Halton sums are prefetched) or round robin (fields).  The records
+// do not depend on which CTA traces a tile.  Guided grabs measured 27.5 ms per 268M rays of the
+// 10,000-heliostat field against 30.3 ms round robin (a CTA's tiles differ much in work, so round robin
+// ends in a long tail).
+constexpr uint32_t kTraceGrab = 8;
 
 template <int kAccel>
 __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace_kernel(
     const typename PlainCfg<kAccel>::Args A) {
     using C = PlainCfg<kAccel>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     TraceSmem<kAccel>& sm = *reinterpret_cast<TraceSmem<kAccel>*>(smem_raw);
     load_instance_smem<C>(A, sm.core);
+    if constexpr (C::kFlat)
+        for (int i = threadIdx.x; i < kTraceBlock * kMaxDepth; i += kTraceBlock)
+            sm.stage.row[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // the shared-memory Halton table serves only launches without the device-wide 3^12 table
     if (!A.h3t12)
         for (uint32_t m = threadIdx.x; m < kH3Tab; m += kTraceBlock) sm.core.t6[m] = halton3(m);
@@ -81,68 +88,85 @@ __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace
     const Sink none{nullptr, nullptr};
     // 32-bit tile indices: launch_trace_t takes fewer than 2^31 tiles
     const uint32_t tiles = (uint32_t)((A.count + kTraceBlock - 1) / kTraceBlock);
-    __shared__ unsigned long long s_grab;
-    __shared__ uint32_t s_want;
+    __shared__ uint32_t s_grab;
     const bool guided = A.tile_counter != nullptr;
-    // this CTA's tiles: [g, g1) of its current grab, or g, g + gridDim.x, ... below g1
-    uint32_t g = guided ? 0u : blockIdx.x, g1 = guided ? 0u : tiles;
+    // this CTA's tiles: g, g + step, ... below g1; the counter hands out those from `base` on
+    uint32_t g, g1, step = 1, base = 0;
+    if (guided) {
+        const uint32_t share = max(1u, min(kTraceGrab, tiles / gridDim.x / (C::kFlat ? 2u : 4u)));
+        base = share * gridDim.x;
+        g = share * blockIdx.x;
+        g1 = g + share;
+    } else if (C::kFlat) {
+        g = (uint32_t)((uint64_t)tiles * blockIdx.x / gridDim.x);
+        g1 = (uint32_t)((uint64_t)tiles * (blockIdx.x + 1) / gridDim.x);
+    } else {
+        g = blockIdx.x;
+        g1 = tiles;
+        step = gridDim.x;
+    }
     bool flush = false;  // no tiles left: the remaining queued rays
-    int qs = 0, gs = 0;
+    int qs = 0;          // queue size (see phase_b)
     for (;;) {
-        if (phase_b<C>(A, none, sm.core, flush, qs, gs)) continue;
+        if (phase_b<C>(A, none, sm.core, flush, qs)) continue;
         if (flush) break;
         if (g >= g1) {
-            if (guided && g1 < tiles) {
-                if (threadIdx.x == 0) {
-                    // the rest as of this CTA's last grab
-                    const uint32_t want = max(1u, min(kTraceGrab, (tiles - g1) / (gridDim.x * 4)));
-                    s_grab = atomicAdd(A.tile_counter, (unsigned long long)want);
-                    s_want = want;
-                }
-                __syncthreads();
-                // every thread reads the grab before thread 0 can write the next one: each tile has
-                // CTA barriers, and a grab past the end is the last
-                g = (uint32_t)min(s_grab, (unsigned long long)tiles);
-                g1 = min(g + min(s_want, tiles - g), tiles);
-            }
-            if (g >= g1) {
-                flush = true;
-                continue;
-            }
+            flush = true;
+            continue;
         }
-        trace_tile<C>(A, none, sm.core, &sm.stage, g, qs, gs);
-        g += guided ? 1u : gridDim.x;
+        const bool last = guided && g + 1 == g1;
+        uint32_t want = 0, at = 0;
+        if (last) {
+            // tiles left as far as this CTA knows
+            const uint32_t left = tiles - min(max(g1, base), tiles);
+            want = max(1u, min(kTraceGrab, left / (gridDim.x * 4)));
+            if (threadIdx.x == 0) at = atomicAdd(A.tile_counter, want);
+        }
+        trace_tile<C>(A, none, sm.core, &sm.stage, g, qs);
+        g += step;
+        if (last) {
+            // the tile's barrier lies between the reads of the last grab and this write
+            if (threadIdx.x == 0) s_grab = at;
+            __syncthreads();
+            g = min(base + s_grab, tiles);
+            g1 = min(g + want, tiles);
+        }
+    }
+    // the last CTA leaves the counter as it found it
+    if (guided && threadIdx.x == 0 && atomicAdd(A.tile_counter + 1, 1u) == gridDim.x - 1) {
+        A.tile_counter[0] = 0u;
+        A.tile_counter[1] = 0u;
     }
 }
 
 template <int kAccel>
 cudaError_t launch_trace_t(const TraceArgs& args, cudaStream_t stream) {
-    // persistent grid: every resident CTA slot of the device, never more CTAs than tiles
-    int dev = 0, sms = 0, per_sm = 0;
+    // persistent grid: every resident CTA slot of the device (found once per device; devices past 63
+    // each time), never more CTAs than tiles
+    static std::atomic<int> slots_of[64];
+    int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // the attribute is set once per device (bit `dev` of the mask; devices past 63 set it every time)
-    static std::atomic<unsigned long long> attr_set{0};
-    const unsigned long long bit = (dev >= 0 && dev < 64) ? 1ull << dev : 0ull;
-    if (e == cudaSuccess && !(bit && (attr_set.load(std::memory_order_acquire) & bit))) {
-        e = cudaFuncSetAttribute(trace_kernel<kAccel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(TraceSmem<kAccel>));
-        if (e == cudaSuccess) attr_set.fetch_or(bit, std::memory_order_acq_rel);
-    }
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kAccel>, kTraceBlock,
-                                                          sizeof(TraceSmem<kAccel>));
     if (e != cudaSuccess) return e;
+    int slots = dev < 64 ? slots_of[dev].load(std::memory_order_acquire) : 0;
+    if (slots == 0) {
+        int sms = 0, per_sm = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(trace_kernel<kAccel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(TraceSmem<kAccel>));
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kAccel>, kTraceBlock,
+                                                              sizeof(TraceSmem<kAccel>));
+        if (e != cudaSuccess) return e;
+        slots = std::max(1, sms * std::max(1, per_sm));
+        if (dev < 64) slots_of[dev].store(slots, std::memory_order_release);
+    }
     const uint64_t tiles = (args.count + kTraceBlock - 1) / kTraceBlock;  // CTAs that have work
     if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // 44 TB of records
-    const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)std::max(1, sms * std::max(1, per_sm)));
+    const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)slots);
     typename PlainCfg<kAccel>::Args a;
     static_cast<TraceArgs&>(a) = args;
     if constexpr (PlainCfg<kAccel>::kSched) philox_keys(args.seed, a.keys);
-    if (args.tile_counter) {
-        e = cudaMemsetAsync(args.tile_counter, 0, sizeof(unsigned long long), stream);
-        if (e != cudaSuccess) return e;
-    }
     trace_kernel<kAccel><<<(unsigned)grid, kTraceBlock, sizeof(TraceSmem<kAccel>), stream>>>(a);
     return cudaGetLastError();
 }
@@ -305,9 +329,9 @@ cudaError_t launch_prepare_sun(const Aabb* aabbs, int n, float sx, float sy, flo
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace(const TraceArgs& args, int n_prims, cudaStream_t stream) {
+cudaError_t launch_trace(const TraceArgs& args, cudaStream_t stream) {
     if (args.count == 0) return cudaSuccess;
-    if (n_prims <= kFlatMax) return launch_trace_t<kAccelFlat>(args, stream);
+    if (args.n_prims <= kFlatMax) return launch_trace_t<kAccelFlat>(args, stream);
     if (!args.sgrid) return cudaErrorInvalidValue;  // scenes above the element list need their sun grid
     if (args.grid) return launch_trace_t<kAccelGrid>(args, stream);
     return launch_trace_t<kAccelBvh>(args, stream);

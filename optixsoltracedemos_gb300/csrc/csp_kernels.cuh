@@ -39,14 +39,14 @@ struct TraceArgs {
     uint64_t count;      // rays in this launch
     uint64_t seed;
     uint32_t instance;
-    int pad;
+    int n_prims;         // elements of the scene
     const GridDesc* grid;  // field grid of the scene, nullptr: BVH (or element list) traversal
     const float* h3t12;    // Halton base-3 partial sums after 12 digits (halton3_table), or nullptr
     const SunGrid* sgrid;  // candidate grid of the sun rays (scenes of more than 8 elements)
-    // single-scene launches: tiles handed out by this device counter (zeroed by launch_trace before
-    // the kernel) in guided grabs; nullptr: static round robin (launches that may overlap on the
-    // GPU with another of the same counter use that)
-    unsigned long long* tile_counter;
+    // single-scene launches: tiles handed out by this device counter ([0] tiles, [1] CTAs done; zero
+    // between launches, the last CTA sees to that) in guided grabs; nullptr: static shares (launches
+    // that may overlap on the GPU with another of the same counter use that)
+    unsigned int* tile_counter;
 };
 
 // Arguments of the single-scene element-list kernel: TraceArgs plus the Philox key schedule of
@@ -103,9 +103,9 @@ void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job);
 cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, cudaStream_t stream);
 
 // Trace rays [ray_begin, ray_begin + count): generation, closest-hit search, shading, the dense
-// hit-record write.  Scenes of up to 8 elements (n_prims) take the shared-memory element list path;
-// larger ones need args.sgrid.
-cudaError_t launch_trace(const TraceArgs& args, int n_prims, cudaStream_t stream);
+// hit-record write.  Scenes of up to 8 elements take the shared-memory element list path; larger ones
+// need args.sgrid.
+cudaError_t launch_trace(const TraceArgs& args, cudaStream_t stream);
 
 // Compact form of a dense hit buffer of n rays (csp_run_to_host_compact): count pass -- per ray the
 // number of records after slot 0 (uint8) and, in block_sums[compact_blocks(n) + 1], the exclusive

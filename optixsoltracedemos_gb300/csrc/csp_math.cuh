@@ -31,24 +31,6 @@
 
 namespace csp {
 
-// ------------------------------------------------------------------------------------ float3 ---
-CSP_HD float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
-CSP_HD float3 add(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
-CSP_HD float3 sub(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
-CSP_HD float3 scale(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
-CSP_HD float3 neg(float3 a) { return make_float3(-a.x, -a.y, -a.z); }
-CSP_HD float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-CSP_HD float3 cross(float3 a, float3 b) {
-    return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
-CSP_HD float length(float3 v) { return sqrtf(dot(v, v)); }
-CSP_HD float3 normalize(float3 v) {
-    const float inv = 1.0f / sqrtf(dot(v, v));
-    return scale(inv, v);
-}
-CSP_HD float3 reflect(float3 i, float3 n) { return sub(i, scale(dot(n, i), scale(2.0f, n))); }
-CSP_HD float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
-
 CSP_HD uint32_t f2u(float f) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(f);
@@ -67,6 +49,41 @@ CSP_HD float u2f(uint32_t u) {
     return f;
 #endif
 }
+
+// ------------------------------------------------------------------------------------ float3 ---
+CSP_HD float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
+CSP_HD float3 add(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
+CSP_HD float3 sub(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
+CSP_HD float3 scale(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
+CSP_HD float3 neg(float3 a) { return make_float3(-a.x, -a.y, -a.z); }
+CSP_HD float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+CSP_HD float3 cross(float3 a, float3 b) {
+    return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
+CSP_HD float length(float3 v) { return sqrtf(dot(v, v)); }
+CSP_HD float3 normalize(float3 v) {
+    const float inv = 1.0f / sqrtf(dot(v, v));
+    return scale(inv, v);
+}
+// 1.0f / sqrtf(x), both rounded, in closed form for x within 2^-12 of 1.  With u = 2^-23, for x = 1 + k u
+// (0 <= k < 2048): sqrt x = 1 + k u / 2 - k^2 u^2 / 8 rounds to 1 + floor(k / 2) u (an odd k lies just
+// below the tie), and the reciprocal of 1 + j u to 1 - j u, since j^2 u^2 is far below half an ulp.
+// For x = 1 - k u / 2 (0 < k <= 2048): sqrt x rounds to 1 - ceil(k / 2) u / 2 (just beyond the tie), and
+// the reciprocal of 1 - j u / 2 to 1 + ceil(j / 2) u.  In the bits of a float around 1 each is a
+// subtraction and a shift.
+CSP_HD float rsqrt_near_1(float x) {
+    const int k = (int)f2u(x) - 0x3f800000;
+    return u2f((uint32_t)(0x3f800000 + (k >= 0 ? -(k & ~1) : (3 - k) >> 2)));
+}
+// normalize(v) for a v expected near unit length (a direction, a slightly tilted normal): the same
+// value without the square root and the division, which cost about 20 instructions more.
+CSP_HD float3 normalize_unit(float3 v) {
+    const float x = dot(v, v);
+    const bool near1 = f2u(x) - (0x3f800000u - 2048u) < 4096u;
+    return scale(near1 ? rsqrt_near_1(x) : 1.0f / sqrtf(x), v);
+}
+CSP_HD float3 reflect(float3 i, float3 n) { return sub(i, scale(dot(n, i), scale(2.0f, n))); }
+CSP_HD float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
 // ------------------------------------------------------------------------------------ Philox ---
 struct u32x4 {

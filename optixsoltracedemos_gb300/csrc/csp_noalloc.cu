@@ -140,7 +140,7 @@ extern "C" int csp_trace_noalloc(int device, const csp_element* elements, uint32
                          "csp_trace_noalloc: prepare_sun_kernel");
         if (!rc && num_rays) {
             TraceArgs a;
-            a.tile_counter = nullptr;  // static round robin: nothing to allocate
+            a.tile_counter = nullptr;  // static shares: nothing to allocate
             a.nodes = reinterpret_cast<const Node*>(scratch + kOffNodes);
             a.prims = reinterpret_cast<const Prim*>(scratch + kOffPrims);
             a.optics = reinterpret_cast<const Optics*>(scratch + kOffOptics);
@@ -151,11 +151,11 @@ extern "C" int csp_trace_noalloc(int device, const csp_element* elements, uint32
             a.count = num_rays;
             a.seed = seed;
             a.instance = instance;
-            a.pad = 0;
+            a.n_prims = (int)count;
             a.grid = nullptr;
             a.h3t12 = nullptr;
             a.sgrid = nullptr;
-            rc = cuda_status(launch_trace(a, (int)count, st), "csp_trace_noalloc: trace_kernel");
+            rc = cuda_status(launch_trace(a, st), "csp_trace_noalloc: trace_kernel");
         }
     }
     if (prev >= 0 && prev != device) cudaSetDevice(prev);

@@ -730,7 +730,7 @@ int Server::step_launch(int par, bool after_other, std::vector<SRequest*>& finis
             d.args.ids = nullptr;
             d.args.seed = r->seed;
             d.args.instance = r->instance;
-            d.args.pad = 0;
+            d.args.n_prims = (int)s.elements.size();
             d.args.grid = g == kAccelGrid ? reinterpret_cast<const GridDesc*>(d_arena + r->o_grid) : nullptr;
             d.args.h3t12 = h3t12;
             d.args.sgrid = nullptr;

@@ -10,22 +10,20 @@
 //   traverse            OptiX traversal: closest hit among the elements whose AABB the ray overlaps
 //   classify/shade      closest-hit programs, cuda/materials.cu:26-231; miss program :236-253
 //
-// Wavefront inside each CTA (kB threads, one tile = kB consecutive rays of one instance):
-//   phase A (one ray per thread, every ray): sun sample and the cheap, branch-free part of the first
-//     segment.  Rays with more to do are pushed into a shared-memory queue (warp ballot + one shared
-//     atomic per warp):
-//       small scenes (kFlat, <= kFlatMax elements, all in shared memory): phase A only runs the AABB
-//         slab tests; rays whose segment overlaps some element box are queued with that mask;
-//       BVH and grid scenes: phase A finds and records the first hit; mirror hits are queued
-//         unshaded.
-//   phase B (only on full batches of kB queued rays, and on the remainder at the end): the rest of
-//     each queued path -- intersection programs, shading, further segments.
-// In the heliostat workloads ~10% of rays meet an element; running their intersection programs and
-// shading on full warps instead of inside warps where ~90% of lanes have finished is the point.
+// Wavefront inside each CTA (kB threads, one tile = kB rays of one instance):
+//   phase A (one ray per thread, every ray): the sun sample and what decides whether the ray goes on.
+//     Rays that do are pushed into a shared-memory queue (warp ballot + one shared atomic per warp):
+//       small scenes (kFlat, <= kFlatMax elements, all in shared memory): the rays whose sun-plane
+//         point lies in some element's reach rectangle;
+//       BVH and grid scenes: the rays whose first segment, traced and recorded here, hits a mirror.
+//   phase B (only on full batches of kB queued rays, and on the remainder at the end): the whole path of
+//     each (kFlat), or its next bounce (shading, search, record; further mirror hits are queued again).
+// In the heliostat workloads ~10% of rays meet an element of a small scene; running their paths on full
+// warps instead of inside warps where ~90% of lanes have finished is the point.
 //
 // Output sinks (compile-time):
 //   kDense  the reference's hit_point_buffer: 5 float4 records per ray (+ optional element ids).
-//           Phase A stages the warp's records in shared memory and writes them as coalesced rows;
+//           Phase A writes every row (kFlat: the warp's rows staged in shared memory, coalesced);
 //           phase B writes its records straight to global memory (their rows were written by phase A
 //           of an earlier tile of this CTA, ordered by the barriers in between).
 //   kFlux   receiver records are binned into the instance's flux map in the shading stage (global
@@ -99,7 +97,8 @@ struct Cfg {
     // launches trace the first segment in place (first_segment)
     using Core = CoreSmem<kB_, kFlat>;
     // phase A record staging of dense element-list launches
-    using Stage = FlatStageSmem<kB_>;
+    struct NoStage {};
+    using Stage = std::conditional_t<kFlat && kDense_, FlatStageSmem<kB_>, NoStage>;
 };
 
 // Coherent ray order: position kk of a launch of `count` rays -> ray offset.  Rays come in blocks
@@ -221,96 +220,7 @@ struct StateSmem {
     float4 part[kStateBlock / 32], slot;
 };
 
-// One block, or one cluster of kCluster blocks, computes the sun frame of one scene: plane distance,
-// u/v bounds, parallelogram (lib/sun_utils.cu:53-179, lib/geometry_manager.cpp:97-148) and cone frame
-// (cuda/sun.cu:76-79).  Two passes over the element boxes, the second after the first's result:
-// latency-bound, so large scenes spread them over a cluster (10,001 elements: 28.4 us in one block).
-template <int kCluster>
-__device__ void sun_frame_state(const Aabb* __restrict__ aabbs, int n, float3 s, float tan_pad, int shape,
-                                float param, SunFrame* __restrict__ out, StateSmem& sm) {
-    const int rank = kCluster > 1 ? (int)(blockIdx.x % kCluster) : 0;
-    const int first = rank * (int)blockDim.x + (int)threadIdx.x, step = kCluster * (int)blockDim.x;
-    const float inf = __int_as_float(0x7f800000);
-    // plane distance: max over every AABB corner of |c . s| (and 0), lib/sun_utils.cu:53-104
-    float md = 0.0f;
-    for (int i = first; i < n; i += step) {
-        const Aabb b = aabbs[i];
-        for (int k = 0; k < 8; ++k) md = fmaxf(md, fabsf(dot(corner(b, k), s)));
-    }
-    const float d = -state_reduce<kCluster>(make_float4(-md, inf, inf, inf), sm.part, &sm.slot, Min4()).x;
-
-    const float3 axis = (fabsf(s.x) < 0.9f) ? f3(1.0f, 0.0f, 0.0f) : f3(0.0f, 1.0f, 0.0f);
-    const float3 su = normalize(cross(axis, s));
-    const float3 sv = normalize(cross(s, su));
-    const float3 pc = scale(d, s);
-    // u/v bounds padded by |c . s| tan(angle), lib/sun_utils.cu:106-179
-    float umin = FLT_MAX, umax = -FLT_MAX, vmin = FLT_MAX, vmax = -FLT_MAX;
-    for (int i = first; i < n; i += step) {
-        const Aabb b = aabbs[i];
-        for (int k = 0; k < 8; ++k) {
-            const float3 pt = corner(b, k);
-            const float buf = fabsf(dot(pt, s)) * tan_pad;
-            const float3 proj = sub(pt, scale(dot(sub(pt, pc), s), s));
-            const float u = dot(proj, su), v = dot(proj, sv);
-            umin = fminf(umin, u - buf);
-            umax = fmaxf(umax, u + buf);
-            vmin = fminf(vmin, v - buf);
-            vmax = fmaxf(vmax, v + buf);
-        }
-    }
-    // the maxima as minima of the negated values
-    const float4 m = state_reduce<kCluster>(make_float4(umin, -umax, vmin, -vmax), sm.part, &sm.slot, Min4());
-    umin = m.x;
-    umax = -m.y;
-    vmin = m.z;
-    vmax = -m.w;
-    if constexpr (kCluster > 1) cooperative_groups::this_cluster().sync();  // the slots are read
-    if (rank != 0 || threadIdx.x != 0) return;
-    const float3 ds = scale(d, s);
-    const float3 v0 = add(add(scale(umin, su), scale(vmin, sv)), ds);
-    const float3 v1 = add(add(scale(umax, su), scale(vmin, sv)), ds);
-    const float3 v2 = add(add(scale(umax, su), scale(vmax, sv)), ds);
-    const float3 v3 = add(add(scale(umin, su), scale(vmax, sv)), ds);
-    // cone frame, cuda/sun.cu:76-79 with dir = -normalize(sun_vector) (cuda/sun.cu:106)
-    const float3 w = normalize(neg(normalize(s)));
-    const float3 cu = normalize(cross(fabsf(w.x) > 0.99f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f), w));
-    const float3 cv = cross(w, cu);
-    SunFrame f;
-    f.s_d = make_float4(s.x, s.y, s.z, d);
-    f.v0 = make_float4(v0.x, v0.y, v0.z, 0.f);
-    const float3 e1 = sub(v1, v0), e2 = sub(v3, v0);
-    f.e1 = make_float4(e1.x, e1.y, e1.z, 0.f);
-    f.e2 = make_float4(e2.x, e2.y, e2.z, 0.f);
-    f.v1 = make_float4(v1.x, v1.y, v1.z, 0.f);
-    f.v2 = make_float4(v2.x, v2.y, v2.z, 0.f);
-    f.v3 = make_float4(v3.x, v3.y, v3.z, 0.f);
-    f.w = make_float4(w.x, w.y, w.z, 0.f);
-    f.u = make_float4(cu.x, cu.y, cu.z, 0.f);
-    f.v = make_float4(cv.x, cv.y, cv.z, 0.f);
-    f.omc = 0.0f;
-    if (shape & 1) {
-        f.cos_theta = 1.0f;
-        f.sigma = param;
-    } else if (shape & 2) {
-        // accurate cone sampler: 1 - cos(half_angle) = 2 sin^2(half_angle / 2), free of the
-        // cancellation of 1 - cosf(half_angle)
-        float sn, cs;
-        det_sincos(param * 0.5f, sn, cs);
-        f.omc = (sn + sn) * sn;
-        f.cos_theta = 1.0f - f.omc;
-        f.sigma = 0.0f;
-    } else {
-        float sn, cs;
-        det_sincos(param, sn, cs);  // cosf(half_angle), cuda/sun.cu:82
-        f.cos_theta = cs;
-        f.sigma = 0.0f;
-    }
-    f.tan_pad = tan_pad;
-    f.shape = shape;
-    f.n_prims = n;
-    f.pad1 = f.pad2 = 0;
-    *out = f;
-}
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // 32-byte accesses (p 32-byte aligned).  Lanes on different records of a scene, or on different
 // rows of the hit buffer, touch a cache line per access and lane: half as many accesses is half the
@@ -409,7 +319,7 @@ __device__ __forceinline__ float halton3_tab(uint64_t i, const float* __restrict
 __device__ __forceinline__ float3 perturb(float3 n, float sigma, float g1, float g2) {
     const float3 t1 = normalize(cross(fabsf(n.x) > 0.9f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f), n));
     const float3 t2 = cross(n, t1);
-    return normalize(add(add(n, scale(sigma * g1, t1)), scale(sigma * g2, t2)));
+    return normalize_unit(add(add(n, scale(sigma * g1, t1)), scale(sigma * g2, t2)));
 }
 
 // ------------------------------------------------------------------------------ intersection --
@@ -480,7 +390,7 @@ __device__ __forceinline__ float3 parab_normal(const Prim& p, float3 o, float3 d
     const float dx = dot(d, e1), dy = dot(d, e2);
     const float xh = ox + t * dx, yh = oy + t * dy;
     const float3 nl = normalize(f3(-p.c.w * xh, -p.d.w * yh, 1.0f));
-    return normalize(add(add(scale(nl.x, e1), scale(nl.y, e2)), scale(nl.z, n)));
+    return normalize_unit(add(add(scale(nl.x, e1), scale(nl.y, e2)), scale(nl.z, n)));
 }
 
 // Cylinder_Y with caps, cuda/intersection.cu:177-296.  `accurate` (extension, the CSP_SUN_ACCURATE
@@ -489,7 +399,7 @@ __device__ __forceinline__ float3 parab_normal(const Prim& p, float3 o, float3 d
 // B^2 - 4AC, which cancels to ~1e-4 relative when the ray starts hundreds of metres from the
 // receiver (about 1 mm on the hit point in float).
 __device__ __forceinline__ bool hit_cyl(const Prim& p, float3 o, float3 draw, float tmin, bool accurate, float& tout) {
-    const float3 d = normalize(draw);
+    const float3 d = normalize_unit(draw);
     const float3 lo = sub(o, xyz(p.a));
     const float3 lx = xyz(p.b), ly = xyz(p.c), lz = xyz(p.d);
     const float Ox = dot(lo, lx), Oy = dot(lo, ly), Oz = dot(lo, lz);
@@ -598,8 +508,6 @@ __device__ __forceinline__ int traverse(const Node* __restrict__ nodes, const Pr
     }
     return best;
 }
-
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // Exact-AABB culling and intersection program of one grid candidate (a BVH leaf's work): the
 // element's exact AABB lo, hi with lo.w = element | type << 28.
@@ -826,19 +734,34 @@ __device__ __forceinline__ uint32_t candidates(const FlatScene& fs, float3 o, fl
     return mask;
 }
 
-// Closest hit among the candidate elements, in ascending index (equal t keeps the lower index).
+// Closest hit among the candidate elements, in ascending index (equal t keeps the lower index): the
+// mirrors, then the receiver, so that a warp whose lanes have different candidates does not run the
+// mirrors' and the receiver's programs in turn.
 __device__ __forceinline__ int closest_in(const FlatScene& fs, uint32_t mask, float3 o, float3 d, float tmin,
                                           bool acc, float& best_t, uint32_t& best_type) {
     int best = -1;
     best_t = __int_as_float(0x7f800000);
-    while (mask) {
-        const int k = __ffs(mask) - 1;
-        mask &= mask - 1u;
+    const int rcv = fs.n - 1;
+    uint32_t mm = mask & ((1u << rcv) - 1u);
+    while (mm) {
+        const int k = __ffs(mm) - 1;
+        mm &= mm - 1u;
+        const uint32_t type = fs.type[k];
         float t;
-        if (hit_prim(fs.type[k], fs.prim[k], o, d, tmin, acc, t) && t < best_t) {
+        const bool hit = type == kParabolicMirror ? hit_parab(fs.prim[k], o, d, tmin, t) : hit_flat(fs.prim[k], o, d, tmin, t);
+        if (hit && t < best_t) {
             best = k;
             best_t = t;
-            best_type = fs.type[k];
+            best_type = type;
+        }
+    }
+    if ((mask >> rcv) & 1u) {
+        const uint32_t type = fs.type[rcv];
+        float t;
+        if (hit_prim(type, fs.prim[rcv], o, d, tmin, acc, t) && t < best_t) {
+            best = rcv;
+            best_t = t;
+            best_type = type;
         }
     }
     return best;
@@ -890,7 +813,7 @@ __device__ __forceinline__ bool shade_mirror(const typename C::Args& A, uint64_t
                                              const Segment& g, const Hit& h, Segment& next) {
     const int nd = g.depth + 1;
     const float3 hit = add(g.o, scale(h.t, g.d));
-    const float3 wn = (h.type == kFlatMirror) ? normalize(xyz(p.a)) : normalize(parab_normal(p, g.o, g.d, h.t));
+    const float3 wn = normalize_unit(h.type == kFlatMirror ? xyz(p.a) : parab_normal(p, g.o, g.d, h.t));
     float3 ffn = (dot(neg(g.d), wn) >= 0.0f) ? wn : neg(wn);
     const bool need_rng = (op.slope > 0.0f) || (op.spec > 0.0f) || !(op.reflectivity >= 1.0f);
     u32x4 ra = {0u, 0u, 0u, 0u};
@@ -905,7 +828,7 @@ __device__ __forceinline__ bool shade_mirror(const typename C::Args& A, uint64_t
         const u32x4 rb = draw<C>(A, ray, (uint32_t)nd, 1);
         float g1, g2;
         box_muller(u01(rb.x), u01(rb.y), g1, g2);
-        rd = perturb(normalize(rd), op.spec, g1, g2);
+        rd = perturb(normalize_unit(rd), op.spec, g1, g2);
     }
     if (need_rng && u01(ra.x) > op.reflectivity) return false;  // absorbed at the mirror
     next = Segment{hit, rd, kTminBounce, nd};
@@ -926,7 +849,7 @@ __device__ __forceinline__ float3 sun_direction(const typename C::Args& A, const
     if (S.shape & 1) {
         float g1, g2;
         box_muller(u01(r0.x), u01(r0.y), g1, g2);
-        dir = normalize(add(add(w, scale(S.sigma * g1, cu)), scale(S.sigma * g2, cv)));
+        dir = normalize_unit(add(add(w, scale(S.sigma * g1, cu)), scale(S.sigma * g2, cv)));
     } else if (S.shape & 2) {
         // the reference's uniform z in [cos(half_angle), 1] (cuda/sun.cu:82-86) carried as
         // 1 - z = (1 - cos(half_angle)) (1 - rand2), so that the cone radius
@@ -939,7 +862,7 @@ __device__ __forceinline__ float3 sun_direction(const typename C::Args& A, const
         const float r = sqrtf(omz * (2.0f - omz));
         float sp, cp;
         det_sincos(phi, sp, cp);
-        dir = normalize(add(scale(r, add(scale(cp, cu), scale(sp, cv))), scale(z, w)));
+        dir = normalize_unit(add(scale(r, add(scale(cp, cu), scale(sp, cv))), scale(z, w)));
     } else {
         const float rand1 = u01(r0.x), rand2 = u01(r0.y);
         const float phi = kTwoPi * rand1;
@@ -947,7 +870,7 @@ __device__ __forceinline__ float3 sun_direction(const typename C::Args& A, const
         const float r = sqrtf(1.0f - z * z);
         float sp, cp;
         det_sincos(phi, sp, cp);
-        dir = normalize(add(scale(r, add(scale(cp, cu), scale(sp, cv))), scale(z, w)));
+        dir = normalize_unit(add(scale(r, add(scale(cp, cu), scale(sp, cv))), scale(z, w)));
     }
     return dir;
 }
@@ -1030,28 +953,132 @@ __device__ __forceinline__ float4 cross_rect(const SunFrame& S, float tan_a, flo
     return widened(b, rad / n1 + 2e-6f, rad / n2 + 2e-6f);
 }
 
+// One block, or one cluster of kCluster blocks, computes the sun frame of one scene: plane distance,
+// u/v bounds, parallelogram (lib/sun_utils.cu:53-179, lib/geometry_manager.cpp:97-148) and cone frame
+// (cuda/sun.cu:76-79).  Two passes over the element boxes, the second after the first's result:
+// latency-bound, so large scenes spread them over a cluster (10,001 elements: 28.4 us in one block).
+template <int kCluster>
+__device__ void sun_frame_state(const Aabb* __restrict__ aabbs, int n, float3 s, float tan_pad, int shape,
+                                float param, SunFrame* __restrict__ out, StateSmem& sm) {
+    const int rank = kCluster > 1 ? (int)(blockIdx.x % kCluster) : 0;
+    const int first = rank * (int)blockDim.x + (int)threadIdx.x, step = kCluster * (int)blockDim.x;
+    const float inf = __int_as_float(0x7f800000);
+    // plane distance: max over every AABB corner of |c . s| (and 0), lib/sun_utils.cu:53-104
+    float md = 0.0f;
+    for (int i = first; i < n; i += step) {
+        const Aabb b = aabbs[i];
+        for (int k = 0; k < 8; ++k) md = fmaxf(md, fabsf(dot(corner(b, k), s)));
+    }
+    const float d = -state_reduce<kCluster>(make_float4(-md, inf, inf, inf), sm.part, &sm.slot, Min4()).x;
+
+    const float3 axis = (fabsf(s.x) < 0.9f) ? f3(1.0f, 0.0f, 0.0f) : f3(0.0f, 1.0f, 0.0f);
+    const float3 su = normalize(cross(axis, s));
+    const float3 sv = normalize(cross(s, su));
+    const float3 pc = scale(d, s);
+    // u/v bounds padded by |c . s| tan(angle), lib/sun_utils.cu:106-179
+    float umin = FLT_MAX, umax = -FLT_MAX, vmin = FLT_MAX, vmax = -FLT_MAX;
+    for (int i = first; i < n; i += step) {
+        const Aabb b = aabbs[i];
+        for (int k = 0; k < 8; ++k) {
+            const float3 pt = corner(b, k);
+            const float buf = fabsf(dot(pt, s)) * tan_pad;
+            const float3 proj = sub(pt, scale(dot(sub(pt, pc), s), s));
+            const float u = dot(proj, su), v = dot(proj, sv);
+            umin = fminf(umin, u - buf);
+            umax = fmaxf(umax, u + buf);
+            vmin = fminf(vmin, v - buf);
+            vmax = fmaxf(vmax, v + buf);
+        }
+    }
+    // the maxima as minima of the negated values
+    const float4 m = state_reduce<kCluster>(make_float4(umin, -umax, vmin, -vmax), sm.part, &sm.slot, Min4());
+    umin = m.x;
+    umax = -m.y;
+    vmin = m.z;
+    vmax = -m.w;
+    if constexpr (kCluster > 1) cooperative_groups::this_cluster().sync();  // the slots are read
+    if (rank != 0) return;
+    if (threadIdx.x == 0) {
+        const float3 ds = scale(d, s);
+        const float3 v0 = add(add(scale(umin, su), scale(vmin, sv)), ds);
+        const float3 v1 = add(add(scale(umax, su), scale(vmin, sv)), ds);
+        const float3 v2 = add(add(scale(umax, su), scale(vmax, sv)), ds);
+        const float3 v3 = add(add(scale(umin, su), scale(vmax, sv)), ds);
+        // cone frame, cuda/sun.cu:76-79 with dir = -normalize(sun_vector) (cuda/sun.cu:106)
+        const float3 w = normalize(neg(normalize(s)));
+        const float3 cu = normalize(cross(fabsf(w.x) > 0.99f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f), w));
+        const float3 cv = cross(w, cu);
+        SunFrame f{};
+        f.s_d = make_float4(s.x, s.y, s.z, d);
+        f.v0 = make_float4(v0.x, v0.y, v0.z, 0.f);
+        const float3 e1 = sub(v1, v0), e2 = sub(v3, v0);
+        f.e1 = make_float4(e1.x, e1.y, e1.z, 0.f);
+        f.e2 = make_float4(e2.x, e2.y, e2.z, 0.f);
+        f.v1 = make_float4(v1.x, v1.y, v1.z, 0.f);
+        f.v2 = make_float4(v2.x, v2.y, v2.z, 0.f);
+        f.v3 = make_float4(v3.x, v3.y, v3.z, 0.f);
+        f.w = make_float4(w.x, w.y, w.z, 0.f);
+        f.u = make_float4(cu.x, cu.y, cu.z, 0.f);
+        f.v = make_float4(cv.x, cv.y, cv.z, 0.f);
+        f.omc = 0.0f;
+        if (shape & 1) {
+            f.cos_theta = 1.0f;
+            f.sigma = param;
+        } else if (shape & 2) {
+            // accurate cone sampler: 1 - cos(half_angle) = 2 sin^2(half_angle / 2), free of the
+            // cancellation of 1 - cosf(half_angle)
+            float sn, cs;
+            det_sincos(param * 0.5f, sn, cs);
+            f.omc = (sn + sn) * sn;
+            f.cos_theta = 1.0f - f.omc;
+            f.sigma = 0.0f;
+        } else {
+            float sn, cs;
+            det_sincos(param, sn, cs);  // cosf(half_angle), cuda/sun.cu:82
+            f.cos_theta = cs;
+            f.sigma = 0.0f;
+        }
+        f.tan_pad = tan_pad;
+        f.shape = shape;
+        f.n_prims = n;
+        f.pad1 = f.pad2 = 0;
+        *out = f;
+    }
+    // reach rectangles of an element-list scene, which every launch of it tests in phase A
+    if (n <= kFlatMax) {
+        __syncthreads();
+        if ((int)threadIdx.x < n) {
+            const Aabb b = aabbs[threadIdx.x];
+            const SunFrame& f = *out;
+            out->reach[threadIdx.x] =
+                reach_rect(f, cone_tan(f), box_span(f, make_float4(0.f, 0.f, 0.f, 0.f), b.lo, b.hi));
+        }
+    }
+}
+
 // Queue entries of BVH/grid launches carry the depth of their pending mirror hit in the top bits of
 // the ray index (ray indices stay below 2^56, kRayIndexLimit, which every host entry point checks).
 constexpr int kDepthShift = 56;
 constexpr uint64_t kRayMask = (1ull << kDepthShift) - 1u;
 static_assert((1ull << kDepthShift) == kRayIndexLimit, "the host ray-window check must match the packing");
 
-// Shared memory of one CTA: the bounce queue, the generation queue of kFlat launches (sun-plane points
-// of the rays waiting for their direction), the Halton table, the sun frame, and the kFlat scene with
+// Shared memory of one CTA: the bounce queue, the generation queue of kFlat launches (Halton
+// coordinates of the rays waiting for their direction), the Halton table, the sun frame, and the kFlat scene with
 // its elements' reach rectangles or the descriptors of the grids of the other launches.
 template <int kB, bool kFlat>
 struct CoreSmem {
-    float qo[3][2 * kB], qd[3][2 * kB], qt[2 * kB];
-    uint32_t qw[2 * kB];  // kFlat: candidate mask; BVH: element | type << 28 of the pending mirror hit
-    uint64_t qray[2 * kB];
-    float go[3][kFlat ? 2 * kB : 1];
+    static constexpr int kQ = kFlat ? 1 : 2 * kB;
+    float qo[3][kQ], qd[3][kQ];
+    float qt[kQ];  // distance of the pending mirror hit
+    uint32_t qw[kQ];  // its element | type << 28
+    uint64_t qray[kQ];
+    float go[2][kFlat ? 2 * kB : 1];
     uint64_t gray[kFlat ? 2 * kB : 1];
-    float4 reach[kFlat ? kFlatMax : 1];
     float t6[kH3Tab];
     FlatScene flat;
     SunFrame sun;
-    GridDesc grid;
-    SunGrid sg;
+    std::conditional_t<kFlat, char, GridDesc> grid;
+    std::conditional_t<kFlat, char, SunGrid> sg;
     // next free queue positions (shared atomics hand them out); every thread also carries the
     // sizes in registers, updated at the barriers that close each append
     int qsize;
@@ -1067,11 +1094,13 @@ __device__ __forceinline__ int find_closest(const typename C::Args& A, const typ
     else return traverse(A.nodes, A.prims, o, d, tmin, self, acc, t, type);
 }
 
-// Dense element-list launches: phase A produces slot 0 of each row only (the sun-plane record);
-// the other slots are empty until phase B writes them straight to global memory.
+// Dense element-list launches: the rows of a tile, slot 0 written by phase A, the others empty for
+// good.  A warp's 32 rows leave as five coalesced 512-byte rows read back from here.  (As one
+// cp.async.bulk per warp, completed before phase B writes into the rows: 296 us against 293 per 16M
+// rays of the single parabolic heliostat.)
 template <int kB>
 struct FlatStageSmem {
-    float4 rec0[kB];
+    float4 row[kB * kMaxDepth];
 };
 
 // Where kFlux records go: the instance's flux target and the CTA's record counters.
@@ -1119,7 +1148,7 @@ __device__ __forceinline__ void emit(const typename C::Args& A, const Sink& k, u
 // warp-aggregated append of the lanes with `want` set to the generation queue; every lane of the
 // warp must call it
 template <class Core>
-__device__ __forceinline__ void push_gen(Core& sm, bool want, uint64_t ray, float3 o) {
+__device__ __forceinline__ void push_gen(Core& sm, bool want, uint64_t ray, float hu, float hv) {
     const unsigned mask = __ballot_sync(0xffffffffu, want);
     if (mask == 0u) return;
     const int lane = threadIdx.x & 31;
@@ -1128,9 +1157,8 @@ __device__ __forceinline__ void push_gen(Core& sm, bool want, uint64_t ray, floa
     base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
     if (want && CSP_BOUNDS(1, base + __popc(mask & ((1u << lane) - 1u)) < (int)(sizeof(sm.gray) / sizeof(sm.gray[0])))) {
         const int k = base + __popc(mask & ((1u << lane) - 1u));
-        sm.go[0][k] = o.x;
-        sm.go[1][k] = o.y;
-        sm.go[2][k] = o.z;
+        sm.go[0][k] = hu;
+        sm.go[1][k] = hv;
         sm.gray[k] = ray;
     }
 }
@@ -1159,17 +1187,17 @@ __device__ __forceinline__ void push(Core& sm, bool want, uint64_t ray, float3 o
     }
 }
 
-// A queued path of an element-list launch, from its first segment `g` with candidate mask `m`: closest
-// hit, record, shade, next segment, until the ray misses, is absorbed, ends on the receiver or reaches
-// the depth limit.
+// The whole path of a queued sun ray of an element-list launch from its Halton coordinates: direction,
+// then box tests, closest hit, record, shade, next segment, until the ray misses, is absorbed, ends on
+// the receiver or reaches the depth limit.
 template <class C>
 __device__ __forceinline__ void flat_path(const typename C::Args& A, const Sink& k, const typename C::Core& sm,
-                                          uint64_t ray, Segment g, uint32_t m) {
-    // the first segment's search on its own: in one copy inside the loop the kernel spills (16 M rays
-    // of the single parabolic heliostat: 381 us against 313)
-    Hit h;
-    h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
+                                          uint64_t ray, float hu, float hv) {
+    Segment g{sun_point(sm.sun, hu, hv), sun_direction<C>(A, sm.sun, ray), kTminSun, 0};
     for (;;) {
+        const uint32_t m = candidates(sm.flat, g.o, g.d, g.tmin);
+        Hit h;
+        h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
         if (h.best < 0) return;  // __miss__ms, cuda/materials.cu:236-253
         const Prim p = sm.flat.prim[h.best];
         float4 rec;
@@ -1180,8 +1208,6 @@ __device__ __forceinline__ void flat_path(const typename C::Args& A, const Sink&
         Segment next;
         if (!shade_mirror<C>(A, ray, p, sm.flat.optics[h.best], g, h, next)) return;
         g = next;
-        m = candidates(sm.flat, g.o, g.d, g.tmin);
-        h.best = closest_in(sm.flat, m, g.o, g.d, g.tmin, (sm.sun.shape & 2) != 0, h.t, h.type);
     }
 }
 
@@ -1200,124 +1226,98 @@ __device__ __forceinline__ uint32_t own_mirror(const Prim& p, const Hit& h, cons
     return skip ? (uint32_t)h.best : kNoElement;
 }
 
-// One batch of up to kB rays from the top of the bounce queue (qs entries): kFlat launches finish
-// their paths, BVH/grid launches advance them by one bounce.  Returns the queue size after it, the
-// same in every thread (the barrier that ends the batch counts the rays queued again), so that no
-// thread reads the shared counter after the batch: a warp that has gone on to the next tile may
-// already be appending to it.
+// One batch of up to kB rays from the top of the bounce queue (qs entries): advances their paths by one
+// bounce.  Returns the queue size after it, the same in every thread (the barrier that ends the batch
+// counts the rays queued again), so that no thread reads the shared counter after the batch: a warp
+// that has gone on to the next tile may already be appending to it.
 template <class C>
 __device__ __forceinline__ int bounce_batch(const typename C::Args& A, const Sink& k, typename C::Core& sm, int qs) {
-    {
-        const int n = min(qs, C::kB);
-        const int base = qs - n;
-        const bool have = (int)threadIdx.x < n;
-        float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f);
-        float t = 0.f;
-        uint32_t w = 0;
-        uint64_t ray = 0;
-        if (have) {
-            const int q = base + threadIdx.x;
-            o = f3(sm.qo[0][q], sm.qo[1][q], sm.qo[2][q]);
-            d = f3(sm.qd[0][q], sm.qd[1][q], sm.qd[2][q]);
-            t = sm.qt[q];
-            w = sm.qw[q];
-            ray = sm.qray[q];
-        }
-        // the barrier both ends the reads of the popped entries and publishes the new size: no
-        // thread appends (atomicAdd on qsize, then writes from `base` on) before it, and none read
-        // qsize since the barrier that closed the last append
-        if (threadIdx.x == 0) sm.qsize = base;
-        __syncthreads();
-        if (have) {
-            if constexpr (C::kFlat) flat_path<C>(A, k, sm, ray, Segment{o, d, kTminSun, 0}, w);
-        }
-        if constexpr (!C::kFlat) {
-            // one bounce per batch: shade the pending mirror hit (its record is out), find the next
-            // hit, record it, and queue it again when it is another mirror below the depth limit
-            bool again = false;
-            Segment next{f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 1.f), 0.f, 0};
-            Hit h2{-1, 0.f, 0u};
-            const uint64_t r = ray & kRayMask;
-            if (have) {
-                const int depth = (int)(ray >> kDepthShift);
-                const Segment g{o, d, depth == 0 ? kTminSun : kTminBounce, depth};
-                const Hit h{(int)(w & kPrimMask), t, w >> kTypeShift};
-                const Prim p = load_prim(A.prims, (uint32_t)h.best);
-                if (shade_mirror<C>(A, r, p, A.optics[h.best], g, h, next)) {
-                    h2.best = find_closest<C>(A, sm, next.o, next.d, next.tmin, own_mirror(p, h, g, next), h2.t, h2.type);
-                    if (h2.best >= 0) {
-                        const Prim p2 = load_prim(A.prims, (uint32_t)h2.best);
-                        float4 rec;
-                        int slot;
-                        again = classify(p2, next, h2, rec, slot);
-                        if (slot >= 0) emit<C>(A, k, r, slot, rec, (uint32_t)h2.best);
-                    }
-                }
-            }
-            push(sm, again, r | ((uint64_t)next.depth << kDepthShift), next.o, next.d, h2.t,
-                 (uint32_t)h2.best | (h2.type << kTypeShift));
-            return base + __syncthreads_count(again);
-        }
-        __syncthreads();
-        return base;
-    }
-}
-
-// One batch of up to kB rays from the top of the generation queue (element-list launches; gs
-// entries): sun direction and the box tests of the first segment, on full warps; rays that meet a box
-// go to the bounce queue (qs entries, fewer than kB on entry) with their candidate mask.  Updates gs
-// and qs, the same in every thread (the closing barrier counts the rays queued).
-template <class C>
-__device__ __forceinline__ void gen_batch(const typename C::Args& A, const Sink& k, typename C::Core& sm, int& gs,
-                                          int& qs) {
-    const int n = min(gs, C::kB);
-    const int base = gs - n;
+    const int n = min(qs, C::kB);
+    const int base = qs - n;
     const bool have = (int)threadIdx.x < n;
-    float a = 0.f, b = 0.f, c = 0.f;
+    float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f);
+    float t = 0.f;
+    uint32_t w = 0;
     uint64_t ray = 0;
     if (have) {
         const int q = base + threadIdx.x;
-        a = sm.go[0][q];
-        b = sm.go[1][q];
-        c = sm.go[2][q];
+        o = f3(sm.qo[0][q], sm.qo[1][q], sm.qo[2][q]);
+        d = f3(sm.qd[0][q], sm.qd[1][q], sm.qd[2][q]);
+        t = sm.qt[q];
+        w = sm.qw[q];
+        ray = sm.qray[q];
+    }
+    // the barrier both ends the reads of the popped entries and publishes the new size: no
+    // thread appends (atomicAdd on qsize, then writes from `base` on) before it, and none read
+    // qsize since the barrier that closed the last append
+    if (threadIdx.x == 0) sm.qsize = base;
+    __syncthreads();
+    // shade the pending mirror hit (its record is out), find the next hit, record it, and queue it
+    // again when it is another mirror below the depth limit
+    bool again = false;
+    Segment next{f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 1.f), 0.f, 0};
+    Hit h2{-1, 0.f, 0u};
+    const uint64_t r = ray & kRayMask;
+    if (have) {
+        const int depth = (int)(ray >> kDepthShift);
+        const Segment g{o, d, depth == 0 ? kTminSun : kTminBounce, depth};
+        const Hit h{(int)(w & kPrimMask), t, w >> kTypeShift};
+        const Prim p = load_prim(A.prims, (uint32_t)h.best);
+        if (shade_mirror<C>(A, r, p, A.optics[h.best], g, h, next)) {
+            h2.best = find_closest<C>(A, sm, next.o, next.d, next.tmin, own_mirror(p, h, g, next), h2.t, h2.type);
+            if (h2.best >= 0) {
+                const Prim p2 = load_prim(A.prims, (uint32_t)h2.best);
+                float4 rec;
+                int slot;
+                again = classify(p2, next, h2, rec, slot);
+                if (slot >= 0) emit<C>(A, k, r, slot, rec, (uint32_t)h2.best);
+            }
+        }
+    }
+    push(sm, again, r | ((uint64_t)next.depth << kDepthShift), next.o, next.d, h2.t,
+         (uint32_t)h2.best | (h2.type << kTypeShift));
+    return base + __syncthreads_count(again);
+}
+
+// One batch of up to kB rays from the top of the generation queue (element-list launches; gs entries):
+// their whole paths, on full warps.  Returns the queue size after it; a warp that is done goes on to
+// the next tile.  (Directions and box tests in a batch of their own, with a second queue and four
+// more barriers, left the later batches fuller -- 82 % of the single parabolic heliostat's queued rays
+// meet a box -- but measured slower: 307 us against 305 per 16M rays, 8.4 against 7.7 per 200,000.)
+template <class C>
+__device__ __forceinline__ int path_batch(const typename C::Args& A, const Sink& k, typename C::Core& sm, int gs) {
+    const int n = min(gs, C::kB);
+    const int base = gs - n;
+    const bool have = (int)threadIdx.x < n;
+    float hu = 0.f, hv = 0.f;
+    uint64_t ray = 0;
+    if (have) {
+        const int q = base + threadIdx.x;
+        hu = sm.go[0][q];
+        hv = sm.go[1][q];
         ray = sm.gray[q];
     }
-    __syncthreads();
     if (threadIdx.x == 0) sm.gsize = base;
-    const float3 o = f3(a, b, c);
-    float3 d = f3(0.f, 0.f, 1.f);
-    uint32_t m = 0;
-    if (have) {
-        d = sun_direction<C>(A, sm.sun, ray);
-        m = candidates(sm.flat, o, d, kTminSun);
-    }
-    push(sm, m != 0u, ray, o, d, 0.0f, m);
-    qs += __syncthreads_count(m != 0u);
-    gs = base;
+    __syncthreads();
+    if (have) flat_path<C>(A, k, sm, ray, hu, hv);
+    return base;
 }
 
 // Phase B: one full batch of queued rays, or with `flush` one of what remains; false when there is
-// none.  The bounce queue is below kB before each generation batch (a bounce batch never grows it), so
-// neither queue exceeds 2 kB.  qs and gs are the sizes of the bounce and generation queues, carried in
-// registers by every thread of the CTA (equal in all of them); the caller has passed a barrier since
-// the last append.
+// none.  Neither queue exceeds 2 kB: a tile appends at most kB to less than kB, and a bounce batch
+// never grows its queue.  n is the size of the launch's queue (the bounce queue, or the generation
+// queue of element lists), carried in a register by every thread of the CTA (equal in all of them);
+// the caller has passed a barrier since the last append.
 // The kernels call this and trace_tile from one place each, in one loop: with a copy of the batches
 // behind every tile loop and every drain the field kernel was 163 KB of code, and its warps waited
 // for instructions wherever they left each other's phase.
 template <class C>
 __device__ __forceinline__ bool phase_b(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool flush,
-                                        int& qs, int& gs) {
-    if (qs >= C::kB || (flush && qs > 0 && gs == 0)) {
-        qs = bounce_batch<C>(A, k, sm, qs);
-        return true;
-    }
-    if constexpr (C::kFlat) {
-        if (gs >= C::kB || (flush && gs > 0)) {
-            gen_batch<C>(A, k, sm, gs, qs);
-            return true;
-        }
-    }
-    return false;
+                                        int& n) {
+    if (!(n >= C::kB || (flush && n > 0))) return false;
+    if constexpr (C::kFlat) n = path_batch<C>(A, k, sm, n);
+    else n = bounce_batch<C>(A, k, sm, n);
+    return true;
 }
 
 // Per-CTA setup of an instance: sun frame and the kFlat element list or the grid descriptors into
@@ -1327,20 +1327,21 @@ template <class C>
 __device__ __forceinline__ void load_instance_smem(const typename C::Args& A, typename C::Core& sm) {
     if (threadIdx.x < sizeof(SunFrame) / 4)
         reinterpret_cast<uint32_t*>(&sm.sun)[threadIdx.x] = reinterpret_cast<const uint32_t*>(A.sun)[threadIdx.x];
-    if (C::kFlat && threadIdx.x < kFlatMax) {
-        const int nprim = A.sun->n_prims;
-        const int k = threadIdx.x;
-        if (k < nprim) {
+    if constexpr (C::kFlat) {
+        // each record by a thread of its own: one latency (the element count comes with the launch)
+        const int k = (int)threadIdx.x & (kFlatMax - 1);
+        if (threadIdx.x < kFlatMax && k < A.n_prims) {
             // a kFlat scene's nodes are its leaves in element order
             const Node nd = A.nodes[k];
-            sm.flat.prim[k] = A.prims[k];
-            sm.flat.optics[k] = A.optics[k];
             sm.flat.box[k].lo = nd.lo;
             sm.flat.box[k].hi = nd.hi;
             sm.flat.type[k] = (__float_as_uint(nd.lo.w) >> kTypeShift) & 7u;
-            sm.reach[k] = reach_rect(*A.sun, cone_tan(*A.sun), box_span(*A.sun, make_float4(0.f, 0.f, 0.f, 0.f), nd.lo, nd.hi));
+        } else if (threadIdx.x >= 32 && threadIdx.x < 32 + kFlatMax && k < A.n_prims) {
+            sm.flat.prim[k] = A.prims[k];
+        } else if (threadIdx.x >= 64 && threadIdx.x < 64 + kFlatMax && k < A.n_prims) {
+            sm.flat.optics[k] = A.optics[k];
         }
-        if (k == 0) sm.flat.n = min(nprim, kFlatMax);
+        if (threadIdx.x == 96) sm.flat.n = A.n_prims;
     }
     if (C::kAccel == kAccelGrid && threadIdx.x < sizeof(GridDesc) / 4)
         reinterpret_cast<uint32_t*>(&sm.grid)[threadIdx.x] = reinterpret_cast<const uint32_t*>(A.grid)[threadIdx.x];
@@ -1411,11 +1412,11 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
 }
 
 // Phase A of one tile (rays A.ray_begin + tile * kB ...); phase_b runs its full batches.
-// `stage` is the kDense staging area of element-list launches (unused otherwise); qs, gs: the queue
-// sizes (see phase_b).
+// `stage` is the kDense staging area of element-list launches (unused otherwise); qs: the queue size
+// (see phase_b).
 template <class C>
 __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink& k, typename C::Core& sm,
-                                           typename C::Stage* stage, uint64_t tile, int& qs, int& gs) {
+                                           typename C::Stage* stage, uint64_t tile, int& qs) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t kk = tile * C::kB + threadIdx.x;
     uint64_t pos = kk;
@@ -1435,44 +1436,46 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
     if (kk < A.count) {
         hu = halton2(ray);
         hv = halton3_tab(ray, sm.t6, A.h3t12);
+        // the next tile's rays follow these (and so do their table entries): its 1 KB of sums into L1,
+        // a line per thread (16 M rays of the single parabolic heliostat 305 -> 298 us)
+        if (A.h3t12 && threadIdx.x < C::kB / 32 + 1)
+            prefetch_l1(A.h3t12 + ((uint32_t)ray + C::kB + 31u * threadIdx.x) % kH3T12);
         o = sun_point(sm.sun, hu, hv);
         const int nr = sm.flat.n;
 #pragma unroll
         for (int e = 0; e < kFlatMax; ++e) {
             if (e >= nr) break;
-            want |= in_rect(sm.reach[e], hu, hv);
+            want |= in_rect(sm.sun.reach[e], hu, hv);
         }
     }
     __syncwarp();
-    push_gen(sm, want, ray, o);
-    if constexpr (C::kDense) {
-        // the warp's 32 x 80 B of records leave as 5 fully coalesced 512-byte rows: record e of the
-        // warp is slot e mod 5 of ray e / 5, the staged sun-plane record for slot 0, else empty
-        float4* wh = stage->rec0 + warp * 32;
-        wh[lane] = make_float4(0.0f, o.x, o.y, o.z);
-        __syncwarp();
+    push_gen(sm, want, ray, hu, hv);
+    if constexpr (C::kDense && C::kFlat) {
         const uint64_t warp_first = tile * C::kB + (uint64_t)warp * 32;
+        float4* rows = stage->row + warp * 32 * kMaxDepth;
+        rows[lane * kMaxDepth] = make_float4(0.0f, o.x, o.y, o.z);
+        __syncwarp();
         if (warp_first < A.count) {
             const uint32_t n_rec = (uint32_t)min((uint64_t)32, A.count - warp_first) * kMaxDepth;
             float4* gh = A.hits + warp_first * kMaxDepth;
 #pragma unroll
-            for (int s = 0; s < kMaxDepth; ++s) {
-                const uint32_t e = (uint32_t)(s * 32 + lane);
-                const uint32_t r = e / kMaxDepth;
-                if (e < n_rec) gh[e] = (e == r * kMaxDepth) ? wh[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < kMaxDepth; ++q) {
+                const uint32_t e = (uint32_t)(q * 32 + lane);
+                if (e < n_rec) gh[e] = rows[e];
             }
             if (A.ids) {
                 uint32_t* gi = A.ids + warp_first * kMaxDepth;
 #pragma unroll
-                for (int s = 0; s < kMaxDepth; ++s) {
-                    const uint32_t e = (uint32_t)(s * 32 + lane);
+                for (int q = 0; q < kMaxDepth; ++q) {
+                    const uint32_t e = (uint32_t)(q * 32 + lane);
                     if (e < n_rec) gi[e] = kNoElement;
                 }
             }
         }
+        __syncwarp();  // the rows are read before the warp's next tile writes them
     }
     // the barrier before phase B counts this tile's appends to the generation queue
-    gs += __syncthreads_count(want);
+    qs += __syncthreads_count(want);
 }
 
 }  // namespace

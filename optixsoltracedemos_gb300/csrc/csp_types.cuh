@@ -73,6 +73,7 @@ struct alignas(16) SunFrame {
     float cos_theta, sigma, tan_pad;
     float omc;     // 1 - cos_theta as 2 sin^2(half angle / 2) (shape 2, the accurate cone sampler)
     int shape, n_prims, pad1, pad2;
+    float4 reach[8];  // scenes of up to 8 elements: reach rectangle of each (reach_rect, csp_trace.cuh)
 };
 
 // Uniform 2D grid over a planar heliostat field (the alternative to the BVH for field-like

@@ -76,3 +76,17 @@ def test_element_records_built_in_ranges_equal_serial(tmp_path):
     r = subprocess.run([exe, field], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.startswith("OK 10001 elements, error 'element 1031:"), r.stdout
+
+
+def test_rsqrt_near_1_equals_square_root_and_division(tmp_path):
+    """The closed form of 1 / sqrt(x) near 1 gives both roundings' bits, over its whole range."""
+    import shutil
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    exe = str(tmp_path / "rsqrt_near_1_check")
+    subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I",
+                    os.path.join(root, "optixsoltracedemos_gb300", "csrc"), "-I", cuda_inc,
+                    os.path.join(root, "tests", "cpp", "rsqrt_near_1_check.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "0 mismatches", r.stdout
