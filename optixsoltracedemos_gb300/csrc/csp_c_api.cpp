@@ -121,6 +121,11 @@ void System::release() {
     d_csums = nullptr;
     d_crecords = nullptr;
     cap_compact_rays = cap_crecords = 0;
+    cudaFree(d_cring);
+    d_cring = nullptr;
+    cap_cring = 0;
+    if (h_ctotal) cudaFreeHost(h_ctotal);
+    h_ctotal = nullptr;
     cudaFree(d_flux);
     cudaFree(d_fstats);
     d_flux = nullptr;
@@ -378,6 +383,99 @@ int System::run_to_host(float* dst, uint32_t* ids_dst) {
     return CSP_OK;
 }
 
+// Chunks of a compact run: traced and compacted on `stream` while the chunk before is copied on
+// `copy_stream`, a quarter of the run each, at most 2^20 rays (84 MB of rows, still in L2 when they are
+// compacted) and at least 2^17 (below, a chunk's kernels are shorter than its launches).  A copy costs
+// about 2 us besides its bytes (16 B per ray of the single parabolic heliostat at the host link's ~190
+// GB/s), so the counts follow in one copy at the end.  4M rays of that heliostat: 577 us in one piece,
+// 445 in eight chunks, 436 in four, 444 to 464 with chunks that start at 2^18 or 2^17 and double; the
+// copies alone 349 us.
+constexpr uint64_t kCompactChunkMin = 1u << 17, kCompactChunkMax = 1u << 20;
+constexpr int kCompactRing = 2;  // chunks whose records wait on the device for their copy
+
+int System::ensure_compact_buffers(uint64_t n) {
+    if (n <= cap_compact_rays) return CSP_OK;
+    cudaFree(d_cpoints);
+    cudaFree(d_ccounts);
+    cudaFree(d_csums);
+    d_cpoints = nullptr;
+    d_ccounts = nullptr;
+    d_csums = nullptr;
+    cap_compact_rays = 0;
+    int rc;
+    if ((rc = cuda_status(dev_alloc((void**)&d_cpoints, std::max<uint64_t>(n, 1) * 3 * sizeof(float)), "cudaMalloc")))
+        return rc;
+    if ((rc = cuda_status(dev_alloc((void**)&d_ccounts, std::max<uint64_t>(n, 1)), "cudaMalloc"))) return rc;
+    // the offsets of the whole run, or of the chunks in flight
+    const size_t sums = std::max<size_t>(compact_blocks(n) + 1, kCompactRing * (kCompactChunkMax / 256 + 1));
+    if ((rc = cuda_status(dev_alloc((void**)&d_csums, sums * sizeof(unsigned long long)), "cudaMalloc"))) return rc;
+    cap_compact_rays = n;
+    return CSP_OK;
+}
+
+// The chunked form of run_to_host_compact, for a host buffer that holds any run's records.
+int System::run_compact_chunks(float* points, uint8_t* counts, float* records, uint64_t chunk, uint64_t* n_records) {
+    struct Chunk {
+        uint64_t begin = 0, count = 0;
+    } prev;
+    cudaEvent_t done[kCompactRing] = {}, copied[kCompactRing] = {};
+    int rc = CSP_OK;
+    for (int i = 0; i < kCompactRing && !rc; ++i) {
+        rc = cuda_status(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming), "cudaEventCreate");
+        if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming), "cudaEventCreate");
+    }
+    const uint64_t n = num_rays;
+    uint64_t total = 0, next = 0;
+    for (uint64_t k = 0; !rc; ++k) {
+        Chunk cur;
+        if (next < n) {
+            // queue chunk k: it takes the place of chunk k - 2, whose copy was queued a turn ago
+            cur = Chunk{next, std::min(chunk, n - next)};
+            next += cur.count;
+            const int at = (int)(k % kCompactRing);
+            unsigned long long* sums = d_csums + (chunk / 256 + 1) * at;
+            const float4* rows = d_hits + cur.begin * kMaxDepth;
+            rc = cuda_status(launch_trace(args(cur.begin, cur.count), stream), "trace_kernel");
+            if (!rc && k >= kCompactRing)
+                rc = cuda_status(cudaStreamWaitEvent(stream, copied[at], 0), "cudaStreamWaitEvent");
+            if (!rc)
+                rc = cuda_status(launch_compact_count(rows, cur.count, d_cpoints + 3 * cur.begin, d_ccounts + cur.begin,
+                                                      sums, h_ctotal + at, stream),
+                                 "compact_count_kernel");
+            if (!rc)
+                rc = cuda_status(launch_compact_write(rows, cur.count, d_ccounts + cur.begin, sums,
+                                                      d_cring + 4 * chunk * at, stream),
+                                 "compact_write_kernel");
+            if (!rc) rc = cuda_status(cudaEventRecord(done[at], stream), "cudaEventRecord");
+        }
+        if (prev.count && !rc) {
+            // copy chunk k - 1, whose number of records is known once it is done
+            const int at = (int)((k - 1) % kCompactRing);
+            if ((rc = cuda_status(cudaEventSynchronize(done[at]), "compact chunk"))) break;
+            const uint64_t found = *(volatile unsigned long long*)(h_ctotal + at);
+            auto copy = [&](void* dst, const void* src, size_t bytes, const char* what) {
+                if (!rc && bytes)
+                    rc = cuda_status(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, copy_stream), what);
+            };
+            copy(points + 3 * prev.begin, d_cpoints + 3 * prev.begin, prev.count * 3 * sizeof(float), "D2H points");
+            copy(records + 4 * total, d_cring + 4 * chunk * at, found * sizeof(float4), "D2H records");
+            if (!rc) rc = cuda_status(cudaEventRecord(copied[at], copy_stream), "cudaEventRecord");
+            total += found;
+        }
+        prev = cur;
+        if (!cur.count) break;
+    }
+    if (!rc) rc = cuda_status(cudaMemcpyAsync(counts, d_ccounts, n, cudaMemcpyDeviceToHost, copy_stream), "D2H counts");
+    const int rc1 = cuda_status(cudaStreamSynchronize(copy_stream), "compact copy");
+    const int rc2 = cuda_status(cudaStreamSynchronize(stream), "compact trace");
+    for (int i = 0; i < kCompactRing; ++i) {
+        if (done[i]) cudaEventDestroy(done[i]);
+        if (copied[i]) cudaEventDestroy(copied[i]);
+    }
+    if (n_records) *n_records = total;
+    return rc ? rc : (rc1 ? rc1 : rc2);
+}
+
 // Trace, then move the records in compact form: per ray its sun-plane point and the number of its
 // further records, and those records in ray order (kernels in csp_kernels.cu).  Nothing is copied
 // when the records exceed `capacity`; *n_records then tells how many there are.
@@ -388,30 +486,42 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     const uint64_t n = num_rays;
-    if (n > cap_compact_rays) {
-        cudaFree(d_cpoints);
-        cudaFree(d_ccounts);
-        cudaFree(d_csums);
-        d_cpoints = nullptr;
-        d_ccounts = nullptr;
-        d_csums = nullptr;
-        cap_compact_rays = 0;
-        if ((rc = cuda_status(dev_alloc((void**)&d_cpoints, std::max<uint64_t>(n, 1) * 3 * sizeof(float)), "cudaMalloc")))
-            return rc;
-        if ((rc = cuda_status(dev_alloc((void**)&d_ccounts, std::max<uint64_t>(n, 1)), "cudaMalloc"))) return rc;
-        if ((rc = cuda_status(dev_alloc((void**)&d_csums, (compact_blocks(n) + 1) * sizeof(unsigned long long)),
-                              "cudaMalloc")))
-            return rc;
-        cap_compact_rays = n;
-    }
+    if ((rc = ensure_compact_buffers(n))) return rc;
     const auto t0 = std::chrono::steady_clock::now();
+    auto timed = [&] {
+        time_trace = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        return CSP_OK;
+    };
+    // in chunks when no number of records can exceed the capacity (else it is known only after the
+    // whole trace, and nothing may be copied before) and the run is longer than the first one
+    const uint64_t chunk = std::min(kCompactChunkMax, std::max(kCompactChunkMin, (n / 4 + 255) / 256 * 256));
+    if (n > chunk && capacity / 4 >= n) {
+        const uint64_t need = 4 * chunk * kCompactRing;
+        if (need > cap_cring) {
+            cudaFree(d_cring);
+            d_cring = nullptr;
+            cap_cring = 0;
+            if (dev_alloc((void**)&d_cring, need * sizeof(float4)) == cudaSuccess) cap_cring = need;
+            else cudaGetLastError();
+        }
+        if (!h_ctotal &&
+            host_alloc((void**)&h_ctotal, kCompactRing * sizeof(unsigned long long)) != cudaSuccess) {
+            h_ctotal = nullptr;
+            cudaGetLastError();
+        }
+        if (cap_cring >= need && h_ctotal) {  // else in one piece, which needs less memory
+            rc = run_compact_chunks(points, counts, records, chunk, n_records);
+            return rc ? rc : timed();
+        }
+    }
     if ((rc = cuda_status(launch_trace(args(0, n), stream), "trace_kernel"))) return rc;
-    if ((rc = cuda_status(launch_compact_count(d_hits, n, d_ccounts, d_csums, stream), "compact_count_kernel")))
+    if ((rc = cuda_status(launch_compact_count(d_hits, n, d_cpoints, d_ccounts, d_csums, nullptr, stream),
+                          "compact_count_kernel")))
         return rc;
     unsigned long long total = 0;
-    if ((rc = cuda_status(cudaMemcpyAsync(&total, d_csums + compact_blocks(n), sizeof total, cudaMemcpyDeviceToHost,
-                                          stream),
-                          "D2H record count")))
+    if (n && (rc = cuda_status(cudaMemcpyAsync(&total, d_csums + compact_blocks(n), sizeof total, cudaMemcpyDeviceToHost,
+                                               stream),
+                               "D2H record count")))
         return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "compact count"))) return rc;
     if (n_records) *n_records = total;
@@ -424,7 +534,7 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
             return rc;
         cap_crecords = total;
     }
-    if ((rc = cuda_status(launch_compact_write(d_hits, n, d_csums, d_cpoints, d_crecords, stream), "compact_write_kernel")))
+    if ((rc = cuda_status(launch_compact_write(d_hits, n, d_ccounts, d_csums, d_crecords, stream), "compact_write_kernel")))
         return rc;
     if (n && (rc = cuda_status(cudaMemcpyAsync(points, d_cpoints, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, stream),
                                "D2H points")))
@@ -436,8 +546,7 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
                                    "D2H records")))
         return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "compact copy"))) return rc;
-    time_trace = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    return CSP_OK;
+    return timed();
 }
 
 double sun_plane_area(const SunFrame& f) {

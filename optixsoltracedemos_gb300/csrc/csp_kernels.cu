@@ -245,13 +245,6 @@ __global__ void __launch_bounds__(kFluxBlock) flux_records_kernel(const float4* 
 // slot 0, then the ray's further records in slots 1.. (stage 1 or 2, so x != 0), then empty slots.
 constexpr int kCompactBlock = 256;
 
-__device__ __forceinline__ uint32_t row_records(const float4* __restrict__ hits, uint64_t r) {
-    uint32_t c = 0;
-#pragma unroll
-    for (int s = 1; s < kMaxDepth; ++s) c += __ldg(&hits[r * kMaxDepth + s].x) != 0.0f ? 1u : 0u;
-    return c;
-}
-
 // Block-wide exclusive prefix of v (kCompactBlock threads); `total` receives the block's sum.
 __device__ uint32_t block_exclusive(uint32_t v, uint32_t* scratch, uint32_t& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -271,62 +264,94 @@ __device__ uint32_t block_exclusive(uint32_t v, uint32_t* scratch, uint32_t& tot
     return before + x - v;
 }
 
-// Records beyond slot 0 of every ray, and their sum per block.
+// Sun-plane points (3 floats per ray), the number of records beyond slot 0 of every ray, and their sum
+// per block: the one pass that reads every row.  A block's 256 rows are read as 1,280 coalesced
+// records (five loads in flight per thread); points and counts are put together in shared memory.
 __global__ void __launch_bounds__(kCompactBlock) compact_count_kernel(const float4* __restrict__ hits, uint64_t n,
+                                                                      float* __restrict__ points,
                                                                       uint8_t* __restrict__ counts,
                                                                       unsigned long long* __restrict__ block_sums) {
-    __shared__ uint32_t scratch[kCompactBlock / 32];
-    const uint64_t r = (uint64_t)blockIdx.x * kCompactBlock + threadIdx.x;
-    uint32_t c = 0;
-    if (r < n) {
-        c = row_records(hits, r);
-        counts[r] = (uint8_t)c;
+    __shared__ uint32_t scratch[kCompactBlock / 32], cnt[kCompactBlock];
+    __shared__ alignas(16) float pts[3 * kCompactBlock];
+    const uint64_t r0 = (uint64_t)blockIdx.x * kCompactBlock;
+    const uint32_t rows = (uint32_t)min((uint64_t)kCompactBlock, n - r0);
+    cnt[threadIdx.x] = 0;
+    __syncthreads();
+    float4 rec[kMaxDepth];
+#pragma unroll
+    for (int q = 0; q < kMaxDepth; ++q) {
+        const uint32_t e = threadIdx.x + q * kCompactBlock;
+        rec[q] = e < rows * kMaxDepth ? __ldg(hits + r0 * kMaxDepth + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+#pragma unroll
+    for (int q = 0; q < kMaxDepth; ++q) {
+        const uint32_t e = threadIdx.x + q * kCompactBlock, row = e / kMaxDepth;
+        if (e == row * kMaxDepth) {
+            pts[3 * row] = rec[q].y;
+            pts[3 * row + 1] = rec[q].z;
+            pts[3 * row + 2] = rec[q].w;
+        } else if (rec[q].x != 0.0f) {
+            atomicAdd(&cnt[row], 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t c = cnt[threadIdx.x];
+    if (threadIdx.x < rows) counts[r0 + threadIdx.x] = (uint8_t)c;
+    float* out = points + 3 * r0;
+    if (rows == kCompactBlock && threadIdx.x < 3 * kCompactBlock / 4)
+        reinterpret_cast<float4*>(out)[threadIdx.x] = reinterpret_cast<const float4*>(pts)[threadIdx.x];
+    else if (rows < kCompactBlock)
+        for (uint32_t k = threadIdx.x; k < 3 * rows; k += kCompactBlock) out[k] = pts[k];
     uint32_t total;
     block_exclusive(c, scratch, total);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-// In place: block sums -> exclusive block offsets, the grand total after the last block.
-__global__ void __launch_bounds__(1024) compact_scan_kernel(unsigned long long* __restrict__ sums, uint64_t nb) {
-    __shared__ unsigned long long part[1024];
-    const uint64_t chunk = (nb + 1023) / 1024;
-    const uint64_t c0 = min(nb, (uint64_t)threadIdx.x * chunk), c1 = min(nb, c0 + chunk);
-    unsigned long long s = 0;
-    for (uint64_t c = c0; c < c1; ++c) s += sums[c];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const unsigned long long v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0ull;
+// In place: block sums -> exclusive block offsets, the grand total after the last block and, when
+// given, in pinned host memory (a copy of its own would queue behind the record copies of the chunk
+// before).
+__global__ void __launch_bounds__(1024) compact_scan_kernel(unsigned long long* __restrict__ sums, uint64_t nb,
+                                                            unsigned long long* host_total) {
+    __shared__ unsigned long long part[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long before = 0;
+    for (uint64_t c0 = 0; c0 < nb; c0 += 1024) {
+        const uint64_t c = c0 + threadIdx.x;
+        const unsigned long long v = c < nb ? sums[c] : 0ull;
+        unsigned long long x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) part[warp] = x;
         __syncthreads();
-        part[threadIdx.x] += v;
+        unsigned long long w = part[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        const unsigned long long all = __shfl_sync(0xffffffffu, w, 31);
+        const unsigned long long mine = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+        if (c < nb) sums[c] = before + (warp ? mine : 0ull) + x - v;
+        before += all;
         __syncthreads();
     }
-    unsigned long long run = part[threadIdx.x] - s;
-    for (uint64_t c = c0; c < c1; ++c) {
-        const unsigned long long k = sums[c];
-        sums[c] = run;
-        run += k;
+    if (threadIdx.x == 0) {
+        sums[nb] = before;
+        if (host_total) *host_total = before;
     }
-    if (threadIdx.x == 1023) sums[nb] = part[1023];
 }
 
-// Sun-plane points (3 floats per ray) and the records beyond slot 0, in ray order.
+// The records beyond slot 0, in ray order.
 __global__ void __launch_bounds__(kCompactBlock) compact_write_kernel(const float4* __restrict__ hits, uint64_t n,
+                                                                      const uint8_t* __restrict__ counts,
                                                                       const unsigned long long* __restrict__ offsets,
-                                                                      float* __restrict__ points,
                                                                       float4* __restrict__ records) {
     __shared__ uint32_t scratch[kCompactBlock / 32];
     const uint64_t r = (uint64_t)blockIdx.x * kCompactBlock + threadIdx.x;
-    uint32_t c = 0;
-    if (r < n) c = row_records(hits, r);
+    const uint32_t c = r < n ? counts[r] : 0u;
     uint32_t total;
     const uint32_t ex = block_exclusive(c, scratch, total);
-    if (r >= n) return;
-    const float4 p = __ldg(&hits[r * kMaxDepth]);
-    points[3 * r] = p.y;
-    points[3 * r + 1] = p.z;
-    points[3 * r + 2] = p.w;
     const uint64_t o = offsets[blockIdx.x] + ex;
     for (uint32_t s = 0; s < c; ++s) records[o + s] = __ldg(&hits[r * kMaxDepth + 1 + s]);
 }
@@ -392,21 +417,22 @@ cudaError_t launch_trace(const TraceArgs& args, cudaStream_t stream) {
 
 uint64_t compact_blocks(uint64_t n) { return (n + kCompactBlock - 1) / kCompactBlock; }
 
-cudaError_t launch_compact_count(const float4* hits, uint64_t n, uint8_t* counts, unsigned long long* block_sums,
+cudaError_t launch_compact_count(const float4* hits, uint64_t n, float* points, uint8_t* counts,
+                                 unsigned long long* block_sums, unsigned long long* host_total,
                                  cudaStream_t stream) {
     const uint64_t nb = compact_blocks(n);
     if (nb == 0) return cudaSuccess;
     if (nb > 0x7FFFFFFFull) return cudaErrorInvalidValue;
-    compact_count_kernel<<<(unsigned)nb, kCompactBlock, 0, stream>>>(hits, n, counts, block_sums);
-    compact_scan_kernel<<<1, 1024, 0, stream>>>(block_sums, nb);
+    compact_count_kernel<<<(unsigned)nb, kCompactBlock, 0, stream>>>(hits, n, points, counts, block_sums);
+    compact_scan_kernel<<<1, 1024, 0, stream>>>(block_sums, nb, host_total);
     return cudaGetLastError();
 }
 
-cudaError_t launch_compact_write(const float4* hits, uint64_t n, const unsigned long long* block_offsets, float* points,
-                                 float4* records, cudaStream_t stream) {
+cudaError_t launch_compact_write(const float4* hits, uint64_t n, const uint8_t* counts,
+                                 const unsigned long long* block_offsets, float4* records, cudaStream_t stream) {
     const uint64_t nb = compact_blocks(n);
     if (nb == 0) return cudaSuccess;
-    compact_write_kernel<<<(unsigned)nb, kCompactBlock, 0, stream>>>(hits, n, block_offsets, points, records);
+    compact_write_kernel<<<(unsigned)nb, kCompactBlock, 0, stream>>>(hits, n, counts, block_offsets, records);
     return cudaGetLastError();
 }
 

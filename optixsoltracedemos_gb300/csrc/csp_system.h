@@ -83,6 +83,11 @@ struct System {
     unsigned long long* d_csums = nullptr;
     float4* d_crecords = nullptr;
     uint64_t cap_compact_rays = 0, cap_crecords = 0;
+    // chunked runs: records of the chunks between their trace and their copy, and those chunks' totals
+    // (pinned host memory)
+    float4* d_cring = nullptr;
+    uint64_t cap_cring = 0;
+    unsigned long long* h_ctotal = nullptr;
     uint32_t* d_flux = nullptr;              // csp_flux_map counts
     unsigned long long* d_fstats = nullptr;  // [4]
     size_t cap_flux = 0;
@@ -112,6 +117,8 @@ struct System {
     int trace_async(cudaStream_t st);
     int run();
     int run_to_host(float* dst, uint32_t* ids);
+    int ensure_compact_buffers(uint64_t n);
+    int run_compact_chunks(float* points, uint8_t* counts, float* records, uint64_t chunk, uint64_t* n_records);
     int run_to_host_compact(float* points, uint8_t* counts, float* records, uint64_t capacity, uint64_t* n_records);
     int flux_map(uint32_t nx, uint32_t ny, uint32_t* counts, double dni, double* flux, bool staged = false);
 };
