@@ -45,6 +45,8 @@ namespace csp {
 namespace {
 
 // offsets 32-byte aligned: the kernels read records and boxes 32 bytes at a time
+constexpr size_t kPoolElements = 4096;    // elements of a run from which its host builds use the batch's threads
+constexpr size_t kKeepElements = 400000;  // elements (of ~160 B) of a run whose host records stay allocated
 size_t align32(size_t x) { return (x + 31) & ~(size_t)31; }
 
 // Tuned launch parameters per (device model, kernel build, kernel group, ray-count class), shared
@@ -244,7 +246,7 @@ int Batch::add_scene(const csp_element* el, uint32_t n, uint32_t* id) {
         return r;
     };
     rc = put(s.d_topo, s.base.nodes, "upload topology");
-    if (!rc && s.grid.valid) rc = put(s.d_cells, s.grid.cell_start, "upload grid cells");
+    if (!rc && s.grid.valid) rc = put(s.d_cells, s.grid.cells, "upload grid cells");
     if (!rc && s.grid.valid) rc = put(s.d_items, s.grid.items, "upload grid items");
     if (!rc && s.grid.valid) rc = put(s.d_global, s.grid.global, "upload grid globals");
     if (rc) {
@@ -293,6 +295,7 @@ int Batch::layout(int si) {
     max_nodes = 0;
     n_sg = 0;
     max_n = 0;
+    max_field_cells = 0;
     size_t off = 0;
     for (size_t i = 0; i < n; ++i) {
         const BScene& s = scenes[inst[i].scene];
@@ -308,10 +311,10 @@ int Batch::layout(int si) {
         off += align32(ne * sizeof(Aabb));
         p.prune = off;
         off += align32(ne * sizeof(Aabb));
-        if (p.group == kAccelGrid && !inst[i].poses.empty()) {
+        if (p.group == kAccelGrid && !inst[i].poses.empty() && !builds[i].grid.on_device) {
             const HostGrid& hg = builds[i].grid;
             p.cells = off;
-            off += align32(hg.cell_start.size() * sizeof(uint32_t));
+            off += align32(hg.cells.size() * sizeof(uint2));
             p.items = off;
             off += align32(hg.items.size() * sizeof(Aabb));
             p.global = off;
@@ -349,6 +352,11 @@ int Batch::layout(int si) {
         if (place[i].sg_slot >= 0) {
             place[i].sgrid = off;
             off += align32(sungrid_bytes(count_of(i)));
+        }
+        if (const InstBuild* ib = own_field(i)) {
+            place[i].field = off;
+            off += align32(field_bytes(ib->grid.nx, ib->grid.ny, ib->grid.cap_items));
+            max_field_cells = std::max(max_field_cells, ib->grid.nx * ib->grid.ny);
         }
     }
     zero_off = off;
@@ -437,11 +445,28 @@ int Batch::build_instance(size_t i, std::string& err) {
     const BInst& b = inst[i];
     if (b.poses.empty()) return CSP_OK;
     InstBuild& ib = builds[i];
-    int rc = build_elements(b.poses.data(), count_of(i), ib.hs, err);
+    GridStats stats;
+    int rc = build_elements(b.poses.data(), count_of(i), ib.hs, err, &stats);
     if (rc) return rc;
     ib.grid = HostGrid{};
-    if (!scenes[b.scene].flat) build_grid(ib.hs, ib.grid);
+    if (!scenes[b.scene].flat) plan_grid(ib.hs, stats, ib.grid);
     return CSP_OK;
+}
+
+// The build of instance i, if its own field grid is left to the device.
+const InstBuild* Batch::own_field(size_t i) const {
+    if (inst[i].poses.empty() || place[i].group != kAccelGrid || !builds[i].grid.on_device) return nullptr;
+    return &builds[i];
+}
+
+// Device arrays of instance i's sun grid (and field grid, if the device builds it).
+void Batch::job_of(size_t i, SunGridJob& gj) const {
+    const Place& p = place[i];
+    sungrid_place(dev(p.sgrid), count_of(i), gj);
+    if (const InstBuild* ib = own_field(i))
+        field_place(dev(p.field), ib->grid, reinterpret_cast<const Aabb*>(dev(p.prune)), gj);
+    gj.sun = reinterpret_cast<const SunFrame*>(dev(p.sun));
+    gj.aabbs = reinterpret_cast<const Aabb*>(dev(p.aabbs));
 }
 
 const HostScene& Batch::scene_of(size_t i) const {
@@ -463,9 +488,9 @@ void Batch::fill_instance(size_t i) {
     std::memcpy(h_stage + p.optics, src->optics.data(), ne * sizeof(Optics));
     std::memcpy(h_stage + p.aabbs, src->aabbs.data(), ne * sizeof(Aabb));
     std::memcpy(h_stage + p.prune, src->prune.data(), ne * sizeof(Aabb));
-    if (p.group == kAccelGrid && !b.poses.empty()) {
+    if (p.group == kAccelGrid && !b.poses.empty() && !builds[i].grid.on_device) {
         const HostGrid& hg = builds[i].grid;
-        std::memcpy(h_stage + p.cells, hg.cell_start.data(), hg.cell_start.size() * sizeof(uint32_t));
+        std::memcpy(h_stage + p.cells, hg.cells.data(), hg.cells.size() * sizeof(uint2));
         std::memcpy(h_stage + p.items, hg.items.data(), hg.items.size() * sizeof(Aabb));
         if (!hg.global.empty()) std::memcpy(h_stage + p.global, hg.global.data(), hg.global.size() * sizeof(Aabb));
     }
@@ -494,9 +519,7 @@ void Batch::fill_instance(size_t i) {
     std::memcpy(h_stage + sunjob_off + i * sizeof(SunJob), &sj, sizeof sj);
     if (p.sg_slot >= 0) {
         SunGridJob gj;
-        sungrid_place(dev(p.sgrid), ne, gj);
-        gj.sun = sj.out;
-        gj.aabbs = sj.aabbs;
+        job_of(i, gj);
         std::memcpy(h_stage + sgjob_off + (size_t)p.sg_slot * sizeof(SunGridJob), &gj, sizeof gj);
     }
 }
@@ -534,15 +557,18 @@ void Batch::fill_descs(const int* block, const std::vector<bool>* sample, std::v
         d.args.sgrid = nullptr;
         if (p.sg_slot >= 0) {
             SunGridJob gj;
-            sungrid_place(dev(p.sgrid), count_of(i), gj);
+            job_of(i, gj);
             d.args.sgrid = gj.desc;
+            if (own_field(i))
+                d.grid = grid_desc(grid_of(i), gj.field_cells, gj.field_items, gj.aabbs + (count_of(i) - 1));
         }
         if (g == kAccelGrid) {
             const bool own = !b.poses.empty();
             const BScene& bs = scenes[b.scene];
-            d.grid = grid_desc(grid_of(i), own ? reinterpret_cast<const uint32_t*>(dev(p.cells)) : bs.d_cells,
-                               own ? reinterpret_cast<const Aabb*>(dev(p.items)) : bs.d_items,
-                               own ? reinterpret_cast<const Aabb*>(dev(p.global)) : bs.d_global);
+            if (!own_field(i))
+                d.grid = grid_desc(grid_of(i), own ? reinterpret_cast<const uint2*>(dev(p.cells)) : bs.d_cells,
+                                   own ? reinterpret_cast<const Aabb*>(dev(p.items)) : bs.d_items,
+                                   own ? reinterpret_cast<const Aabb*>(dev(p.global)) : bs.d_global);
             d.args.grid = reinterpret_cast<const GridDesc*>(dev(desc_off[g] + p.slot * sizeof(InstanceDesc)) +
                                                             offsetof(InstanceDesc, grid));
         }
@@ -595,7 +621,8 @@ int Batch::enqueue_scene_setup(cudaStream_t st) {
                                                    (int)inst.size(), max_n, st),
                           "prepare_sun_batch_kernel")))
         return rc;
-    return cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(dev(sgjob_off)), n_sg, max_n, st),
+    return cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(dev(sgjob_off)), n_sg, max_n,
+                                            max_field_cells, st),
                        "sun grid build");
 }
 
@@ -735,31 +762,20 @@ int Batch::run_async() {
     // host builds of the instances with their own poses, then the copies into the staging image,
     // both parallel over instances
     const size_t n = inst.size();
-    builds.clear();
-    builds.resize(n);
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t workers = std::min<size_t>(std::min<size_t>(hw, 64), n);
+    builds.resize(n);  // the vectors of the last run's are reused
+    size_t total = 0;
+    for (size_t i = 0; i < n; ++i) total += inst[i].poses.empty() ? 0 : count_of(i);
+    const bool pooled = total >= kPoolElements && n > 1;
+    if (pooled && !pool.started()) pool.start(std::min(63u, std::max(2u, std::thread::hardware_concurrency()) - 1));
     auto parallel = [&](auto&& fn) {
-        std::vector<int> wrc(workers, CSP_OK);
-        std::vector<std::string> werr(workers);
-        auto work = [&](size_t w) {
-            for (size_t i = w; i < n; i += workers) {
-                const int r = fn(i, werr[w]);
-                if (r) {
-                    wrc[w] = r;
-                    werr[w] = "instance " + std::to_string(i) + ": " + werr[w];
-                    return;
-                }
-            }
-        };
-        if (workers <= 1) work(0);
-        else {
-            std::vector<std::thread> th;
-            for (size_t w = 0; w < workers; ++w) th.emplace_back(work, w);
-            for (auto& t : th) t.join();
-        }
-        for (size_t w = 0; w < workers; ++w)
-            if (wrc[w]) return set_error(wrc[w], werr[w]);
+        std::vector<int> irc(n, CSP_OK);
+        std::vector<std::string> ierr(n);
+        auto one = [&](size_t i) { irc[i] = fn(i, ierr[i]); };
+        if (pooled) pool.run(n, one);
+        else
+            for (size_t i = 0; i < n; ++i) one(i);
+        for (size_t i = 0; i < n; ++i)
+            if (irc[i]) return set_error(irc[i], "instance " + std::to_string(i) + ": " + ierr[i]);
         return (int)CSP_OK;
     };
     if ((rc = parallel([&](size_t i, std::string& err) { return build_instance(i, err); }))) return rc;
@@ -777,15 +793,20 @@ int Batch::run_async() {
     std::vector<uint64_t> tb[kBatchGroups];
     fill_descs(block, nullptr, desc, tb);
     write_descs(desc, tb, h_stage);
-    builds.clear();  // everything the device needs is in the staging image now
-    builds.shrink_to_fit();
+    // everything the device needs is in the staging image now; the builds of small batches keep their
+    // memory for the next run
+    if (total > kKeepElements) {
+        builds.clear();
+        builds.shrink_to_fit();
+    }
     uint64_t tiles[kBatchGroups];
     for (int g = 0; g < kBatchGroups; ++g) tiles[g] = tb[g][n_group[g]];
 
     // graph signature: everything the captured launches depend on besides the staged contents
     std::vector<uint64_t> sig = {(uint64_t)(uintptr_t)d_comp, (uint64_t)(uintptr_t)S.d_up, (uint64_t)(uintptr_t)S.h_stage,
                                  (uint64_t)(uintptr_t)S.h_result, up_bytes, zero_bytes, res_bytes, n, nx, ny,
-                                 desc_off[0], zero_off, res_off};
+                                 desc_off[0], zero_off, res_off, (uint64_t)n_refit, (uint64_t)max_nodes,
+                                 (uint64_t)n_sg, (uint64_t)max_n, (uint64_t)max_field_cells};
     for (int g = 0; g < kBatchGroups; ++g) {
         sig.push_back(tiles[g]);
         sig.push_back((uint64_t)n_group[g]);

@@ -10,6 +10,7 @@
 
 #include "csp_c_api.h"
 #include "csp_kernels.cuh"
+#include "csp_pool.h"
 #include "csp_scene.h"
 
 namespace csp {
@@ -20,7 +21,7 @@ struct BScene {
     Node* d_topo = nullptr; // topology on the device (links; boxes of the scene's own poses)
     bool flat = false;      // <= kFlatListMax elements: shared-memory element list kernel
     HostGrid grid;          // field grid of the scene's own poses (valid for field-like scenes)
-    uint32_t* d_cells = nullptr;
+    uint2* d_cells = nullptr;
     Aabb* d_items = nullptr;
     Aabb* d_global = nullptr;
 };
@@ -44,7 +45,8 @@ struct BInst {
 // Byte offsets of one instance's arrays in the device arena (and the staging image).
 struct Place {
     size_t prims = 0, optics = 0, aabbs = 0, prune = 0, nodes = 0, sun = 0, counts = 0, stats = 0;
-    size_t cells = 0, items = 0, global = 0;  // own grid arrays (instances with poses in the grid group)
+    size_t cells = 0, items = 0, global = 0;  // own grid arrays, where the host built them (poses, grid group)
+    size_t field = 0;                         // own grid built on the device
     size_t sgrid = 0;  // sun-ray candidate grid (BVH and grid groups), built on the device
     int sg_slot = -1;  // index of its build job
     int rf_slot = -1;  // index of its refit job (grid instances have no nodes)
@@ -106,8 +108,10 @@ struct Batch {
     size_t desc_off[kBatchGroups] = {}, tb_off[kBatchGroups] = {}, refit_off = 0, sunjob_off = 0, counter_off = 0;
     size_t sgjob_off = 0;
     int n_group[kBatchGroups] = {};
+    int max_field_cells = 0;  // of the field grids that the device builds
     int n_sg = 0, max_n = 0;  // sun grid build jobs; largest element count of the instances
     std::vector<InstBuild> builds;  // per instance, during a run (instances with poses)
+    HostPool pool;                  // host builds of batches of kPoolElements or more
     int n_refit = 0, max_nodes = 0;  // refit jobs and their largest node count
 
     double time_setup = 0.0, time_trace = 0.0;  // of the last completed run
@@ -122,6 +126,8 @@ struct Batch {
     uint32_t count_of(size_t i) const;
     int layout(int s);
     int build_instance(size_t i, std::string& err);
+    const InstBuild* own_field(size_t i) const;
+    void job_of(size_t i, SunGridJob& gj) const;
     const HostScene& scene_of(size_t i) const;
     const HostGrid& grid_of(size_t i) const;
     void fill_instance(size_t i);

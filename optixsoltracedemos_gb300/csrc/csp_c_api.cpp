@@ -91,9 +91,14 @@ System::~System() { release(); }
 void System::release() {
     if (device >= 0) cudaSetDevice(device);
     cudaFree(d_nodes);
-    cudaFree(d_prims);
-    cudaFree(d_optics);
-    cudaFree(d_aabbs);
+    cudaFree(d_records);
+    if (h_records) cudaFreeHost(h_records);
+    d_records = h_records = nullptr;
+    cap_records = 0;
+    cudaFree(d_field);
+    d_field = nullptr;
+    cap_field = 0;
+    topology = false;
     cudaFree(d_sun);
     cudaFree(d_hits);
     cudaFree(d_ids);
@@ -127,18 +132,17 @@ void System::release() {
     if (h_ctotal) cudaFreeHost(h_ctotal);
     h_ctotal = nullptr;
     cudaFree(d_flux);
-    cudaFree(d_fstats);
-    d_flux = nullptr;
-    d_fstats = nullptr;
+    if (h_flux) cudaFreeHost(h_flux);
+    d_flux = h_flux = nullptr;
     cap_flux = 0;
     d_nodes = nullptr;
     d_prims = nullptr;
     d_optics = nullptr;
-    d_aabbs = nullptr;
+    d_aabbs = d_prune = nullptr;
     d_sun = nullptr;
     d_hits = nullptr;
     d_ids = nullptr;
-    cap_nodes = cap_prims = cap_optics = cap_aabbs = 0;
+    cap_nodes = 0;
     cap_rays = 0;
     ids_allocated = false;
     if (ev0) cudaEventDestroy(ev0);
@@ -161,29 +165,102 @@ int System::ensure_streams() {
     return cuda_status(cudaEventCreate(&ev1), "cudaEventCreate");
 }
 
-int System::upload_scene() {
+// Element count from which a scene's records are packed on the handle's host threads (10,001 elements
+// take 904 us on one thread of a 16-core host; a whole update() takes 323 us on sixteen).
+constexpr uint32_t kPoolElements = 2048;
+
+// Element records of the current elements, packed and put on the device, and the plan of their field
+// grid.  An error of the elements or of the plan leaves the device's scene (and `grid`) as it was; from
+// there on the handle counts as not initialized until the caller is through.
+int System::build_scene(const char* not_planar) {
+    const uint32_t n = (uint32_t)elements.size();
     int rc;
-    if ((rc = upload(d_prims, cap_prims, scene.prims, stream, "upload prims"))) return rc;
-    if ((rc = upload(d_optics, cap_optics, scene.optics, stream, "upload optics"))) return rc;
-    if ((rc = upload(d_aabbs, cap_aabbs, scene.aabbs, stream, "upload aabbs"))) return rc;
-    if ((rc = upload(d_nodes, cap_nodes, scene.nodes, stream, "upload bvh"))) return rc;
-    if (!d_sun) {
-        if ((rc = cuda_status(dev_alloc((void**)&d_sun, sizeof(SunFrame)), "cudaMalloc sun"))) return rc;
+    // the last upload from h_records may still be under way if its call failed after it
+    if (records_busy && (rc = cuda_status(cudaStreamSynchronize(stream), "element records"))) return rc;
+    records_busy = false;
+    auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t o_optics = align(n * sizeof(Prim)), o_aabbs = o_optics + align(n * sizeof(Optics));
+    const size_t o_prune = o_aabbs + align(n * sizeof(Aabb)), bytes = o_prune + align(n * sizeof(Aabb));
+    if (bytes > cap_records) {
+        // larger buffers next to the old ones, which still serve the device's scene
+        unsigned char *d = nullptr, *h = nullptr;
+        if ((rc = cuda_status(dev_alloc((void**)&d, bytes), "cudaMalloc element records"))) return rc;
+        if ((rc = cuda_status(host_alloc((void**)&h, bytes), "cudaHostAlloc element records"))) {
+            cudaFree(d);
+            return rc;
+        }
+        initialized = false;
+        cudaFree(d_records);
+        if (h_records) cudaFreeHost(h_records);
+        d_records = d;
+        h_records = h;
+        cap_records = bytes;
     }
-    return CSP_OK;
+    auto stage = [&](uint32_t b, uint32_t e) {
+        std::memcpy(h_records + b * sizeof(Prim), &scene.prims[b], (e - b) * sizeof(Prim));
+        std::memcpy(h_records + o_optics + b * sizeof(Optics), &scene.optics[b], (e - b) * sizeof(Optics));
+        std::memcpy(h_records + o_aabbs + b * sizeof(Aabb), &scene.aabbs[b], (e - b) * sizeof(Aabb));
+        std::memcpy(h_records + o_prune + b * sizeof(Aabb), &scene.prune[b], (e - b) * sizeof(Aabb));
+    };
+    std::string err;
+    GridStats stats;
+    if (n >= kPoolElements) {
+        if (!pool.started()) pool.start(std::min(15u, std::max(2u, std::thread::hardware_concurrency()) - 1));
+        rc = build_elements(
+            elements.data(), n, scene, err,
+            [this](size_t tasks, const std::function<void(size_t)>& body) { pool.run(tasks, body); }, &stats, stage);
+    } else {
+        rc = build_elements(elements.data(), n, scene, err, &stats);
+        if (!rc) stage(0, n);
+    }
+    if (rc) return fail(rc, err);
+    // the grid holds one set of poses: planned anew for these
+    HostGrid plan;
+    if (accel != CSP_ACCEL_BVH) plan_grid(scene, stats, plan);
+    if (accel == CSP_ACCEL_GRID && !plan.valid && n > kFlatListMax) return fail(CSP_ERR_BAD_SCENE, not_planar);
+    initialized = false;
+    grid = std::move(plan);
+    d_prims = reinterpret_cast<Prim*>(d_records);
+    d_optics = reinterpret_cast<Optics*>(d_records + o_optics);
+    d_aabbs = reinterpret_cast<Aabb*>(d_records + o_aabbs);
+    d_prune = reinterpret_cast<Aabb*>(d_records + o_prune);
+    records_busy = true;
+    return cuda_status(cudaMemcpyAsync(d_records, h_records, bytes, cudaMemcpyHostToDevice, stream), "upload records");
 }
 
-// Field grid on the device: the cell arrays (when `arrays`) and the descriptor.
-int System::upload_grid(bool arrays) {
+int System::upload_nodes() {
+    // scenes that trace through the field grid need no BVH
+    if (grid.valid) return CSP_OK;
+    if (topology) refit_bvh(scene);
+    else build_bvh(scene);
+    topology = true;
+    return upload(d_nodes, cap_nodes, scene.nodes, stream, "upload bvh");
+}
+
+// Field grid on the device: its arrays where the host built them, else room for the device's, and the
+// descriptor.
+int System::upload_grid() {
     if (!grid.valid) return CSP_OK;
     int rc;
-    if (arrays) {
-        if ((rc = upload(d_cells, cap_cells, grid.cell_start, stream, "upload grid cells"))) return rc;
+    if (grid.on_device) {
+        const size_t bytes = field_bytes(grid.nx, grid.ny, grid.cap_items);
+        if (bytes > cap_field) {
+            cudaFree(d_field);
+            d_field = nullptr;
+            cap_field = 0;
+            if ((rc = cuda_status(dev_alloc((void**)&d_field, bytes), "cudaMalloc field grid"))) return rc;
+            cap_field = bytes;
+        }
+        SunGridJob at{};
+        field_place(d_field, grid, d_prune, at);
+        grid_host = csp::grid_desc(grid, at.field_cells, at.field_items, d_aabbs + (scene.prims.size() - 1));
+    } else {
+        if ((rc = upload(d_cells, cap_cells, grid.cells, stream, "upload grid cells"))) return rc;
         if ((rc = upload(d_items, cap_items, grid.items, stream, "upload grid items"))) return rc;
         if ((rc = upload(d_global, cap_global, grid.global, stream, "upload grid globals"))) return rc;
+        grid_host = csp::grid_desc(grid, d_cells, d_items, d_global);
     }
     if (!d_grid && (rc = cuda_status(dev_alloc((void**)&d_grid, sizeof(GridDesc)), "cudaMalloc grid"))) return rc;
-    grid_host = csp::grid_desc(grid, d_cells, d_items, d_global);
     return cuda_status(cudaMemcpyAsync(d_grid, &grid_host, sizeof(GridDesc), cudaMemcpyHostToDevice, stream),
                        "upload grid");
 }
@@ -223,10 +300,12 @@ int System::build_sungrid() {
     sungrid_place(d_sgrid, n, sgjob_host);
     sgjob_host.sun = d_sun;
     sgjob_host.aabbs = d_aabbs;
+    const int field_cells = grid.valid && grid.on_device ? grid.nx * grid.ny : 0;
+    if (field_cells) field_place(d_field, grid, d_prune, sgjob_host);
     if ((rc = cuda_status(cudaMemcpyAsync(d_sgjob, &sgjob_host, sizeof(SunGridJob), cudaMemcpyHostToDevice, stream),
                           "upload sun grid job")))
         return rc;
-    return cuda_status(launch_sungrid_build(d_sgjob, 1, (int)n, stream), "sun grid build");
+    return cuda_status(launch_sungrid_build(d_sgjob, 1, (int)n, field_cells, stream), "sun grid build");
 }
 
 int System::ensure_hit_buffers() {
@@ -262,19 +341,16 @@ int System::initialize() {
         if ((rc = cuda_status(cudaMemsetAsync(d_tile_counter, 0, 2 * sizeof(unsigned int), stream), "memset"))) return rc;
     }
     h3t12 = halton3_table();
-    std::string err;
-    if ((rc = build_elements(elements.data(), (uint32_t)elements.size(), scene, err))) return fail(rc, err);
-    build_bvh(scene);
-    grid = HostGrid{};
-    if (accel != CSP_ACCEL_BVH) build_grid(scene, grid);
-    if (accel == CSP_ACCEL_GRID && !grid.valid && elements.size() > kFlatListMax)
-        return fail(CSP_ERR_BAD_SCENE, "the scene is not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
-    if ((rc = upload_scene())) return rc;
-    if ((rc = upload_grid(true))) return rc;
+    topology = false;
+    if ((rc = build_scene("the scene is not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)"))) return rc;
+    if (!d_sun && (rc = cuda_status(dev_alloc((void**)&d_sun, sizeof(SunFrame)), "cudaMalloc sun"))) return rc;
+    if ((rc = upload_nodes())) return rc;
+    if ((rc = upload_grid())) return rc;
     if ((rc = prepare_sun())) return rc;
     if ((rc = build_sungrid())) return rc;
     if ((rc = ensure_hit_buffers())) return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "initialize"))) return rc;
+    records_busy = false;
     initialized = true;
     time_setup = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return CSP_OK;
@@ -285,21 +361,17 @@ int System::update() {
     if (!initialized) return fail(CSP_ERR_STATE, "update() before initialize()");
     if (elements.size() != scene.prims.size())
         return fail(CSP_ERR_STATE, "update() needs the element count of initialize(); call initialize() again");
-    std::string err;
-    int rc = build_elements(elements.data(), (uint32_t)elements.size(), scene, err);
-    if (rc) return fail(rc, err);
-    refit_bvh(scene);
-    // the grid holds one set of poses: rebuilt for the new ones
-    grid = HostGrid{};
-    if (accel != CSP_ACCEL_BVH) build_grid(scene, grid);
-    if (accel == CSP_ACCEL_GRID && !grid.valid && elements.size() > kFlatListMax)
-        return fail(CSP_ERR_BAD_SCENE, "the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
-    if ((rc = upload_scene())) return rc;
-    if ((rc = upload_grid(true))) return rc;
+    int rc = build_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
+    if (rc) return rc;
+    if ((rc = upload_nodes())) return rc;
+    if ((rc = upload_grid())) return rc;
     if ((rc = prepare_sun())) return rc;
     if ((rc = build_sungrid())) return rc;
     if ((rc = ensure_hit_buffers())) return rc;
-    return cuda_status(cudaStreamSynchronize(stream), "update");
+    if ((rc = cuda_status(cudaStreamSynchronize(stream), "update"))) return rc;
+    records_busy = false;
+    initialized = true;
+    return CSP_OK;
 }
 
 TraceArgs System::args(uint64_t begin, uint64_t count) const {
@@ -567,36 +639,43 @@ int System::flux_map(uint32_t nx, uint32_t ny, uint32_t* counts, double dni, dou
     if (!initialized || !d_hits) return fail(CSP_ERR_STATE, "flux map before initialize()/run()");
     if (nx == 0 || ny == 0 || (uint64_t)nx * ny > (1u << 26)) return fail(CSP_ERR_INVALID_ARGUMENT, "bad flux grid");
     const size_t nb = (size_t)nx * ny;
+    // device: counters and map, zeroed in one go; pinned host memory: the map and the sun frame
+    constexpr size_t kStats = 4 * sizeof(unsigned long long);
+    const size_t map_bytes = nb * sizeof(uint32_t);
     int rc;
     if (nb > cap_flux) {
         cudaFree(d_flux);
-        d_flux = nullptr;
+        if (h_flux) cudaFreeHost(h_flux);
+        d_flux = h_flux = nullptr;
         cap_flux = 0;
-        if ((rc = cuda_status(dev_alloc((void**)&d_flux, nb * sizeof(uint32_t)), "cudaMalloc flux map"))) return rc;
+        if ((rc = cuda_status(dev_alloc((void**)&d_flux, kStats + map_bytes), "cudaMalloc flux map"))) return rc;
+        if ((rc = cuda_status(host_alloc((void**)&h_flux, sizeof(SunFrame) + map_bytes), "cudaHostAlloc flux map"))) {
+            cudaFree(d_flux);
+            d_flux = h_flux = nullptr;
+            return rc;
+        }
         cap_flux = nb;
     }
-    if (!d_fstats && (rc = cuda_status(dev_alloc((void**)&d_fstats, 4 * sizeof(unsigned long long)), "cudaMalloc")))
-        return rc;
     FluxTarget F;
     flux_target(elements.back(), nx, ny, F);
-    F.counts = d_flux;
-    F.stats = d_fstats;
+    F.stats = reinterpret_cast<unsigned long long*>(d_flux);
+    F.counts = reinterpret_cast<uint32_t*>(d_flux + kStats);
     F.staged = staged ? 1 : 0;
-    if ((rc = cuda_status(cudaMemsetAsync(d_flux, 0, nb * sizeof(uint32_t), stream), "memset flux"))) return rc;
-    if ((rc = cuda_status(cudaMemsetAsync(d_fstats, 0, 4 * sizeof(unsigned long long), stream), "memset"))) return rc;
+    if ((rc = cuda_status(cudaMemsetAsync(d_flux, 0, kStats + map_bytes, stream), "memset flux"))) return rc;
     if ((rc = cuda_status(launch_flux_records(d_hits, num_rays * kMaxDepth, F, stream), "flux_records_kernel")))
         return rc;
-    std::vector<uint32_t> host(nb);
-    if ((rc = cuda_status(cudaMemcpyAsync(host.data(), d_flux, nb * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
+    if ((rc = cuda_status(cudaMemcpyAsync(h_flux + sizeof(SunFrame), F.counts, map_bytes, cudaMemcpyDeviceToHost, stream),
                           "D2H flux map")))
         return rc;
-    SunFrame f;
-    if ((rc = cuda_status(cudaMemcpyAsync(&f, d_sun, sizeof(f), cudaMemcpyDeviceToHost, stream), "D2H sun frame")))
+    if ((rc = cuda_status(cudaMemcpyAsync(h_flux, d_sun, sizeof(SunFrame), cudaMemcpyDeviceToHost, stream),
+                          "D2H sun frame")))
         return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "flux map"))) return rc;
-    if (counts) std::copy(host.begin(), host.end(), counts);
+    const SunFrame& f = *reinterpret_cast<const SunFrame*>(h_flux);
+    const uint32_t* host = reinterpret_cast<const uint32_t*>(h_flux + sizeof(SunFrame));
+    if (counts) std::copy(host, host + nb, counts);
     if (flux)
-        counts_to_flux(host.data(), nb, dni, sun_plane_area(f), num_rays, flux_bin_area(elements.back(), nx, ny), flux);
+        counts_to_flux(host, nb, dni, sun_plane_area(f), num_rays, flux_bin_area(elements.back(), nx, ny), flux);
     return CSP_OK;
 }
 

@@ -8,6 +8,8 @@
 
 namespace csp {
 
+struct HostGrid;
+
 // Bounds-check builds (-DCSP_BOUNDS_CHECK): the failed-check sites recorded on the current device by
 // the kernels of each translation unit, read and cleared (0 in other builds).
 #ifdef CSP_BOUNDS_CHECK
@@ -81,6 +83,14 @@ struct SunGridJob {
     float4* rect;             // [n] candidate rectangles
     float4* reach_rect;       // [n] reach rectangles
     uint32_t* reach;          // [kReachRaster^2 / 32]
+    // the state's field grid, when the device builds it (cells null: not)
+    const Aabb* prune;        // [n] pruning boxes
+    uint2* field_cells;       // [field_nx * field_ny]
+    uint32_t* field_alloc;
+    Aabb* field_items;        // [field_cap]
+    float field_x0, field_y0, field_inv;
+    int field_nx, field_ny;
+    uint32_t field_cap;
     float4* item_rect;        // [cap_items]
     Aabb* item_box;           // [cap_items]
     uint32_t* global_id;      // [n]
@@ -98,9 +108,15 @@ size_t sungrid_bytes(uint32_t n);
 // aligned); fills every SunGridJob field except sun and aabbs.
 void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job);
 
-// Build the sun grids of n_jobs scene states (jobs: device array) on `stream`; max_n =
-// the largest element count among the jobs.
-cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, cudaStream_t stream);
+// Build the sun grids (and field grids, where the jobs have them) of n_jobs scene states (jobs: device
+// array) on `stream`; max_n, max_field_cells = the largest element count and field_nx * field_ny
+// among the jobs (0: no field grids).
+cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, int max_field_cells,
+                                 cudaStream_t stream);
+// Bytes of a device-built field grid of nx * ny cells and cap items (256-byte aligned parts), and its
+// place in `base` (256-byte aligned): fills the job's field members.
+size_t field_bytes(int nx, int ny, uint32_t cap);
+void field_place(unsigned char* base, const HostGrid& g, const Aabb* prune, SunGridJob& job);
 
 // Trace rays [ray_begin, ray_begin + count): generation, closest-hit search, shading, the dense
 // hit-record write.  Scenes of up to 8 elements take the shared-memory element list path; larger ones

@@ -85,6 +85,13 @@ CSP_HD float3 normalize_unit(float3 v) {
 CSP_HD float3 reflect(float3 i, float3 n) { return sub(i, scale(dot(n, i), scale(2.0f, n))); }
 CSP_HD float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
+// Box that registers an element in the field grid: its pruning box in xy, widened by 2e-5 |coordinate|
+// + 5 cm.
+CSP_HD float4 grid_box(float4 lo, float4 hi) {
+    const float m = 2e-5f * fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))) + 0.05f;
+    return make_float4(lo.x - m, lo.y - m, hi.x + m, hi.y + m);
+}
+
 // ------------------------------------------------------------------------------------ Philox ---
 struct u32x4 {
     uint32_t x, y, z, w;

@@ -274,22 +274,23 @@ int check_count(uint32_t n, std::string& err) {
 }
 
 void size_scene(uint32_t n, HostScene& s) {
-    s.prims.assign(n, Prim{});
-    s.optics.assign(n, Optics{});
-    s.aabbs.assign(n, Aabb{});
-    s.prune.assign(n, Aabb{});
-    s.types.assign(n, 0);
+    s.prims.resize(n);
+    s.optics.resize(n);
+    s.aabbs.resize(n);
+    s.prune.resize(n);
+    s.types.resize(n);
 }
 
 // Packs elements [begin, end); returns the index of the first that fails (and its status and
 // message), or end.
 uint32_t pack_range(const csp_element* el, uint32_t n, uint32_t begin, uint32_t end, HostScene& s, int& rc,
-                    const char*& why) {
+                    const char*& why, GridStats* stats) {
     for (uint32_t i = begin; i < end; ++i) {
         rc = pack_element(el[i], i + 1 == n, s.types[i], s.aabbs[i], s.prims[i], s.optics[i], &s.prune[i], why);
         // the exact box carries its element and entity type (the sun grid's candidate tests)
         s.aabbs[i].lo.w = u2f((s.types[i] << kTypeShift) | i);
         if (rc) return i;
+        if (stats && i + 1 < n) stats->add(s.prune[i]);
     }
     return end;
 }
@@ -304,30 +305,68 @@ int pack_error(const csp_element* el, uint32_t i, int rc, const char* why, std::
 
 }  // namespace
 
-int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err) {
+void GridStats::add(const Aabb& prune) {
+    const float4 b = grid_box(prune.lo, prune.hi);
+    const float side = std::max(b.z - b.x, b.w - b.y);
+    finite = finite && std::isfinite(side) && std::isfinite(prune.lo.z) && std::isfinite(prune.hi.z);
+    ++n;
+    sum += side;
+    min = std::min(min, side);
+    max = std::max(max, side);
+    x0 = std::min(x0, b.x);
+    y0 = std::min(y0, b.y);
+    x1 = std::max(x1, b.z);
+    y1 = std::max(y1, b.w);
+    z0 = std::min(z0, prune.lo.z);
+    z1 = std::max(z1, prune.hi.z);
+}
+
+void GridStats::add(const GridStats& o) {
+    finite = finite && o.finite;
+    n += o.n;
+    sum += o.sum;
+    min = std::min(min, o.min);
+    max = std::max(max, o.max);
+    x0 = std::min(x0, o.x0);
+    y0 = std::min(y0, o.y0);
+    x1 = std::max(x1, o.x1);
+    y1 = std::max(y1, o.y1);
+    z0 = std::min(z0, o.z0);
+    z1 = std::max(z1, o.z1);
+}
+
+int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, GridStats* stats) {
     int rc = check_count(n, err);
     if (rc) return rc;
     size_scene(n, s);
     const char* why = "";
-    const uint32_t bad = pack_range(el, n, 0, n, s, rc, why);
+    const uint32_t bad = pack_range(el, n, 0, n, s, rc, why, stats);
     return bad < n ? pack_error(el, bad, rc, why, err) : CSP_OK;
 }
 
-int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, const ParallelFor& pf) {
+int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, const ParallelFor& pf,
+                   GridStats* stats, const std::function<void(uint32_t, uint32_t)>& packed) {
     int rc = check_count(n, err);
     if (rc) return rc;
     size_scene(n, s);
-    const size_t chunks = (n + kBuildChunk - 1) / kBuildChunk;
+    constexpr uint32_t kRange = kBuildChunk / 2;
+    const size_t chunks = (n + kRange - 1) / kRange;
     std::vector<uint32_t> bad(chunks);
     std::vector<int> status(chunks, CSP_OK);
     std::vector<const char*> whys(chunks, "");
+    std::vector<GridStats> part(stats ? chunks : 0);
     pf(chunks, [&](size_t c) {
-        const uint32_t b = (uint32_t)(c * kBuildChunk), e = std::min<uint32_t>(n, b + kBuildChunk);
-        bad[c] = pack_range(el, n, b, e, s, status[c], whys[c]);
-        if (bad[c] == e) bad[c] = n;
+        const uint32_t b = (uint32_t)(c * kRange), e = std::min<uint32_t>(n, b + kRange);
+        bad[c] = pack_range(el, n, b, e, s, status[c], whys[c], stats ? &part[c] : nullptr);
+        if (bad[c] == e) {
+            bad[c] = n;
+            if (packed) packed(b, e);
+        }
     });
-    for (size_t c = 0; c < chunks; ++c)
+    for (size_t c = 0; c < chunks; ++c) {
         if (bad[c] < n) return pack_error(el, bad[c], status[c], whys[c], err);
+        if (stats) stats->add(part[c]);
+    }
     return CSP_OK;
 }
 
@@ -526,6 +565,62 @@ constexpr size_t kGridMaxCells = 1u << 22;
 
 }  // namespace
 
+// Grid over [X0, X1] x [Y0, Y1] in cells of about `cell` (larger ones past kGridMaxCells), the layer
+// [zmin, zmax].
+static void set_bounds(HostGrid& g, double X0, double Y0, double X1, double Y1, float zmin, float zmax, double& cell) {
+    double nxd = std::ceil((X1 - X0) / cell), nyd = std::ceil((Y1 - Y0) / cell);
+    while (nxd * nyd > (double)kGridMaxCells) {
+        cell = (double)(float)(cell * 1.5);
+        nxd = std::ceil((X1 - X0) / cell);
+        nyd = std::ceil((Y1 - Y0) / cell);
+    }
+    g.nx = std::max(1, (int)nxd);
+    g.ny = std::max(1, (int)nyd);
+    g.x0 = (float)X0;
+    g.y0 = (float)Y0;
+    g.cell = (float)cell;
+    g.inv_cell = 1.0f / g.cell;
+    g.x1 = g.x0 + (float)g.nx * g.cell;
+    g.y1 = g.y0 + (float)g.ny * g.cell;
+    // the float bounds must still cover every registered box
+    while ((double)g.x1 < X1 || (double)g.y1 < Y1 || (double)g.x0 > X0 || (double)g.y0 > Y0) {
+        g.x0 = std::nextafter(g.x0, -FLT_MAX);
+        g.y0 = std::nextafter(g.y0, -FLT_MAX);
+        g.x1 = std::nextafter(g.x1, FLT_MAX);
+        g.y1 = std::nextafter(g.y1, FLT_MAX);
+    }
+    // the layer: every gridded surface lies in its pruning box
+    const float mz = 1e-5f * std::max(std::fabs(zmin), std::fabs(zmax)) + 0.01f;
+    g.zlo = std::nextafter(zmin - mz, -FLT_MAX);
+    g.zhi = std::nextafter(zmax + mz, FLT_MAX);
+}
+
+// Whether mirrors in [z0, z1] over the given horizontal extent form a thin layer.
+static bool thin_layer(double z0, double z1, double extent) { return !(z1 - z0 > 0.25 * extent); }
+
+void plan_grid(const HostScene& s, const GridStats& st, HostGrid& g) {
+    g = HostGrid{};
+    if (s.prims.size() <= kFlatListMax) return;
+    double cell = (double)(float)(1.4 * (st.sum / st.n));
+    // the device indexes cells in float: far fewer than 2^24 / 100 of them, and coordinates whose rounding
+    // is below a thousandth of one
+    const double far = std::max(std::max(std::fabs(st.x0), std::fabs(st.x1)), std::max(std::fabs(st.y0), std::fabs(st.y1)));
+    if (!st.finite || !(cell > 0) || !(st.max <= 4.0 * cell) || !(st.max <= 8.0 * 1.4 * st.min) ||
+        !(far <= 4000.0 * cell)) {
+        build_grid(s, g);
+        return;
+    }
+    if (!(st.x1 > st.x0) || !(st.y1 > st.y0)) return;
+    if (!thin_layer(st.z0, st.z1, std::max((double)st.x1 - st.x0, (double)st.y1 - st.y0))) return;
+    set_bounds(g, st.x0, st.y0, st.x1, st.y1, st.z0, st.z1, cell);
+    // a box of side w touches at most floor(w / cell) + 2 cells along an axis (the hundredth covers the
+    // rounding of the cell index)
+    const uint32_t k = (uint32_t)(st.max / cell + 0.01) + 2;
+    g.cap_items = st.n * k * k;
+    g.on_device = true;
+    g.valid = true;
+}
+
 void build_grid(const HostScene& s, HostGrid& g) {
     g = HostGrid{};
     const uint32_t n = (uint32_t)s.prims.size();
@@ -562,32 +657,8 @@ void build_grid(const HostScene& s, HostGrid& g) {
         zmax = std::max(zmax, s.prune[i].hi.z);
     }
     if (!(X1 > X0) || !(Y1 > Y0)) return;
-    if ((double)zmax - (double)zmin > 0.25 * std::max(X1 - X0, Y1 - Y0)) return;  // not a thin layer
-    double nxd = std::ceil((X1 - X0) / cell), nyd = std::ceil((Y1 - Y0) / cell);
-    while (nxd * nyd > (double)kGridMaxCells) {
-        cell = (double)(float)(cell * 1.5);
-        nxd = std::ceil((X1 - X0) / cell);
-        nyd = std::ceil((Y1 - Y0) / cell);
-    }
-    g.nx = std::max(1, (int)nxd);
-    g.ny = std::max(1, (int)nyd);
-    g.x0 = (float)X0;
-    g.y0 = (float)Y0;
-    g.cell = (float)cell;
-    g.inv_cell = 1.0f / g.cell;
-    g.x1 = g.x0 + (float)g.nx * g.cell;
-    g.y1 = g.y0 + (float)g.ny * g.cell;
-    // the float bounds must still cover every registered box
-    while ((double)g.x1 < X1 || (double)g.y1 < Y1 || (double)g.x0 > X0 || (double)g.y0 > Y0) {
-        g.x0 = std::nextafter(g.x0, -FLT_MAX);
-        g.y0 = std::nextafter(g.y0, -FLT_MAX);
-        g.x1 = std::nextafter(g.x1, FLT_MAX);
-        g.y1 = std::nextafter(g.y1, FLT_MAX);
-    }
-    // the layer: every gridded surface lies in its pruning box
-    const float mz = 1e-5f * std::max(std::fabs(zmin), std::fabs(zmax)) + 0.01f;
-    g.zlo = std::nextafter(zmin - mz, -FLT_MAX);
-    g.zhi = std::nextafter(zmax + mz, FLT_MAX);
+    if (!thin_layer(zmin, zmax, std::max(X1 - X0, Y1 - Y0))) return;
+    set_bounds(g, X0, Y0, X1, Y1, zmin, zmax, cell);
     auto cell_range = [&](uint32_t i, int& ax, int& ay, int& bx, int& by) {
         ax = std::max(0, std::min(g.nx - 1, (int)std::floor((lo[2 * i] - g.x0) / cell)));
         ay = std::max(0, std::min(g.ny - 1, (int)std::floor((lo[2 * i + 1] - g.y0) / cell)));
@@ -606,10 +677,13 @@ void build_grid(const HostScene& s, HostGrid& g) {
         for (int y = ay; y <= by; ++y)
             for (int x = ax; x <= bx; ++x) count[(size_t)y * g.nx + x]++;
     }
-    g.cell_start.assign((size_t)g.nx * g.ny + 1, 0);
-    for (size_t c = 0; c < (size_t)g.nx * g.ny; ++c) g.cell_start[c + 1] = g.cell_start[c] + count[c];
-    g.items.assign(g.cell_start.back(), Aabb{});
-    std::vector<uint32_t> fill(g.cell_start.begin(), g.cell_start.end() - 1);
+    g.cells.resize((size_t)g.nx * g.ny);
+    uint32_t total = 0;
+    for (size_t c = 0; c < g.cells.size(); ++c) {
+        g.cells[c] = make_uint2(total, total);  // y: the fill's cursor, at the end of the cell's items when done
+        total += count[c];
+    }
+    g.items.assign(total, Aabb{});
     auto item = [&](uint32_t i) {
         Aabb a = s.aabbs[i];
         a.lo.w = u2f((s.types[i] << kTypeShift) | i);
@@ -622,14 +696,14 @@ void build_grid(const HostScene& s, HostGrid& g) {
         cell_range(i, ax, ay, bx, by);
         const Aabb a = item(i);
         for (int y = ay; y <= by; ++y)
-            for (int x = ax; x <= bx; ++x) g.items[fill[(size_t)y * g.nx + x]++] = a;
+            for (int x = ax; x <= bx; ++x) g.items[g.cells[(size_t)y * g.nx + x].y++] = a;
     }
     for (uint32_t i = 0; i < n; ++i)
         if (!gridded[i]) g.global.push_back(item(i));
     g.valid = true;
 }
 
-GridDesc grid_desc(const HostGrid& g, const uint32_t* cell_start, const Aabb* items, const Aabb* global) {
+GridDesc grid_desc(const HostGrid& g, const uint2* cells, const Aabb* items, const Aabb* global) {
     GridDesc d{};
     d.x0 = g.x0;
     d.y0 = g.y0;
@@ -641,9 +715,9 @@ GridDesc grid_desc(const HostGrid& g, const uint32_t* cell_start, const Aabb* it
     d.zhi = g.zhi;
     d.nx = g.nx;
     d.ny = g.ny;
-    d.n_global = (int)g.global.size();
+    d.n_global = g.on_device ? 1 : (int)g.global.size();
     d.pad = 0;
-    d.cell_start = cell_start;
+    d.cells = cells;
     d.items = items;
     d.global = global;
     d.reserved = nullptr;

@@ -1,6 +1,7 @@
 // csp_scene.h -- host scene model: elements -> device records, acceleration structure, refit.
 #pragma once
 
+#include <cfloat>
 #include <cstdint>
 #include <functional>
 #include <string>
@@ -26,16 +27,29 @@ struct HostScene {
 // Build prims, optics, AABBs, pruning boxes and entity types.  Returns CSP_OK or an error status
 // with `err` filled.  The geometry arithmetic is the reference's (lib/element.cpp, lib/math_util.h,
 // cuda/GeometryDataST.h constructors), in the same double/float operation order.
-int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err);
+// `stats` (when not null): what plan_grid needs to know of the elements before the last.
+struct GridStats {
+    uint32_t n = 0;
+    double sum = 0.0;               // of the registered boxes' larger sides (grid_box)
+    float min = FLT_MAX, max = 0.f; // of the same
+    float x0 = FLT_MAX, y0 = FLT_MAX, x1 = -FLT_MAX, y1 = -FLT_MAX;  // union of the registered boxes
+    float z0 = FLT_MAX, z1 = -FLT_MAX;                               // and of the pruning boxes' heights
+    bool finite = true;
+    void add(const Aabb& prune);
+    void add(const GridStats& o);
+};
+int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, GridStats* stats = nullptr);
 
 // Runs body(k) for every k in [0, tasks), possibly on several threads, and returns when all are
 // done.
 using ParallelFor = std::function<void(size_t tasks, const std::function<void(size_t)>& body)>;
 
-// build_elements with the elements packed in ranges of kBuildChunk through `pf`: the same records
+// build_elements with the elements packed in ranges of half of kBuildChunk through `pf`: the same records
 // (each element's packing reads only that element), and the same error (the lowest failing element).
+// `packed(begin, end)` is called on the thread that packed the range, if given.
 constexpr uint32_t kBuildChunk = 1024;
-int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, const ParallelFor& pf);
+int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, const ParallelFor& pf,
+                   GridStats* stats = nullptr, const std::function<void(uint32_t, uint32_t)>& packed = nullptr);
 
 // The records of one element, as build_elements makes them: entity type, exact AABB, Prim, Optics
 // and (when `prune` is not null) the pruning box.  Allocates nothing.  Returns CSP_OK, or
@@ -64,7 +78,11 @@ struct HostGrid {
     bool valid = false;
     float x0 = 0, y0 = 0, x1 = 0, y1 = 0, cell = 1, inv_cell = 1, zlo = 0, zhi = 0;
     int nx = 0, ny = 0;
-    std::vector<uint32_t> cell_start;  // [nx * ny + 1]
+    // cells and items are left to the device (launch_sungrid_build) where every element but the last is
+    // registered, at most cap_items times in all; else they are here
+    bool on_device = false;
+    uint32_t cap_items = 0;
+    std::vector<uint2> cells;  // [nx * ny]
     std::vector<Aabb> items;
     std::vector<Aabb> global;
 };
@@ -75,8 +93,14 @@ struct HostGrid {
 // used).  Reads s.prune (registration, layer), s.aabbs (items) and s.types.
 void build_grid(const HostScene& s, HostGrid& g);
 
+// The grid of a scene as build_grid makes it, without its cell lists where the device can build them
+// (on_device): bounds and cell size follow from the elements' `stats`.  That is the case when the
+// boxes are alike enough that none is oversized (at most 4 cells and 8 times 1.4 times the smallest,
+// hence the median) -- any ordinary field; others take build_grid.
+void plan_grid(const HostScene& s, const GridStats& stats, HostGrid& g);
+
 // Device descriptor of a grid whose arrays live at the given device addresses.
-GridDesc grid_desc(const HostGrid& g, const uint32_t* cell_start, const Aabb* items, const Aabb* global);
+GridDesc grid_desc(const HostGrid& g, const uint2* cells, const Aabb* items, const Aabb* global);
 
 // Flux map target of a receiver element for an nx x ny grid (counts and stats pointers left null),
 // and the area of one bin in m^2 (flat: (w/nx)(h/ny); cylinder: (2 pi r/nx)(h/ny)).

@@ -39,83 +39,12 @@
 #include "csp_c_api.h"
 #include "csp_kernels.cuh"
 #include "csp_math.cuh"
+#include "csp_pool.h"
 #include "csp_scene.h"
 #include "csp_system.h"
 
 namespace csp {
 namespace {
-
-// Fixed set of host threads for the parallel part of a submission (element records in ranges).
-// run() executes body(k) for k in [0, tasks) on the pool and the calling thread and returns when all
-// are done; concurrent callers take turns.
-class HostPool {
-public:
-    void start(unsigned threads) {
-        for (unsigned t = 0; t < threads; ++t) th_.emplace_back([this] { loop(); });
-    }
-    void stop() {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            quit_ = true;
-        }
-        cv_.notify_all();
-        for (auto& t : th_) t.join();
-        th_.clear();
-    }
-    void run(size_t tasks, const std::function<void(size_t)>& body) {
-        std::lock_guard<std::mutex> turn(run_mu_);
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            body_ = &body;
-            tasks_ = tasks;
-            next_ = 0;
-            left_ = tasks;
-            ++gen_;
-        }
-        cv_.notify_all();
-        work();
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_done_.wait(lk, [&] { return left_ == 0; });
-        body_ = nullptr;
-    }
-
-private:
-    // take tasks of the current job until none is left
-    void work() {
-        for (;;) {
-            size_t k;
-            const std::function<void(size_t)>* body;
-            {
-                std::lock_guard<std::mutex> lk(mu_);
-                if (!body_ || next_ >= tasks_) return;
-                k = next_++;
-                body = body_;
-            }
-            (*body)(k);
-            std::lock_guard<std::mutex> lk(mu_);
-            if (--left_ == 0) cv_done_.notify_all();
-        }
-    }
-    void loop() {
-        uint64_t seen = 0;
-        for (;;) {
-            {
-                std::unique_lock<std::mutex> lk(mu_);
-                cv_.wait(lk, [&] { return quit_ || gen_ != seen; });
-                if (quit_) return;
-                seen = gen_;
-            }
-            work();
-        }
-    }
-    std::mutex mu_, run_mu_;
-    std::condition_variable cv_, cv_done_;
-    std::vector<std::thread> th_;
-    const std::function<void(size_t)>* body_ = nullptr;
-    size_t tasks_ = 0, next_ = 0, left_ = 0;
-    uint64_t gen_ = 0;
-    bool quit_ = false;
-};
 
 using Clock = std::chrono::steady_clock;
 
@@ -127,7 +56,7 @@ struct SScene {
     HostGrid grid;
     int group = kAccelBvh;
     Node* d_topo = nullptr;
-    uint32_t* d_cells = nullptr;
+    uint2* d_cells = nullptr;
     Aabb* d_items = nullptr;
     Aabb* d_global = nullptr;
     // the scene's own element records, for requests without poses
@@ -162,7 +91,7 @@ struct SRequest {
     int group = kAccelBvh;
     size_t off = 0, bytes = 0;  // arena block
     size_t o_prims = 0, o_optics = 0, o_aabbs = 0, o_prune = 0, o_nodes = 0, o_sun = 0, o_grid = 0, o_counts = 0,
-           o_stats = 0, o_cells = 0, o_items = 0, o_global = 0, o_sgrid = 0;
+           o_stats = 0, o_cells = 0, o_items = 0, o_global = 0, o_sgrid = 0, o_field = 0;
     bool own_records = false;
     int result_slot = -1;
     Clock::time_point t_submit, t_admit, t_done;
@@ -277,7 +206,7 @@ struct Server {
     int start(int dev, size_t budget_bytes, int max_act, uint64_t step_target);
     void stop();
     int add_scene(const csp_element* el, uint32_t n, uint32_t* id);
-    int submit(const SRequest& r, uint64_t* id);
+    int submit(SRequest&& r, uint64_t* id);
     void run_worker();
     size_t request_bytes(const SRequest& r) const;
     int admit(std::vector<SRequest*>& admitted, std::string& err);
@@ -412,7 +341,7 @@ int Server::add_scene(const csp_element* el, uint32_t n, uint32_t* id) {
     if (!rc) rc = put(s->d_prims, s->base.prims, "upload prims");
     if (!rc) rc = put(s->d_optics, s->base.optics, "upload optics");
     if (!rc) rc = put(s->d_aabbs, s->base.aabbs, "upload aabbs");
-    if (!rc && s->grid.valid) rc = put(s->d_cells, s->grid.cell_start, "upload grid cells");
+    if (!rc && s->grid.valid) rc = put(s->d_cells, s->grid.cells, "upload grid cells");
     if (!rc && s->grid.valid) rc = put(s->d_items, s->grid.items, "upload grid items");
     if (!rc && s->grid.valid) rc = put(s->d_global, s->grid.global, "upload grid globals");
     std::lock_guard<std::mutex> lk(mu);
@@ -428,7 +357,7 @@ int Server::add_scene(const csp_element* el, uint32_t n, uint32_t* id) {
 // kernels write: the sun frame, the refitted BVH nodes and the sun-ray candidate grid.
 struct BlockLayout {
     size_t grid = 0, counts = 0, stats = 0, prims = 0, optics = 0, aabbs = 0, prune = 0, cells = 0, items = 0,
-           global = 0, upload = 0, sun = 0, nodes = 0, sgrid = 0, total = 0;
+           global = 0, upload = 0, sun = 0, nodes = 0, sgrid = 0, field = 0, total = 0;
 };
 
 static BlockLayout block_layout(const SRequest& r, uint32_t nx, uint32_t ny) {
@@ -448,8 +377,8 @@ static BlockLayout block_layout(const SRequest& r, uint32_t nx, uint32_t ny) {
         take(L.optics, n * sizeof(Optics));
         take(L.aabbs, n * sizeof(Aabb));
         take(L.prune, n * sizeof(Aabb));
-        if (r.group == kAccelGrid) {
-            take(L.cells, r.grid.cell_start.size() * sizeof(uint32_t));
+        if (r.group == kAccelGrid && !r.grid.on_device) {
+            take(L.cells, r.grid.cells.size() * sizeof(uint2));
             take(L.items, r.grid.items.size() * sizeof(Aabb));
             take(L.global, std::max<size_t>(1, r.grid.global.size()) * sizeof(Aabb));
         }
@@ -458,20 +387,23 @@ static BlockLayout block_layout(const SRequest& r, uint32_t nx, uint32_t ny) {
     take(L.sun, sizeof(SunFrame));
     if (!r.poses.empty() && r.group != kAccelGrid) take(L.nodes, s.base.nodes.size() * sizeof(Node));
     if (r.group != kAccelFlat) take(L.sgrid, sungrid_bytes((uint32_t)n));
+    if (!r.poses.empty() && r.group == kAccelGrid && r.grid.on_device)
+        take(L.field, field_bytes(r.grid.nx, r.grid.ny, r.grid.cap_items));
     L.total = o;
     return L;
 }
 
 size_t Server::request_bytes(const SRequest& r) const { return block_layout(r, nx, ny).total; }
 
-int Server::submit(const SRequest& in, uint64_t* id) {
+int Server::submit(SRequest&& request, uint64_t* id) {
     const SScene* sp = nullptr;
     {
         std::lock_guard<std::mutex> lk(mu);
-        if (in.scene < scenes.size()) sp = scenes[in.scene].get();
+        if (request.scene < scenes.size()) sp = scenes[request.scene].get();
     }
     if (!sp) return set_error(CSP_ERR_INVALID_ARGUMENT, "no such scene");
-    auto r = std::make_unique<SRequest>(in);
+    auto r = std::make_unique<SRequest>(std::move(request));
+    const SRequest& in = *r;
     const SScene& s = *sp;
     if (!in.poses.empty()) {
         if (in.poses.size() != s.elements.size())
@@ -483,14 +415,16 @@ int Server::submit(const SRequest& in, uint64_t* id) {
         // ranges on the server's host threads): element records and grid of its poses
         std::string err;
         const uint32_t n = (uint32_t)r->poses.size();
-        const int rc = n >= 4 * kBuildChunk
-                           ? build_elements(r->poses.data(), n, r->hs, err,
-                                            [this](size_t tasks, const std::function<void(size_t)>& body) {
-                                                pool.run(tasks, body);
-                                            })
-                           : build_elements(r->poses.data(), n, r->hs, err);
+        GridStats stats;
+        const int rc = n >= 4096 ? build_elements(
+                                       r->poses.data(), n, r->hs, err,
+                                       [this](size_t tasks, const std::function<void(size_t)>& body) {
+                                           pool.run(tasks, body);
+                                       },
+                                       &stats)
+                                 : build_elements(r->poses.data(), n, r->hs, err, &stats);
         if (rc) return set_error(rc, err);
-        if (s.group != kAccelFlat) build_grid(r->hs, r->grid);
+        if (s.group != kAccelFlat) plan_grid(r->hs, stats, r->grid);
     }
     std::lock_guard<std::mutex> lk(mu);
     if (!fatal.empty()) return set_error(CSP_ERR_CUDA, "server stopped: " + fatal);
@@ -556,6 +490,7 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
         r.o_sun = r.off + L.sun;
         r.o_nodes = r.off + L.nodes;
         r.o_sgrid = r.off + L.sgrid;
+        r.o_field = r.off + L.field;
         r.own_records = !r.poses.empty();
         stage_off[i] = stage;
         upload[i] = L.upload;
@@ -590,7 +525,7 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
     RefitJob* refits = reinterpret_cast<RefitJob*>(h_adm + refit_at);
     SunJob* suns = reinterpret_cast<SunJob*>(h_adm + sun_at);
     SunGridJob* sgs = reinterpret_cast<SunGridJob*>(h_adm + sg_at);
-    int n_refit = 0, n_sun = 0, max_nodes = 0, n_sg = 0, max_n = 0;
+    int n_refit = 0, n_sun = 0, max_nodes = 0, n_sg = 0, max_n = 0, max_field_cells = 0;
     for (size_t i = 0; i < admitted.size(); ++i) {
         SRequest& r = *admitted[i];
         const SScene& s = *r.sc;
@@ -621,12 +556,16 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
         }
         if (r.group == kAccelGrid) {
             GridDesc g;
-            if (r.own_records) {
+            if (r.own_records && r.grid.on_device) {
+                SunGridJob gj{};
+                field_place(d_arena + r.o_field, r.grid, nullptr, gj);
+                g = grid_desc(r.grid, gj.field_cells, gj.field_items, d_aabbs + (n - 1));
+            } else if (r.own_records) {
                 const HostGrid& hg = r.grid;
-                std::memcpy(at(r.o_cells), hg.cell_start.data(), hg.cell_start.size() * sizeof(uint32_t));
+                std::memcpy(at(r.o_cells), hg.cells.data(), hg.cells.size() * sizeof(uint2));
                 if (!hg.items.empty()) std::memcpy(at(r.o_items), hg.items.data(), hg.items.size() * sizeof(Aabb));
                 if (!hg.global.empty()) std::memcpy(at(r.o_global), hg.global.data(), hg.global.size() * sizeof(Aabb));
-                g = grid_desc(hg, reinterpret_cast<const uint32_t*>(d_arena + r.o_cells),
+                g = grid_desc(hg, reinterpret_cast<const uint2*>(d_arena + r.o_cells),
                               reinterpret_cast<const Aabb*>(d_arena + r.o_items),
                               reinterpret_cast<const Aabb*>(d_arena + r.o_global));
             } else {
@@ -654,6 +593,10 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
             sungrid_place(d_arena + r.o_sgrid, n, gj);
             gj.sun = sj.out;
             gj.aabbs = d_aabbs;
+            if (r.own_records && r.group == kAccelGrid && r.grid.on_device) {
+                field_place(d_arena + r.o_field, r.grid, reinterpret_cast<const Aabb*>(d_arena + r.o_prune), gj);
+                max_field_cells = std::max(max_field_cells, r.grid.nx * r.grid.ny);
+            }
         }
         max_n = std::max(max_n, (int)n);
         r.t_admit = Clock::now();
@@ -674,7 +617,7 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
             "prepare_sun_batch_kernel");
     if (!rc && n_sg)
         rc = cuda_status(launch_sungrid_build(reinterpret_cast<const SunGridJob*>(d_jobs + (sg_at - refit_at)), n_sg,
-                                              max_n, adm_stream),
+                                              max_n, max_field_cells, adm_stream),
                          "sun grid build");
     return rc;
 }
@@ -979,7 +922,7 @@ int csp_server_submit(csp_server sh, uint32_t scene, const csp_element* poses, c
     r.rays = rays;
     r.seed = seed;
     r.instance = instance;
-    return s->submit(r, request);
+    return s->submit(std::move(r), request);
 }
 
 int csp_server_set_output(csp_server sh, int flags) {

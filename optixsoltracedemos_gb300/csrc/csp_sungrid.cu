@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "csp_kernels.cuh"
+#include "csp_scene.h"
 #include "csp_trace.cuh"
 
 namespace csp {
@@ -79,6 +80,10 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
     for (int c = tid; c < kReachRaster * kReachRaster / 128; c += kThreads)
         reinterpret_cast<uint4*>(J.reach)[c] = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) *J.alloc = 0u;
+    if (J.field_cells) {
+        for (int c = tid; c < J.field_nx * J.field_ny; c += kThreads) J.field_cells[c] = make_uint2(0u, 0u);
+        if (tid == 0) *J.field_alloc = 0u;
+    }
     __syncthreads();
     const float inf = __int_as_float(0x7f800000);
     const float tan_a = cone_tan(S);
@@ -181,8 +186,28 @@ struct ElemCells {
     __device__ int at(int k) const { return (iv0 + k / w) * nu + iu0 + k % w; }
 };
 
+// Field-grid cells of element e's registered box (every element but the last has one).  The index is
+// the walk's own expression, monotonic in the coordinate, so a point of the box lies in one of them.
+template <class F>
+__device__ __forceinline__ void field_cells_of(const SunGridJob& J, int e, F&& f) {
+    if (!J.field_cells || e + 1 >= J.n) return;
+    const Aabb p = J.prune[e];
+    const float4 b = grid_box(p.lo, p.hi);
+    auto index = [](float x, float x0, float inv, int n) {
+        return (int)fminf(fmaxf(floorf((x - x0) * inv), 0.0f), (float)(n - 1));
+    };
+    const int ax = index(b.x, J.field_x0, J.field_inv, J.field_nx), bx = index(b.z, J.field_x0, J.field_inv, J.field_nx);
+    const int ay = index(b.y, J.field_y0, J.field_inv, J.field_ny), by = index(b.w, J.field_y0, J.field_inv, J.field_ny);
+    for (int y = ay; y <= by; ++y)
+        for (int x = ax; x <= bx; ++x) f(J.field_cells + y * J.field_nx + x);
+}
+
 __global__ void __launch_bounds__(kElemBlock) sungrid_count_kernel(const SunGridJob* __restrict__ jobs) {
     const SunGridJob& J = jobs[blockIdx.y];
+    if (blockIdx.z == 1) {
+        field_cells_of(J, (int)(blockIdx.x * kElemBlock + threadIdx.x), [](uint2* c) { atomicAdd(&c->y, 1u); });
+        return;
+    }
     const int e = (int)(blockIdx.x * kElemBlock + threadIdx.x) / kElemLanes;
     const int lane = threadIdx.x & (kElemLanes - 1);
     if (e >= J.n) return;
@@ -201,13 +226,17 @@ __global__ void __launch_bounds__(kElemBlock) sungrid_count_kernel(const SunGrid
 
 __global__ void __launch_bounds__(kElemBlock) sungrid_ranges_kernel(const SunGridJob* __restrict__ jobs) {
     const SunGridJob& J = jobs[blockIdx.y];
-    const int nc = J.desc->nu * J.desc->nv;
+    const bool field = blockIdx.z == 1;
+    if (field && !J.field_cells) return;
+    uint2* const cells = field ? J.field_cells : J.cells;
+    uint32_t* const alloc = field ? J.field_alloc : J.alloc;
+    const int nc = field ? J.field_nx * J.field_ny : J.desc->nu * J.desc->nv;
     const int c = 4 * (int)(blockIdx.x * kElemBlock + threadIdx.x), lane = threadIdx.x & 31;
     if (c - 4 * lane >= nc) return;  // whole warps
     uint32_t k[4], sum = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        k[i] = c + i < nc ? J.cells[c + i].y : 0u;
+        k[i] = c + i < nc ? cells[c + i].y : 0u;
         sum += k[i];
     }
     uint32_t incl = sum;
@@ -216,17 +245,25 @@ __global__ void __launch_bounds__(kElemBlock) sungrid_ranges_kernel(const SunGri
         if (lane >= o) incl += y;
     }
     uint32_t base = 0;
-    if (lane == 31 && incl) base = atomicAdd(J.alloc, incl);
+    if (lane == 31 && incl) base = atomicAdd(alloc, incl);
     base = __shfl_sync(0xffffffffu, base, 31) + incl - sum;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        if (c + i < nc) J.cells[c + i] = make_uint2(base, base);
+        if (c + i < nc) cells[c + i] = make_uint2(base, base);
         base += k[i];
     }
 }
 
 __global__ void __launch_bounds__(kElemBlock) sungrid_fill_kernel(const SunGridJob* __restrict__ jobs) {
     const SunGridJob& J = jobs[blockIdx.y];
+    if (blockIdx.z == 1) {
+        const int e = (int)(blockIdx.x * kElemBlock + threadIdx.x);
+        field_cells_of(J, e, [&](uint2* c) {
+            const uint32_t at = atomicAdd(&c->y, 1u);
+            if (CSP_BOUNDS(6, at < J.field_cap)) J.field_items[at] = J.aabbs[e];
+        });
+        return;
+    }
     const int e = (int)(blockIdx.x * kElemBlock + threadIdx.x) / kElemLanes;
     if (e >= J.n) return;
     const float4 r = J.rect[e];
@@ -278,23 +315,52 @@ void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job) {
     job.item_rect = reinterpret_cast<float4*>(take((size_t)c.cap_items * sizeof(float4)));
     job.item_box = reinterpret_cast<Aabb*>(take((size_t)c.cap_items * sizeof(Aabb)));
     job.global_id = reinterpret_cast<uint32_t*>(take((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t)));
+    job.prune = nullptr;
+    job.field_cells = nullptr;
+    job.field_alloc = nullptr;
+    job.field_items = nullptr;
+    job.field_x0 = job.field_y0 = job.field_inv = 0.0f;
+    job.field_nx = job.field_ny = 0;
+    job.field_cap = 0;
     job.n = (int)n;
     job.cap_cells = c.cap_cells;
     job.cap_items = c.cap_items;
     job.pad = 0;
 }
 
-cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, cudaStream_t stream) {
+size_t field_bytes(int nx, int ny, uint32_t cap) {
+    return a256((size_t)nx * ny * sizeof(uint2)) + a256(sizeof(uint32_t)) + a256((size_t)cap * sizeof(Aabb));
+}
+
+void field_place(unsigned char* base, const HostGrid& g, const Aabb* prune, SunGridJob& job) {
+    job.prune = prune;
+    job.field_cells = reinterpret_cast<uint2*>(base);
+    base += a256((size_t)g.nx * g.ny * sizeof(uint2));
+    job.field_alloc = reinterpret_cast<uint32_t*>(base);
+    base += a256(sizeof(uint32_t));
+    job.field_items = reinterpret_cast<Aabb*>(base);
+    job.field_x0 = g.x0;
+    job.field_y0 = g.y0;
+    job.field_inv = g.inv_cell;
+    job.field_nx = g.nx;
+    job.field_ny = g.ny;
+    job.field_cap = g.cap_items;
+}
+
+cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, int max_field_cells,
+                                 cudaStream_t stream) {
     if (n_jobs <= 0 || max_n <= 0) return cudaSuccess;
     const unsigned elem_blocks = (unsigned)(((uint64_t)max_n * kElemLanes + kElemBlock - 1) / kElemBlock);
-    const unsigned cell_blocks = (unsigned)((sungrid_caps((uint32_t)max_n).cap_cells / 4 + kElemBlock) / kElemBlock);
+    const int max_cells = std::max(sungrid_caps((uint32_t)max_n).cap_cells, max_field_cells);
+    const unsigned cell_blocks = (unsigned)((max_cells / 4 + kElemBlock) / kElemBlock);
+    const unsigned parts = max_field_cells > 0 ? 2u : 1u;  // blockIdx.z: the sun grids, the field grids
     for (int j0 = 0; j0 < n_jobs; j0 += kMaxJobsPerLaunch) {
         const unsigned nj = (unsigned)std::min(kMaxJobsPerLaunch, n_jobs - j0);
         const SunGridJob* J = jobs + j0;
         sungrid_size_kernel<<<nj * kStateCluster, kStateBlock, 0, stream>>>(J);
-        sungrid_count_kernel<<<dim3(elem_blocks, nj), kElemBlock, 0, stream>>>(J);
-        sungrid_ranges_kernel<<<dim3(cell_blocks, nj), kElemBlock, 0, stream>>>(J);
-        sungrid_fill_kernel<<<dim3(elem_blocks, nj), kElemBlock, 0, stream>>>(J);
+        sungrid_count_kernel<<<dim3(elem_blocks, nj, parts), kElemBlock, 0, stream>>>(J);
+        sungrid_ranges_kernel<<<dim3(cell_blocks, nj, parts), kElemBlock, 0, stream>>>(J);
+        sungrid_fill_kernel<<<dim3(elem_blocks, nj, parts), kElemBlock, 0, stream>>>(J);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

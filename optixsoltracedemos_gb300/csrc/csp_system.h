@@ -10,6 +10,7 @@
 
 #include "csp_c_api.h"
 #include "csp_kernels.cuh"
+#include "csp_pool.h"
 #include "csp_scene.h"
 
 namespace csp {
@@ -56,20 +57,33 @@ struct System {
     HostGrid grid;
     int accel = CSP_ACCEL_AUTO;
 
+    HostPool pool;                  // element records of scenes of kPoolElements or more, in ranges
+    bool topology = false;          // scene.nodes are the BVH (or leaf list) of this element count
     Node* d_nodes = nullptr;
+    // element records: prims, optics, exact and pruning boxes in one device block, put together in
+    // pinned memory and uploaded in one copy
+    unsigned char* d_records = nullptr;
+    unsigned char* h_records = nullptr;
+    size_t cap_records = 0;
+    bool records_busy = false;  // an upload from h_records that no synchronisation has followed yet
     Prim* d_prims = nullptr;
     Optics* d_optics = nullptr;
     Aabb* d_aabbs = nullptr;
+    Aabb* d_prune = nullptr;
     SunFrame* d_sun = nullptr;
     float4* d_hits = nullptr;
     uint32_t* d_ids = nullptr;
     GridDesc* d_grid = nullptr;
     const float* h3t12 = nullptr;  // Halton table of the device (halton3_table)
     GridDesc grid_host{};  // host copy of the descriptor (source of the async upload)
-    uint32_t* d_cells = nullptr;
+    // cells, items and global list of a field grid built on the host, or the block of one that the
+    // device builds
+    uint2* d_cells = nullptr;
     Aabb* d_items = nullptr;
     Aabb* d_global = nullptr;
     size_t cap_cells = 0, cap_items = 0, cap_global = 0;
+    unsigned char* d_field = nullptr;
+    size_t cap_field = 0;
     // sun-ray candidate grid (scenes of more than kFlatListMax elements): its arrays, and the build
     // job (host copy = source of the async upload)
     unsigned char* d_sgrid = nullptr;
@@ -88,10 +102,10 @@ struct System {
     float4* d_cring = nullptr;
     uint64_t cap_cring = 0;
     unsigned long long* h_ctotal = nullptr;
-    uint32_t* d_flux = nullptr;              // csp_flux_map counts
-    unsigned long long* d_fstats = nullptr;  // [4]
+    unsigned char* d_flux = nullptr;  // csp_flux_map: counters [4], then the map
+    unsigned char* h_flux = nullptr;  // pinned: the sun frame, then the map
     size_t cap_flux = 0;
-    size_t cap_nodes = 0, cap_prims = 0, cap_optics = 0, cap_aabbs = 0;
+    size_t cap_nodes = 0;
     uint64_t cap_rays = 0;
     bool ids_allocated = false;
 
@@ -105,8 +119,9 @@ struct System {
     ~System();
     void release();
     int ensure_streams();
-    int upload_scene();
-    int upload_grid(bool arrays);
+    int build_scene(const char* not_planar);
+    int upload_nodes();
+    int upload_grid();
     int prepare_sun();
     int build_sungrid();
     float pad_angle() const;

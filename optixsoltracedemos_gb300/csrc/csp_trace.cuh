@@ -579,7 +579,7 @@ __device__ __forceinline__ int traverse_grid(const GridDesc& G, const Prim* __re
     uint32_t j = 0, e = (uint32_t)G.n_global;
     bool next = walk;
     float ctc = ta;
-    if (next) prefetch_l1(G.cell_start + (iy * G.nx + ix));
+    if (next) prefetch_l1(G.cells + (iy * G.nx + ix));
     int step = 0;
     for (;;) {
         for (; j < e; ++j) {
@@ -592,8 +592,9 @@ __device__ __forceinline__ int traverse_grid(const GridDesc& G, const Prim* __re
         const int c = iy * G.nx + ix;
         if (!CSP_BOUNDS(4, c >= 0 && c < G.nx * G.ny)) break;
         list = G.items;
-        j = __ldg(G.cell_start + c);
-        e = __ldg(G.cell_start + c + 1);
+        const uint2 range = __ldg(G.cells + c);
+        j = range.x;
+        e = range.y;
         ++step;
         // the cell after it: parameters of the next x and y cell boundaries, from the cell index
         const float tnx = (d.x != 0.0f) ? (G.x0 + (float)(ix + (sx > 0)) * G.cell - o.x) * inv.x : inf;
@@ -607,7 +608,7 @@ __device__ __forceinline__ int traverse_grid(const GridDesc& G, const Prim* __re
             iy += sy;
             next = iy >= 0 && iy < G.ny;
         }
-        if (next) prefetch_l1(G.cell_start + (iy * G.nx + ix));
+        if (next) prefetch_l1(G.cells + (iy * G.nx + ix));
     }
     return best;
 }

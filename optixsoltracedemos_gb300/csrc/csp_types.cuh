@@ -78,7 +78,7 @@ struct alignas(16) SunFrame {
 
 // Uniform 2D grid over a planar heliostat field (the alternative to the BVH for field-like
 // scenes), built for one set of poses.  Cells of size `cell` cover [x0, x1] x [y0, y1]; the items of
-// cell (ix, iy) are items[cell_start[iy * nx + ix] .. cell_start[iy * nx + ix + 1]), one per element
+// cell (ix, iy) are items [x, y) of cells[iy * nx + ix], one per element
 // whose pruning box (widened by a margin) overlaps the cell in xy: the element's exact AABB with
 // lo.w = element | type << 28 (bits).  Rays walk the cells their xy path crosses inside the layer
 // [zlo, zhi], which holds every gridded surface; the global items (the receiver, oversized
@@ -88,7 +88,7 @@ struct alignas(16) GridDesc {
     float x0, y0, x1, y1;
     float cell, inv_cell, zlo, zhi;
     int nx, ny, n_global, pad;
-    const uint32_t* cell_start;
+    const uint2* cells;
     const Aabb* items;
     const Aabb* global;
     const void* reserved;

@@ -55,6 +55,13 @@ def _walls():
     return scenes.Scene("walls", e, np.array([0.8, 0.1, 1.0]), scenes.SUN_PILLBOX, 4.65e-3, 1)
 
 
+def _mixed_sizes(ratio):
+    """Mirrors of two sizes: the device builds the field grid up to boxes 11.2 times the smallest."""
+    sc = _field(150, 35.0)
+    sc.elements["width"][:150:3] = sc.elements["height"][:150:3] = 10.0 / ratio
+    return sc
+
+
 CASES = {
     "nine_elements": lambda: _field(8, 35.0),
     # the sun frame is one block below 1,024 elements, a cluster from there
@@ -67,6 +74,10 @@ CASES = {
     "slope": lambda: _field(200, 40.0, slope=0.6),
     # coordinates far from the origin: the margins against rounding
     "offset_20_km": lambda: _field(200, 25.0, offset=2e4),
+    # the field grid: device-built, and on the host past the limits of sizes and of coordinates
+    "mixed_sizes_4": lambda: _mixed_sizes(4.0),
+    "mixed_sizes_40": lambda: _mixed_sizes(40.0),
+    "offset_90_km": lambda: _field(200, 60.0, offset=9e4),
     # incidences around the limit of the own-mirror rule and beyond it, mirrors facing each other
     "incidence_65_deg": lambda: _facing(12, 25.0, [0.0, 0.0, 1.0], 9.0),
     "incidence_85_deg": lambda: _facing(12, 5.0, [0.0, 0.0, 1.0], 9.0, specularity=5e-2),
@@ -87,3 +98,36 @@ def test_search_edges_bit_exact(gpu, oracle32, name, accel):
     np.testing.assert_array_equal(ids, oi)
     np.testing.assert_array_equal(hits, oh.astype(np.float32))
     assert (oh[:, 1:, 0] != 0).any()
+
+
+def test_update_between_grid_and_bvh(gpu, oracle32):
+    """update() of a planar field to steep ground and back: the BVH is built when it is first needed."""
+    flat, steep = _field(300, 40.0), _field(300, 40.0, slope=0.6)
+    n = 20000
+    t = native.tracer_for(flat, seed=5, num_rays=n)
+    for sc, accel in ((flat, native.ACCEL_GRID), (steep, native.ACCEL_BVH), (flat, native.ACCEL_GRID),
+                      (steep, native.ACCEL_BVH)):
+        t.set_elements(sc.elements)
+        t.update()
+        assert t.accel() == accel
+        t.run()
+        hits, ids = t.copy_hits()
+        oh, oi = oracle32.trace(sc.elements, sc.sun_dir, sc.sun_shape, sc.sun_param, count=n, seed=5)
+        np.testing.assert_array_equal(ids, oi)
+        np.testing.assert_array_equal(hits, oh.astype(np.float32))
+    # an update that is refused leaves the scene as it was
+    t.set_accel(native.ACCEL_GRID)
+    t.set_elements(flat.elements)
+    t.initialize()
+    bad = flat.elements.copy()
+    bad["width"][7] = -1.0
+    for refused in (bad, steep.elements):
+        t.set_elements(refused)
+        with pytest.raises(native.CspError):
+            t.update()
+    t.run()
+    hits, ids = t.copy_hits()
+    oh, oi = oracle32.trace(flat.elements, flat.sun_dir, flat.sun_shape, flat.sun_param, count=n, seed=5)
+    np.testing.assert_array_equal(ids, oi)
+    np.testing.assert_array_equal(hits, oh.astype(np.float32))
+    t.close()
