@@ -35,13 +35,13 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kCluster)
     sun_frame_state<kCluster>(aabbs, n, s, tan_pad, shape, param, out, sm);
 }
 
-template <int kAccel>
-using PlainCfg = Cfg<kTraceBlock, kAccel, true, false>;
+template <int kAccel, bool kIds>
+using PlainCfg = Cfg<kTraceBlock, kAccel, true, false, kIds>;
 
 template <int kAccel>
 struct TraceSmem {
-    typename PlainCfg<kAccel>::Stage stage;
-    typename PlainCfg<kAccel>::Core core;
+    typename PlainCfg<kAccel, false>::Stage stage;
+    typename PlainCfg<kAccel, false>::Core core;
 };
 
 // Resident CTAs per SM the register budget is cut for: eight of 128 threads (64 registers, 1,024
@@ -67,10 +67,10 @@ constexpr int trace_min_blocks() {
 // ends in a long tail).
 constexpr uint32_t kTraceGrab = 8;
 
-template <int kAccel>
+template <int kAccel, bool kIds>
 __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace_kernel(
-    const typename PlainCfg<kAccel>::Args A) {
-    using C = PlainCfg<kAccel>;
+    const typename PlainCfg<kAccel, kIds>::Args A) {
+    using C = PlainCfg<kAccel, kIds>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TraceSmem<kAccel>& sm = *reinterpret_cast<TraceSmem<kAccel>*>(smem_raw);
     load_instance_smem<C>(A, sm.core);
@@ -139,36 +139,60 @@ __global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace
     }
 }
 
+// Resident CTA slots of the device for a trace kernel; the first call on a device prepares the kernel.
+template <int kAccel, bool kIds>
+cudaError_t find_slots(int dev, int& slots) {
+    int sms = 0, per_sm = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(trace_kernel<kAccel, kIds>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(TraceSmem<kAccel>));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kAccel, kIds>, kTraceBlock,
+                                                          sizeof(TraceSmem<kAccel>));
+    slots = std::max(1, sms * std::max(1, per_sm));
+    return e;
+}
+
+template <int kAccel, bool kIds>
+cudaError_t launch_trace_ids(const TraceArgs& args, unsigned grid, cudaStream_t stream) {
+    typename PlainCfg<kAccel, kIds>::Args a;
+    static_cast<TraceArgs&>(a) = args;
+    if constexpr (PlainCfg<kAccel, kIds>::kSched) philox_keys(args.seed, a.keys);
+    using Smem = TraceSmem<kAccel>;
+    // field launches leave the unused Halton table to L1 (64M rays over 10,000 heliostats 4680 -> 4660 us);
+    // element lists gain nothing from it (200,000 rays of the single parabolic heliostat 7.20, 7.64 without)
+    const size_t smem = sizeof(Smem) - (kAccel != kAccelFlat && args.h3t12 ? sizeof(Smem::core.t6) : 0);
+    trace_kernel<kAccel, kIds><<<grid, kTraceBlock, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+// Launches with and without element ids are kernels of their own: in one kernel the ids' stores cost the
+// launches without them registers (64M rays over 10,000 heliostats 4807 us, against 4653 apart).
 template <int kAccel>
 cudaError_t launch_trace_t(const TraceArgs& args, cudaStream_t stream) {
-    // persistent grid: every resident CTA slot of the device (found once per device; devices past 63
-    // each time), never more CTAs than tiles
-    static std::atomic<int> slots_of[64];
+    // persistent grid: every resident CTA slot of the device (found once per device, for both kernels, so
+    // that the first launch of either prepares the other too; devices past 63 each time), never more
+    // CTAs than tiles
+    static std::atomic<uint64_t> slots_of[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    int slots = dev < 64 ? slots_of[dev].load(std::memory_order_acquire) : 0;
-    if (slots == 0) {
-        int sms = 0, per_sm = 0;
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(trace_kernel<kAccel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(TraceSmem<kAccel>));
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<kAccel>, kTraceBlock,
-                                                              sizeof(TraceSmem<kAccel>));
+    uint64_t both = dev < 64 ? slots_of[dev].load(std::memory_order_acquire) : 0;
+    if (both == 0) {
+        int plain = 0, ids = 0;
+        e = find_slots<kAccel, false>(dev, plain);
+        if (e == cudaSuccess) e = find_slots<kAccel, true>(dev, ids);
         if (e != cudaSuccess) return e;
-        slots = std::max(1, sms * std::max(1, per_sm));
-        if (dev < 64) slots_of[dev].store(slots, std::memory_order_release);
+        both = (uint64_t)ids << 32 | (uint32_t)plain;
+        if (dev < 64) slots_of[dev].store(both, std::memory_order_release);
     }
+    const uint64_t slots = args.ids ? both >> 32 : (uint32_t)both;
     const uint64_t tiles = (args.count + kTraceBlock - 1) / kTraceBlock;  // CTAs that have work
     if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // 44 TB of records
-    const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)slots);
-    typename PlainCfg<kAccel>::Args a;
-    static_cast<TraceArgs&>(a) = args;
-    if constexpr (PlainCfg<kAccel>::kSched) philox_keys(args.seed, a.keys);
-    trace_kernel<kAccel><<<(unsigned)grid, kTraceBlock, sizeof(TraceSmem<kAccel>), stream>>>(a);
-    return cudaGetLastError();
+    const unsigned grid = (unsigned)std::min(tiles, slots);
+    return args.ids ? launch_trace_ids<kAccel, true>(args, grid, stream)
+                    : launch_trace_ids<kAccel, false>(args, grid, stream);
 }
 
 // Pass over n_records float4 records {stage, x, y, z}: stage-1 records are counted, stage-2 records

@@ -77,14 +77,18 @@ template <int kB, bool kFlat>
 struct CoreSmem;
 template <int kB>
 struct FlatStageSmem;
+template <int kB>
+struct RowStageSmem;
+struct NoStage {};
 
-template <int kB_, int kAccel_, bool kDense_, bool kFlux_>
+template <int kB_, int kAccel_, bool kDense_, bool kFlux_, bool kIds_ = false>
 struct Cfg {
     static constexpr int kB = kB_;        // CTA size = tile size (rays)
     static constexpr int kAccel = kAccel_;
     static constexpr bool kFlat = kAccel_ == kAccelFlat;
     static constexpr bool kDense = kDense_;
     static constexpr bool kFlux = kFlux_;
+    static constexpr bool kIds = kIds_;   // dense launches: element ids out as well
     // grid and BVH launches give each warp 32 rays whose sun-plane points are close together
     static constexpr bool kCoherent = kAccel_ != kAccelFlat;
     // Philox from the precomputed key schedule: the single-scene element-list kernel only (the field
@@ -97,60 +101,52 @@ struct Cfg {
     // launches trace the first segment in place (first_segment)
     using Core = CoreSmem<kB_, kFlat>;
     // phase A record staging of dense element-list launches
-    struct NoStage {};
-    using Stage = std::conditional_t<kFlat && kDense_, FlatStageSmem<kB_>, NoStage>;
+    using Stage = std::conditional_t<!kDense_, NoStage, std::conditional_t<kFlat, FlatStageSmem<kB_>, RowStageSmem<kB_>>>;
 };
 
 // Coherent ray order: position kk of a launch of `count` rays -> ray offset.  Rays come in blocks
 // of 32 S; in a block, the warp at position m takes offsets m + j S (lane j).  The Halton
 // coordinates of offsets that differ by a multiple of S = 2^a 3^b differ by less than 2^-a in u
 // (base 2) and 3^-b in v (base 3), so a warp's rays start within a small patch of the sun plane and
-// walk the same grid cells.  Whole blocks of S = 2^8 3^5 first, then of S = 2^7 3^4 over the rest,
-// then the identity order for the tail: a bijection on [0, count).  kFine puts whole blocks of
-// S = 2^9 3^6 (11,943,936 rays) before them: launches without dense records gain from the smaller
-// patches, while in dense launches a warp's 32 rows would then span ~1 GB of the hit buffer, which
-// measured slower.  With G > 1 groups of G consecutive warps (of one tile, i.e. CTA) take
-// neighbouring patches: warp k of group t in a block gets m = k S / G + t, and offsets that differ
-// by S / G = 2^(a-log2 G) 3^b have u coordinates 2^-a apart -- a strip of G adjacent patches whose
-// grid cells the group's warps share in L1.
-constexpr uint64_t kCoherentS0 = 512u * 729u, kCoherentB0 = 32u * kCoherentS0;
-constexpr uint64_t kCoherentS1 = 256u * 243u, kCoherentB1 = 32u * kCoherentS1;
-constexpr uint64_t kCoherentS2 = 128u * 81u, kCoherentB2 = 32u * kCoherentS2;
+// walk the same grid cells.  A launch is cut into whole blocks of S1 = 2^8 3^5 first, then over what is
+// left of S2 = 2^7 3^4 and of S3 = 2^6 3^3 (55,296 rays), then the identity order for the tail: a
+// bijection on [0, count).  Without S3 up to 331,775 rays went in identity order (1.2M rays of a
+// hillside of 600: 91.5 us, 87.3 with it).  Launches without dense records (kFine) take blocks of
+// S0 = 2^9 3^6 (11,943,936 rays) before S1 and none of S3: they gain from the smaller patches, while in
+// dense launches a warp's 32 rows would span ~1 GB of the hit buffer (64M rays of 10,000 heliostats:
+// 5349 us against 4861).
+// With G > 1 groups of G consecutive warps (of one tile, i.e. CTA) take neighbouring patches: warp k of
+// group t in a block gets m = k S / G + t, and offsets that differ by S / G = 2^(a-log2 G) 3^b have u
+// coordinates 2^-a apart -- a strip of G adjacent patches whose grid cells the group's warps share in L1.
+// With G = 1 the warps of a tile have consecutive rows: what shares a sector is written together.
+constexpr uint32_t kCoherentS0 = 512u * 729u, kCoherentS1 = 256u * 243u, kCoherentS2 = 128u * 81u, kCoherentS3 = 64u * 27u;
 
-// warp position m in a block of S warps for the warp at index r >> 5 of the block (G | S)
-template <int G, class U>
-__device__ __forceinline__ U coherent_warp(U r, U S) {
-    const U w = r >> 5;
-    if constexpr (G == 1) return w;
-    else return (w % G) * (S / G) + w / G;
+// The whole blocks of S over the `count` rays left: true with kk the offset of position kk in them, else
+// kk, count and `first` moved past them.
+template <uint32_t S, int G, class U>
+__device__ __forceinline__ bool coherent_level(U& kk, U& count, U& first) {
+    static_assert(S % G == 0, "warp groups must divide every S");
+    constexpr U B = (U)32u * S;
+    const U full = count / B * B;
+    if (kk < full) {
+        const U blk = kk / B, r = kk - blk * B, w = r >> 5;
+        kk = blk * B + (w % G) * (U)(S / G) + w / G + (r & 31u) * S;
+        return true;
+    }
+    kk -= full;
+    count -= full;
+    first += full;
+    return false;
 }
 
 template <bool kFine, int G, class U>
 __device__ __forceinline__ U coherent_order_t(U kk, U count) {
-    static_assert(G == 1 || G == 2 || G == 4 || G == 8 || G == 16, "warp groups must divide every S");
-    constexpr U B0 = (U)kCoherentB0, S0 = (U)kCoherentS0, B1 = (U)kCoherentB1, S1 = (U)kCoherentS1;
-    constexpr U B2 = (U)kCoherentB2, S2 = (U)kCoherentS2;
-    U full0 = 0;
-    if constexpr (kFine) {
-        full0 = (count / B0) * B0;
-        if (kk < full0) {
-            const U blk = kk / B0, r = kk - blk * B0;
-            return blk * B0 + (U)coherent_warp<G>(r, S0) + (r & 31u) * S0;
-        }
-    }
-    const U k1 = kk - full0, c1 = count - full0;
-    const U full1 = (c1 / B1) * B1;
-    if (k1 < full1) {
-        const U blk = k1 / B1, r = k1 - blk * B1;
-        return full0 + blk * B1 + (U)coherent_warp<G>(r, S1) + (r & 31u) * S1;
-    }
-    const U k2 = k1 - full1;
-    const U full2 = ((c1 - full1) / B2) * B2;
-    if (k2 < full2) {
-        const U blk = k2 / B2, r = k2 - blk * B2;
-        return full0 + full1 + blk * B2 + (U)coherent_warp<G>(r, S2) + (r & 31u) * S2;
-    }
-    return kk;
+    U first = 0;
+    if (kFine && coherent_level<kCoherentS0, G>(kk, count, first)) return first + kk;
+    if (coherent_level<kCoherentS1, G>(kk, count, first)) return first + kk;
+    if (coherent_level<kCoherentS2, G>(kk, count, first)) return first + kk;
+    if (!kFine) coherent_level<kCoherentS3, G>(kk, count, first);
+    return first + kk;
 }
 
 // Launches of fewer than 2^32 rays (all but the largest) take the 32-bit form: the same
@@ -222,19 +218,13 @@ struct StateSmem {
 
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-// 32-byte accesses (p 32-byte aligned).  Lanes on different records of a scene, or on different
-// rows of the hit buffer, touch a cache line per access and lane: half as many accesses is half the
-// time in the L1 pipe, which was 56 % busy in the field kernel with 16-byte ones (64M rays over 10,000
-// heliostats 5855 -> 5461 us, 3M rays over 1,000 focused ones with ids 256 -> 230 us).
+// 32-byte load (p 32-byte aligned).  Lanes on different records of a scene touch a cache line per access
+// and lane: half as many accesses is half the time in the L1 pipe, which was 56 % busy in the field kernel
+// with 16-byte ones (64M rays over 10,000 heliostats 5855 -> 5461 us, the stores of that time included).
 __device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
         : "l"(p));
-}
-__device__ __forceinline__ void stg32(void* p, float4 a, float4 b) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
-                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-                 : "memory");
 }
 
 // ------------------------------------------------------------------------------ sampling ------
@@ -1075,8 +1065,7 @@ struct CoreSmem {
     uint64_t qray[kQ];
     float go[2][kFlat ? 2 * kB : 1];
     uint64_t gray[kFlat ? 2 * kB : 1];
-    float t6[kH3Tab];
-    FlatScene flat;
+    std::conditional_t<kFlat, FlatScene, char> flat;
     SunFrame sun;
     std::conditional_t<kFlat, char, GridDesc> grid;
     std::conditional_t<kFlat, char, SunGrid> sg;
@@ -1084,6 +1073,7 @@ struct CoreSmem {
     // sizes in registers, updated at the barriers that close each append
     int qsize;
     int gsize;
+    float t6[kH3Tab];  // the last member: field launches with the device-wide 3^12 table leave it out
 };
 
 // Closest hit of a segment in a BVH or grid launch.
@@ -1102,6 +1092,12 @@ __device__ __forceinline__ int find_closest(const typename C::Args& A, const typ
 template <int kB>
 struct FlatStageSmem {
     float4 row[kB * kMaxDepth];
+};
+
+// Dense BVH and grid launches: slots 0 and 1 of a tile's rays, on their way to the lanes that store them.
+template <int kB>
+struct RowStageSmem {
+    float4 rec[2][kB];
 };
 
 // Where kFlux records go: the instance's flux target and the CTA's record counters.
@@ -1132,17 +1128,18 @@ __device__ __noinline__ void flux_record(const Sink& k, float4 rec, int slot) {
     }
 }
 
-__device__ __forceinline__ void store_record(const TraceArgs& A, uint64_t ray, int slot, float4 rec, uint32_t id) {
+template <class C>
+__device__ __forceinline__ void store_record(const typename C::Args& A, uint64_t ray, int slot, float4 rec, uint32_t id) {
     const uint64_t row = (ray - A.ray_begin) * kMaxDepth + (uint64_t)slot;
     if (!CSP_BOUNDS(2, ray >= A.ray_begin && row < A.count * kMaxDepth)) return;
     A.hits[row] = rec;
-    if (A.ids) A.ids[row] = id;
+    if constexpr (C::kIds) A.ids[row] = id;
 }
 
 template <class C>
 __device__ __forceinline__ void emit(const typename C::Args& A, const Sink& k, uint64_t ray, int slot, float4 rec,
                                      uint32_t id) {
-    if constexpr (C::kDense) store_record(A, ray, slot, rec, id);
+    if constexpr (C::kDense) store_record<C>(A, ray, slot, rec, id);
     if constexpr (C::kFlux) flux_record(k, rec, slot);
 }
 
@@ -1360,8 +1357,9 @@ __device__ __forceinline__ void load_instance_smem(const typename C::Args& A, ty
 // stored a second time) 64M rays over 10,000 heliostats went from 6249 to 5855 us, 1.2M rays over a
 // hillside of 600 from 118 to 107 us.
 template <class C>
-__device__ __forceinline__ void first_segment(const typename C::Args& A, const Sink& k, typename C::Core& sm, bool have,
-                                              uint64_t pos, uint64_t ray, int& qs) {
+__device__ __forceinline__ void first_segment(const typename C::Args& A, const Sink& k, typename C::Core& sm,
+                                              typename C::Stage* stage, bool have, uint64_t pos, uint64_t ray,
+                                              int& qs) {
     Segment g{f3(0.f, 0.f, 0.f), f3(0.f, 0.f, 1.f), kTminSun, 0};
     Hit h{-1, 0.f, 0u};
     bool again = false;
@@ -1384,27 +1382,37 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
     }
     push(sm, again, ray, g.o, g.d, h.t, (uint32_t)h.best | (h.type << kTypeShift));
     if constexpr (C::kDense) {
-        // each lane writes its own ray's 80 B row: the sun-plane record, the first hit's, empty slots
-        // (the bounce batches overwrite the slots they fill, after the barriers between)
-        if (have && CSP_BOUNDS(2, pos < A.count)) {
-            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), rec0 = make_float4(0.0f, g.o.x, g.o.y, g.o.z);
-            if (slot < 0) rec = zero;
-            float4* gh = A.hits + pos * kMaxDepth;
-            // rows lie 80 B apart: every other one starts on a 32-byte boundary, the same for all
-            // lanes of a coherent warp (their rows are even counts of rows apart)
-            if ((reinterpret_cast<uintptr_t>(gh) & 31u) == 0) {
-                stg32(gh, rec0, rec);
-                stg32(gh + 2, zero, zero);
-                gh[4] = zero;
-            } else {
-                gh[0] = rec0;
-                stg32(gh + 1, rec, zero);
-                stg32(gh + 3, zero, zero);
-            }
-            if (A.ids) {
-                uint32_t* gi = A.ids + pos * kMaxDepth;
+        // The warp writes its rays' rows, `step` apart, six at a time: five lanes to a row, its sun-plane record,
+        // the first hit's, empty slots (the bounce batches overwrite the slots they fill, after the barriers
+        // between).  A store then covers six rows in some nine lines; with a lane per row (32-byte stores) it
+        // met 32, and the launch was bound by its store requests to L2 wherever few rays meet a mirror: 64M rays
+        // of a hillside of 600 2481 -> 2164 us, with ids 4094 -> 3053 (the same pattern, and G = 1).
+        const int lane = threadIdx.x & 31, part = lane % kMaxDepth, row = lane < 30 ? lane / kMaxDepth : 32;
+        const uint64_t first = __shfl_sync(0xffffffffu, pos, 0);
+        const uint32_t step = __shfl_sync(0xffffffffu, (uint32_t)pos, 1) - (uint32_t)first;
+        // rows of the warp: 32, or fewer where the launch ends in a warp in identity order
+        const int n = (int)min((uint64_t)32, first < A.count ? step == 1u ? A.count - first : 32u : 0u);
+        if (slot < 0) rec = make_float4(0.f, 0.f, 0.f, 0.f);
+        stage->rec[0][threadIdx.x] = make_float4(0.0f, g.o.x, g.o.y, g.o.z);
+        stage->rec[1][threadIdx.x] = rec;
+        __syncwarp();
+        const float4* src = &stage->rec[part & 1][(threadIdx.x & ~31u) + row];
+        float4* dst = A.hits + (first + (uint64_t)row * step) * kMaxDepth + part;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int s = 0; s < kMaxDepth; ++s) gi[s] = s == 1 && slot == 1 ? (uint32_t)h.best : kNoElement;
+        for (int q = 0; q < 6; ++q) {
+            if (q * 6 + row < n) {
+                if (part < 2) v = src[q * 6];
+                dst[(uint64_t)(q * 6 * kMaxDepth) * step] = v;
+            }
+        }
+        if constexpr (C::kIds) {
+            const uint32_t id = slot == 1 ? (uint32_t)h.best : kNoElement;
+            uint32_t* out = A.ids + (first + (uint64_t)row * step) * kMaxDepth + part;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const uint32_t e = __shfl_sync(0xffffffffu, id, (q * 6 + row) & 31);
+                if (q * 6 + row < n) out[(uint64_t)(q * 6 * kMaxDepth) * step] = part == 1 ? e : kNoElement;
             }
         }
     }
@@ -1412,23 +1420,12 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
     qs += __syncthreads_count(again);
 }
 
-// Phase A of one tile (rays A.ray_begin + tile * kB ...); phase_b runs its full batches.
-// `stage` is the kDense staging area of element-list launches (unused otherwise); qs: the queue size
-// (see phase_b).
+// Phase A of one tile of an element-list launch.
 template <class C>
-__device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink& k, typename C::Core& sm,
-                                           typename C::Stage* stage, uint64_t tile, int& qs) {
+__device__ __forceinline__ void flat_points(const typename C::Args& A, typename C::Core& sm, typename C::Stage* stage,
+                                            uint64_t tile, int& qs) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t kk = tile * C::kB + threadIdx.x;
-    uint64_t pos = kk;
-    // dense launches group warps in pairs: larger groups scatter their record rows more than the
-    // shared cells save
-    if constexpr (C::kCoherent) pos = coherent_order<!C::kDense, C::kDense ? 2 : C::kB / 32>(kk, A.count);
-    const uint64_t ray = A.ray_begin + pos;
-    if constexpr (!C::kFlat) {
-        first_segment<C>(A, k, sm, kk < A.count, pos, ray, qs);
-        return;
-    }
+    const uint64_t kk = tile * C::kB + threadIdx.x, ray = A.ray_begin + kk;
     // sun-plane point; the direction waits in the generation queue unless the point lies outside
     // every reach rectangle (then the ray meets no element box and its record is the point alone)
     bool want = false;
@@ -1451,7 +1448,7 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
     }
     __syncwarp();
     push_gen(sm, want, ray, hu, hv);
-    if constexpr (C::kDense && C::kFlat) {
+    if constexpr (C::kDense) {
         const uint64_t warp_first = tile * C::kB + (uint64_t)warp * 32;
         float4* rows = stage->row + warp * 32 * kMaxDepth;
         rows[lane * kMaxDepth] = make_float4(0.0f, o.x, o.y, o.z);
@@ -1464,7 +1461,7 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
                 const uint32_t e = (uint32_t)(q * 32 + lane);
                 if (e < n_rec) gh[e] = rows[e];
             }
-            if (A.ids) {
+            if constexpr (C::kIds) {
                 uint32_t* gi = A.ids + warp_first * kMaxDepth;
 #pragma unroll
                 for (int q = 0; q < kMaxDepth; ++q) {
@@ -1477,6 +1474,22 @@ __device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink
     }
     // the barrier before phase B counts this tile's appends to the generation queue
     qs += __syncthreads_count(want);
+}
+
+// Phase A of one tile (rays A.ray_begin + tile * kB ...); phase_b runs its full batches.
+// `stage` is the staging area of kDense launches (unused otherwise); qs: the queue size (see phase_b).
+template <class C>
+__device__ __forceinline__ void trace_tile(const typename C::Args& A, const Sink& k, typename C::Core& sm,
+                                           typename C::Stage* stage, uint64_t tile, int& qs) {
+    const uint64_t kk = tile * C::kB + threadIdx.x;
+    uint64_t pos = kk;
+    // Warps of a group: those of the tile, but one with ids, whose 20-byte rows share their sectors.
+    // 64M rays in groups of 2 / 4 / 8: without ids 4827 / 4611 / 4771 us over 10,000 heliostats, 2255 / 2167 /
+    // 2446 over a hillside of 600; in groups of 1 / 2 / 4 with ids 5222 / 5170 / 5224 and 3053 / 3311 / 3932.
+    if constexpr (C::kCoherent) pos = coherent_order<!C::kDense, C::kIds ? 1 : C::kB / 32>(kk, A.count);
+    const uint64_t ray = A.ray_begin + pos;
+    if constexpr (C::kFlat) flat_points<C>(A, sm, stage, tile, qs);
+    else first_segment<C>(A, k, sm, stage, kk < A.count, pos, ray, qs);
 }
 
 }  // namespace
