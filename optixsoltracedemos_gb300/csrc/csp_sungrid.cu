@@ -19,6 +19,7 @@
 //   ranges  one thread per four cells: a warp takes the sum of its cells' counts from the state's
 //           item counter
 //   fill    kElemLanes threads per element: rectangles and exact boxes into their cells
+// The last three also build the field grid (GridDesc) of each state that has one, as blockIdx.z = 1.
 // Each is a chain of memory latencies, so the wide ones take the whole device rather than one block
 // or cluster per state: 16 + 7 + 4.5 + 6 us for 10,001 elements, against 98 us with the count per
 // element and the scan in one block, and 96 us with all phases in one cluster.

@@ -1401,7 +1401,7 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-            if (q * 6 + row < n) {
+            if (q * 6 + row < n && CSP_BOUNDS(2, first + (uint64_t)(q * 6 + row) * step < A.count)) {
                 if (part < 2) v = src[q * 6];
                 dst[(uint64_t)(q * 6 * kMaxDepth) * step] = v;
             }
@@ -1412,7 +1412,8 @@ __device__ __forceinline__ void first_segment(const typename C::Args& A, const S
 #pragma unroll
             for (int q = 0; q < 6; ++q) {
                 const uint32_t e = __shfl_sync(0xffffffffu, id, (q * 6 + row) & 31);
-                if (q * 6 + row < n) out[(uint64_t)(q * 6 * kMaxDepth) * step] = part == 1 ? e : kNoElement;
+                if (q * 6 + row < n && CSP_BOUNDS(2, first + (uint64_t)(q * 6 + row) * step < A.count))
+                    out[(uint64_t)(q * 6 * kMaxDepth) * step] = part == 1 ? e : kNoElement;
             }
         }
     }
