@@ -56,24 +56,24 @@ sys.path.insert(0, ROOT)
 METRIC = "rays/s on 1 GB300 (batched/served vs plain trace) at flux L2<=1%; p50/p99 latency"
 BYTES_PER_RAY = 80  # 5 float4 hit records per ray, fully rewritten by every plain trace
 # dram__bytes_read.sum + dram__bytes_write.sum of the single parabolic workload's trace_kernel per
-# launch of 16,777,216 rays: 4 x (8,776,704 + 291,551,232) bytes, scaled by the rays from
-# `ncu --set full -k regex:^trace_kernel -s 2 -c 1` of `python bench.py --workload single_parabolic
+# launch of 16,777,216 rays: 4 x (7,841,024 + 290,515,456) bytes, scaled by the rays from
+# `ncu -k regex:^trace_kernel -s 2 -c 1` of `python bench.py --workload single_parabolic
 # --rays 4194304 --steps 2 --warmup 2 --no-cpu-baseline --no-accuracy --e2e-steps 0` (the record
 # stream grows with the rays; at that size ~35 MB of the last records are still in L2 when the
 # kernel ends)
-NCU_TRAFFIC_PER_LAUNCH = 4 * (8776704 + 291551232)
+NCU_TRAFFIC_PER_LAUNCH = 4 * (7841024 + 290515456)
 # The same for the field kernel (trace_kernel<grid>) of the 10,000-heliostat field per launch of
-# 268,435,456 rays: 64 x (15,834,112 + 297,401,344) bytes from `ncu --set full -k regex:^trace_kernel
+# 268,435,456 rays: 64 x (38,493,696 + 304,543,232) bytes from `ncu -k regex:^trace_kernel
 # -s 2 -c 1` of `python bench.py --workload large_field --rays 4194304 --steps 2 --warmup 2
 # --no-cpu-baseline --no-accuracy --e2e-steps 0`, scaled by the rays
-NCU_TRAFFIC_PER_LAUNCH_FIELD = 64 * (15834112 + 297401344)
+NCU_TRAFFIC_PER_LAUNCH_FIELD = 64 * (38493696 + 304543232)
 # Batch kernel (field grid) on the batched workload: warp instructions and DRAM bytes per traced ray,
-# from `ncu --set full -k regex:^batch_kernel -s 2 -c 1` of `python bench.py --workload batched
+# from `ncu -k regex:^batch_kernel -s 2 -c 1` of `python bench.py --workload batched
 # --instances 8 --tuning 256,4,256 --steps 1 --warmup 3 --no-systems --no-cpu-baseline
-# --plain-instances 1` (one launch over 42,028,566 rays): smsp__inst_executed.sum = 3,229,355,334
-# and dram__bytes_read.sum + dram__bytes_write.sum = 52,126,464 + 1,675,776 bytes, per ray.
-BATCH_WARP_INST_PER_RAY = 3229355334 / 42028566
-BATCH_DRAM_BYTES_PER_RAY = (52126464 + 1675776) / 42028566
+# --plain-instances 1` (one launch over 42,028,566 rays): smsp__inst_executed.sum = 2,694,909,092
+# and dram__bytes_read.sum + dram__bytes_write.sum = 53,576,448 + 1,150,208 bytes, per ray.
+BATCH_WARP_INST_PER_RAY = 2694909092 / 42028566
+BATCH_DRAM_BYTES_PER_RAY = (53576448 + 1150208) / 42028566
 ISSUE_PER_SM_PER_CYCLE = 4  # one warp instruction per cycle per scheduler, 4 schedulers per SM
 
 
