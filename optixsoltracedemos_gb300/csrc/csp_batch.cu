@@ -82,7 +82,10 @@ struct BatchSmem {
     typename Cfg<kB, kAccel, false, true>::Core core;
     TraceArgs A;
     FluxTarget F;
-    unsigned long long stat[4];
+    uint32_t stat[4];             // record counters since the last grab: 32-bit shared atomics are one
+                                  // instruction, 64-bit ones a loop (64 instances of three heliostats 0.456 ->
+                                  // 0.437 ms, 16 fields 7.42 -> 7.39)
+    unsigned long long total[4];  // of the instance before it
     unsigned long long grab;
     unsigned long long want;
 };
@@ -96,13 +99,16 @@ constexpr int batch_threads_per_sm() {
     return kAccel == kAccelFlat ? 1152 : 1024;
 }
 
+// Tiles of a grab: its rays' records (at most 4 each) and a queue's stay far below a 32-bit counter.
+constexpr int kMaxGrab = 1 << 20;
+
 template <int kB, int kAccel>
 __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch_kernel(const BatchLaunch L) {
     using C = Cfg<kB, kAccel, false, true>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchSmem<kB, kAccel>& sm = *reinterpret_cast<BatchSmem<kB, kAccel>*>(smem_raw);
     for (uint32_t m = threadIdx.x; m < kH3Tab; m += kB) sm.core.t6[m] = halton3(m);
-    if (threadIdx.x < 4) sm.stat[threadIdx.x] = 0;
+    if (threadIdx.x < 4) sm.stat[threadIdx.x] = sm.total[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         sm.core.qsize = 0;
         sm.core.gsize = 0;
@@ -122,9 +128,9 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
             // every ray of the instance is through: its record counters to the instance's totals
             __syncthreads();
             if (threadIdx.x > 0 && threadIdx.x < 4) {
-                const unsigned long long v = sm.stat[threadIdx.x];
+                const unsigned long long v = sm.total[threadIdx.x] + sm.stat[threadIdx.x];
                 if (v) atomicAdd(sm.F.stats + threadIdx.x, v);
-                sm.stat[threadIdx.x] = 0;
+                sm.stat[threadIdx.x] = sm.total[threadIdx.x] = 0;
             }
             if (done) break;
             flush = have = false;
@@ -132,6 +138,10 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
         }
         if (g == g1) {
             __syncthreads();
+            if (threadIdx.x > 0 && threadIdx.x < 4) {
+                sm.total[threadIdx.x] += sm.stat[threadIdx.x];
+                sm.stat[threadIdx.x] = 0;
+            }
             if (threadIdx.x == 0) {
                 // guided grabs: a quarter of an even share of the tiles left (as this CTA last saw
                 // them), at most L.chunk and at least one, so grabs shrink towards single tiles at the
@@ -140,7 +150,7 @@ __global__ void __launch_bounds__(kB, batch_threads_per_sm<kAccel>() / kB) batch
                 // batches.
                 const unsigned long long left = L.total_tiles > sm.grab ? L.total_tiles - sm.grab : 0;
                 const unsigned long long want =
-                    max(1ull, min((unsigned long long)L.chunk, left / ((unsigned long long)gridDim.x * 4)));
+                    max(1ull, min((unsigned long long)min(L.chunk, kMaxGrab), left / ((unsigned long long)gridDim.x * 4)));
                 sm.grab = atomicAdd(L.next_tile, want);
                 sm.want = want;
             }

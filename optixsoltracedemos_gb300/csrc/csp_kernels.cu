@@ -46,9 +46,9 @@ struct TraceSmem {
 
 // Resident CTAs per SM the register budget is cut for: eight of 128 threads (64 registers, 1,024
 // threads), more warps to cover the record stream of the element-list kernel and the dependent loads
-// of the candidate and cell lists of the others.  Four of 256 threads, with the barriers of a tile over
-// twice the warps: the 10,000-heliostat field 5170 against 5069 us per 64M rays, the single parabolic
-// heliostat 302 against 287 us per 16M; ten of 128 (48 registers, spills) 299 us, two of 512 322 us.
+// of the candidate and cell lists of the others.  64M rays over 10,000 heliostats: seven / eight / nine 4905 /
+// 4656 / 4726 us, four of 256 threads (a tile's barriers over twice the warps) 4691; the single
+// parabolic heliostat, 16M rays: four of 256 302 against 287 us, ten of 128 (48 registers, spills) 299, two of 512 322.
 template <int kAccel>
 constexpr int trace_min_blocks() {
     return 1024 / kTraceBlock;
@@ -59,8 +59,8 @@ constexpr int trace_min_blocks() {
 // tiles differ much in work) and then takes guided grabs (a quarter of an even share of the tiles
 // left, shrinking to single tiles at the end), each requested while the last tile of the one before is
 // traced; grabs and shares are at most kTraceGrab tiles, so that the CTAs work on the same stretch of
-// the sun plane and share its scene data in L2 (the field at caps of 2 / 4 / 8 / 16 / 32 / 64 tiles:
-// 4887 / 4855 / 4857 / 4893 / 4992 / 5070 us per 64M rays).  Without a counter: one contiguous even share
+// the sun plane and share its scene data in L2 (64M rays over 10,000 heliostats at caps of 4 / 8 / 16
+// tiles: 4679 / 4656 / 4652 us; before rows were written by five lanes 32 / 64: 4992 / 5070 against 4857).  Without a counter: one contiguous even share
 // (element lists: the next tile's Halton sums are prefetched) or round robin (fields).  The records
 // do not depend on which CTA traces a tile.  Guided grabs measured 27.5 ms per 268M rays of the
 // 10,000-heliostat field against 30.3 ms round robin (a CTA's tiles differ much in work, so round robin

@@ -1103,28 +1103,22 @@ struct RowStageSmem {
 // Where kFlux records go: the instance's flux target and the CTA's record counters.
 struct Sink {
     const FluxTarget* F;
-    unsigned long long* stat;  // shared memory, [4]
+    uint32_t* stat;  // shared memory, [4]
 };
-
-// warp-aggregated increment by the lanes that execute it together
-__device__ __forceinline__ void warp_count(unsigned long long* s) {
-    const unsigned m = __activemask();
-    if ((int)(threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(s, (unsigned long long)__popc(m));
-}
 
 // Out of line: one copy serves every emit site (the phase A and phase B paths), which keeps the
 // flux kernels' instruction footprint close to the dense ones'.
 __device__ __noinline__ void flux_record(const Sink& k, float4 rec, int slot) {
     if (rec.x == 1.0f) {
-        warp_count(k.stat + 1);
+        atomicAdd(k.stat + 1, 1u);
         return;
     }
     if (slot == 1 && k.F->staged) return;  // direct sun on the receiver: not a staged result
-    warp_count(k.stat + 2);
+    atomicAdd(k.stat + 2, 1u);
     const int b = flux_bin(*k.F, make_float3(rec.y, rec.z, rec.w));
     if (b >= 0 && CSP_BOUNDS(3, b < k.F->nx * k.F->ny)) {
         atomicAdd(k.F->counts + b, 1u);
-        warp_count(k.stat + 3);
+        atomicAdd(k.stat + 3, 1u);
     }
 }
 

@@ -24,3 +24,26 @@ def test_flux_map_edges(gpu, oracle32, name, n):
         counts, _ = t.flux_map(37, 23, staged=staged)
         np.testing.assert_array_equal(counts, oracle32.flux_counts(recs, target, 37, 23)[0])
     t.close()
+
+
+@pytest.mark.parametrize("tuning", [(128, 0, 1), (256, 0, 1 << 30)])
+@pytest.mark.parametrize("name", ["three_heliostats", "single_parabolic"])
+def test_batch_record_counters(gpu, oracle32, name, tuning):
+    """Record counters of batch instances, kept per grab of tiles: grabs of one tile and as large as they
+    get, instances smaller than a CTA among them; equal to the oracle's counts."""
+    rays = [1, 100, 200_003]
+    sc = getattr(scenes, name)(num_rays=1)
+    b = native.Batch(0, 100, 100)
+    sid = b.add_scene(sc.elements)
+    for k, n in enumerate(rays):
+        b.add_instance(sid, sc.sun_dir, sc.sun_shape, sc.sun_param, n, seed=5, instance=k)
+    b.set_tuning(*tuning)
+    b.run()
+    target = native.flux_target(sc.elements[-1])
+    for k, n in enumerate(rays):
+        oh, _ = oracle32.trace(sc.elements, sc.sun_dir, sc.sun_shape, sc.sun_param, 0, n, seed=5, instance=k)
+        counts, _ = oracle32.flux_counts(oh.astype(np.float32), target)
+        np.testing.assert_array_equal(b.counts(k), counts)
+        want = [n, (oh[..., 0] == 1.0).sum(), (oh[..., 0] == 2.0).sum(), counts.sum()]
+        assert [int(v) for v in b.stats(k)] == [int(v) for v in want]
+    b.close()
