@@ -170,8 +170,9 @@ int System::ensure_streams() {
 constexpr uint32_t kPoolElements = 2048;
 
 // Element records of the current elements, packed and put on the device, and the plan of their field
-// grid.  An error of the elements or of the plan leaves the device's scene (and `grid`) as it was; from
-// there on the handle counts as not initialized until the caller is through.
+// grid.  An error of the elements or of the plan, whatever their count, leaves the device's scene
+// (n_scene, the record buffers, `grid`) as it was and traceable; from there on the handle counts as not
+// initialized until the caller is through.
 int System::build_scene(const char* not_planar) {
     const uint32_t n = (uint32_t)elements.size();
     int rc;
@@ -181,26 +182,24 @@ int System::build_scene(const char* not_planar) {
     auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t o_optics = align(n * sizeof(Prim)), o_aabbs = o_optics + align(n * sizeof(Optics));
     const size_t o_prune = o_aabbs + align(n * sizeof(Aabb)), bytes = o_prune + align(n * sizeof(Aabb));
-    if (bytes > cap_records) {
-        // larger buffers next to the old ones, which still serve the device's scene
+    // larger buffers next to the old ones, which serve the device's scene until the new one is accepted
+    struct Grown {
         unsigned char *d = nullptr, *h = nullptr;
-        if ((rc = cuda_status(dev_alloc((void**)&d, bytes), "cudaMalloc element records"))) return rc;
-        if ((rc = cuda_status(host_alloc((void**)&h, bytes), "cudaHostAlloc element records"))) {
-            cudaFree(d);
-            return rc;
+        ~Grown() {
+            if (d) cudaFree(d);
+            if (h) cudaFreeHost(h);
         }
-        initialized = false;
-        cudaFree(d_records);
-        if (h_records) cudaFreeHost(h_records);
-        d_records = d;
-        h_records = h;
-        cap_records = bytes;
+    } grown;
+    if (bytes > cap_records) {
+        if ((rc = cuda_status(dev_alloc((void**)&grown.d, bytes), "cudaMalloc element records"))) return rc;
+        if ((rc = cuda_status(host_alloc((void**)&grown.h, bytes), "cudaHostAlloc element records"))) return rc;
     }
+    unsigned char* const staged = grown.h ? grown.h : h_records;
     auto stage = [&](uint32_t b, uint32_t e) {
-        std::memcpy(h_records + b * sizeof(Prim), &scene.prims[b], (e - b) * sizeof(Prim));
-        std::memcpy(h_records + o_optics + b * sizeof(Optics), &scene.optics[b], (e - b) * sizeof(Optics));
-        std::memcpy(h_records + o_aabbs + b * sizeof(Aabb), &scene.aabbs[b], (e - b) * sizeof(Aabb));
-        std::memcpy(h_records + o_prune + b * sizeof(Aabb), &scene.prune[b], (e - b) * sizeof(Aabb));
+        std::memcpy(staged + b * sizeof(Prim), &scene.prims[b], (e - b) * sizeof(Prim));
+        std::memcpy(staged + o_optics + b * sizeof(Optics), &scene.optics[b], (e - b) * sizeof(Optics));
+        std::memcpy(staged + o_aabbs + b * sizeof(Aabb), &scene.aabbs[b], (e - b) * sizeof(Aabb));
+        std::memcpy(staged + o_prune + b * sizeof(Aabb), &scene.prune[b], (e - b) * sizeof(Aabb));
     };
     std::string err;
     GridStats stats;
@@ -219,6 +218,12 @@ int System::build_scene(const char* not_planar) {
     if (accel != CSP_ACCEL_BVH) plan_grid(scene, stats, plan);
     if (accel == CSP_ACCEL_GRID && !plan.valid && n > kFlatListMax) return fail(CSP_ERR_BAD_SCENE, not_planar);
     initialized = false;
+    if (grown.d) {
+        std::swap(d_records, grown.d);
+        std::swap(h_records, grown.h);
+        cap_records = bytes;
+    }
+    n_scene = n;
     grid = std::move(plan);
     d_prims = reinterpret_cast<Prim*>(d_records);
     d_optics = reinterpret_cast<Optics*>(d_records + o_optics);
@@ -253,7 +258,7 @@ int System::upload_grid() {
         }
         SunGridJob at{};
         field_place(d_field, grid, d_prune, at);
-        grid_host = csp::grid_desc(grid, at.field_cells, at.field_items, d_aabbs + (scene.prims.size() - 1));
+        grid_host = csp::grid_desc(grid, at.field_cells, at.field_items, d_aabbs + (n_scene - 1));
     } else {
         if ((rc = upload(d_cells, cap_cells, grid.cells, stream, "upload grid cells"))) return rc;
         if ((rc = upload(d_items, cap_items, grid.items, stream, "upload grid items"))) return rc;
@@ -276,7 +281,7 @@ int System::prepare_sun() {
     scene.sun[1] = s[1];
     scene.sun[2] = s[2];
     const float tan_pad = tanf(pad_angle());
-    return cuda_status(launch_prepare_sun(d_aabbs, (int)scene.prims.size(), s[0], s[1], s[2], tan_pad, sun_shape,
+    return cuda_status(launch_prepare_sun(d_aabbs, (int)n_scene, s[0], s[1], s[2], tan_pad, sun_shape,
                                           (float)sun_param, d_sun, stream),
                        "prepare_sun_kernel");
 }
@@ -284,7 +289,7 @@ int System::prepare_sun() {
 // Sun-ray candidate grid of the current poses and sun frame, built on the device behind the sun
 // plane (scenes of more than kFlatListMax elements; the element list needs none).
 int System::build_sungrid() {
-    const uint32_t n = (uint32_t)scene.prims.size();
+    const uint32_t n = n_scene;
     if (n <= kFlatListMax) return CSP_OK;
     int rc;
     const size_t bytes = sungrid_bytes(n);
@@ -359,7 +364,7 @@ int System::initialize() {
 int System::update() {
     NvtxRange nvtx("csp update");
     if (!initialized) return fail(CSP_ERR_STATE, "update() before initialize()");
-    if (elements.size() != scene.prims.size())
+    if (elements.size() != n_scene)
         return fail(CSP_ERR_STATE, "update() needs the element count of initialize(); call initialize() again");
     int rc = build_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
     if (rc) return rc;
@@ -386,10 +391,10 @@ TraceArgs System::args(uint64_t begin, uint64_t count) const {
     a.count = count;
     a.seed = seed;
     a.instance = instance;
-    a.n_prims = (int)scene.prims.size();
+    a.n_prims = (int)n_scene;
     a.grid = grid.valid ? d_grid : nullptr;
     a.h3t12 = h3t12;
-    a.sgrid = scene.prims.size() > kFlatListMax && d_sgrid ? sgjob_host.desc : nullptr;
+    a.sgrid = n_scene > kFlatListMax && d_sgrid ? sgjob_host.desc : nullptr;
     a.tile_counter = d_tile_counter;
     return a;
 }

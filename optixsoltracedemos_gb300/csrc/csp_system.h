@@ -53,8 +53,9 @@ struct System {
     bool record_ids = false;
     bool initialized = false;
 
-    HostScene scene;
-    HostGrid grid;
+    HostScene scene;       // of the last elements packed (a refused set-up leaves its own here)
+    HostGrid grid;         // of the scene on the device
+    uint32_t n_scene = 0;  // elements of the scene on the device
     int accel = CSP_ACCEL_AUTO;
 
     HostPool pool;                  // element records of scenes of kPoolElements or more, in ranges
