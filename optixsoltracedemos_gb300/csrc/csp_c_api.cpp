@@ -145,6 +145,7 @@ void System::release() {
     cap_nodes = 0;
     cap_rays = 0;
     ids_allocated = false;
+    loaded = false;
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (copy_stream) cudaStreamDestroy(copy_stream);
@@ -171,8 +172,8 @@ constexpr uint32_t kPoolElements = 2048;
 
 // Element records of the current elements, packed and put on the device, and the plan of their field
 // grid.  An error of the elements or of the plan, whatever their count, leaves the device's scene
-// (n_scene, the record buffers, `grid`) as it was and traceable; from there on the handle counts as not
-// initialized until the caller is through.
+// (n_scene, the record buffers, `grid`) as it was and traceable; from there on the scene is not loaded
+// until the caller is through.
 int System::build_scene(const char* not_planar) {
     const uint32_t n = (uint32_t)elements.size();
     int rc;
@@ -217,7 +218,7 @@ int System::build_scene(const char* not_planar) {
     HostGrid plan;
     if (accel != CSP_ACCEL_BVH) plan_grid(scene, stats, plan);
     if (accel == CSP_ACCEL_GRID && !plan.valid && n > kFlatListMax) return fail(CSP_ERR_BAD_SCENE, not_planar);
-    initialized = false;
+    loaded = false;
     if (grown.d) {
         std::swap(d_records, grown.d);
         std::swap(h_records, grown.h);
@@ -334,6 +335,22 @@ int System::ensure_hit_buffers() {
     return CSP_OK;
 }
 
+// The current elements and sun on the device, complete when it returns.  After a failure past
+// build_scene's checks (device memory) the handle traces nothing until a later update() or initialize()
+// gets through; the records and the flux map of its last run stay readable.
+int System::load_scene(const char* not_planar) {
+    int rc;
+    if ((rc = build_scene(not_planar))) return rc;
+    if ((rc = upload_nodes())) return rc;
+    if ((rc = upload_grid())) return rc;
+    if ((rc = prepare_sun())) return rc;
+    if ((rc = build_sungrid())) return rc;
+    if ((rc = cuda_status(cudaStreamSynchronize(stream), "scene set-up"))) return rc;
+    records_busy = false;
+    loaded = true;
+    return CSP_OK;
+}
+
 int System::initialize() {
     NvtxRange nvtx("csp initialize");
     const auto t0 = std::chrono::steady_clock::now();
@@ -347,15 +364,9 @@ int System::initialize() {
     }
     h3t12 = halton3_table();
     topology = false;
-    if ((rc = build_scene("the scene is not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)"))) return rc;
     if (!d_sun && (rc = cuda_status(dev_alloc((void**)&d_sun, sizeof(SunFrame)), "cudaMalloc sun"))) return rc;
-    if ((rc = upload_nodes())) return rc;
-    if ((rc = upload_grid())) return rc;
-    if ((rc = prepare_sun())) return rc;
-    if ((rc = build_sungrid())) return rc;
+    if ((rc = load_scene("the scene is not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)"))) return rc;
     if ((rc = ensure_hit_buffers())) return rc;
-    if ((rc = cuda_status(cudaStreamSynchronize(stream), "initialize"))) return rc;
-    records_busy = false;
     initialized = true;
     time_setup = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return CSP_OK;
@@ -366,17 +377,8 @@ int System::update() {
     if (!initialized) return fail(CSP_ERR_STATE, "update() before initialize()");
     if (elements.size() != n_scene)
         return fail(CSP_ERR_STATE, "update() needs the element count of initialize(); call initialize() again");
-    int rc = build_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
-    if (rc) return rc;
-    if ((rc = upload_nodes())) return rc;
-    if ((rc = upload_grid())) return rc;
-    if ((rc = prepare_sun())) return rc;
-    if ((rc = build_sungrid())) return rc;
-    if ((rc = ensure_hit_buffers())) return rc;
-    if ((rc = cuda_status(cudaStreamSynchronize(stream), "update"))) return rc;
-    records_busy = false;
-    initialized = true;
-    return CSP_OK;
+    const int rc = load_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)");
+    return rc ? rc : ensure_hit_buffers();
 }
 
 TraceArgs System::args(uint64_t begin, uint64_t count) const {
@@ -400,7 +402,7 @@ TraceArgs System::args(uint64_t begin, uint64_t count) const {
 }
 
 int System::trace_async(cudaStream_t st) {
-    if (!initialized) return fail(CSP_ERR_STATE, "trace before initialize()");
+    if (!ready()) return fail(CSP_ERR_STATE, "trace before initialize()");
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     // it writes the hit buffer: it never overlaps the handle's other launches, so the tile counter
@@ -410,7 +412,7 @@ int System::trace_async(cudaStream_t st) {
 
 int System::run() {
     NvtxRange nvtx("csp run");
-    if (!initialized) return fail(CSP_ERR_STATE, "run() before initialize()");
+    if (!ready()) return fail(CSP_ERR_STATE, "run() before initialize()");
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     if ((rc = cuda_status(cudaEventRecord(ev0, stream), "cudaEventRecord"))) return rc;
@@ -425,7 +427,7 @@ int System::run() {
 
 int System::run_to_host(float* dst, uint32_t* ids_dst) {
     NvtxRange nvtx("csp run_to_host");
-    if (!initialized) return fail(CSP_ERR_STATE, "run() before initialize()");
+    if (!ready()) return fail(CSP_ERR_STATE, "run() before initialize()");
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     const uint64_t chunk = std::max<uint64_t>(1u << 20, (num_rays + 15) / 16);
@@ -559,7 +561,7 @@ int System::run_compact_chunks(float* points, uint8_t* counts, float* records, u
 int System::run_to_host_compact(float* points, uint8_t* counts, float* records, uint64_t capacity,
                                 uint64_t* n_records) {
     NvtxRange nvtx("csp run_to_host_compact");
-    if (!initialized) return fail(CSP_ERR_STATE, "run() before initialize()");
+    if (!ready()) return fail(CSP_ERR_STATE, "run() before initialize()");
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     const uint64_t n = num_rays;
@@ -875,7 +877,7 @@ int csp_copy_hits(csp_handle h, float* dst, uint32_t* ids, uint64_t first, uint6
 int csp_trace_into(csp_handle h, void* hits, void* ids, uint64_t first, uint64_t count, void* stream) {
     CSP_GUARD(h);
     System* s = reinterpret_cast<System*>(h);
-    if (!s->initialized) return fail(CSP_ERR_STATE, "trace before initialize()");
+    if (!s->ready()) return fail(CSP_ERR_STATE, "trace before initialize()");
     if (!hits && count) return fail(CSP_ERR_INVALID_ARGUMENT, "null hit buffer");
     if (!csp::valid_ray_window(first, count))
         return fail(CSP_ERR_INVALID_ARGUMENT, "ray window [first_ray, first_ray + count) must stay below 2^56");

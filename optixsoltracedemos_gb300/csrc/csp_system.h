@@ -51,7 +51,8 @@ struct System {
     uint64_t seed = 0;
     uint32_t instance = 0;
     bool record_ids = false;
-    bool initialized = false;
+    bool initialized = false;  // since the last set_accel
+    bool loaded = false;       // the device's scene is complete (a set-up that fails half-way leaves it false)
 
     HostScene scene;       // of the last elements packed (a refused set-up leaves its own here)
     HostGrid grid;         // of the scene on the device
@@ -120,7 +121,9 @@ struct System {
     ~System();
     void release();
     int ensure_streams();
+    bool ready() const { return initialized && loaded; }
     int build_scene(const char* not_planar);
+    int load_scene(const char* not_planar);
     int upload_nodes();
     int upload_grid();
     int prepare_sun();

@@ -51,3 +51,58 @@ def test_refused_initialize_keeps_the_scene(gpu, oracle32, held, refused, why):
     t.update()
     _expect(t, sc, oracle32)
     t.close()
+
+
+@pytest.mark.parametrize("heliostats", [4, 300])
+def test_update_without_memory_for_the_records(gpu, oracle32, heliostats):
+    """More rays than memory for their records: update() fails, and fewer rays trace its scene."""
+    sc = _field(heliostats)
+    t = native.tracer_for(sc, seed=5, num_rays=RAYS)
+    moved = scenes.reaim(sc.elements, scenes.sun_vector(50.0, -10.0))
+    sc.elements, sc.sun_dir = moved, scenes.sun_vector(50.0, -10.0)
+    t.set_elements(moved)
+    t.set_sun_vector(sc.sun_dir)
+    t.set_num_rays(2 * RAYS)
+    native.debug_fail_allocation(0)
+    try:
+        with pytest.raises(native.CspError) as e:
+            t.update()
+        assert e.value.status == -3
+    finally:
+        native.debug_fail_allocation(-1)
+    t.set_num_rays(RAYS)
+    _expect(t, sc, oracle32)
+    t.close()
+
+
+@pytest.mark.parametrize("accel", [native.ACCEL_GRID, native.ACCEL_BVH])
+def test_update_that_fails_can_be_repeated(gpu, oracle32, accel):
+    """A re-initialize() whose k-th allocation fails traces nothing; update() alone completes it."""
+    small, sc = _field(20), _field(300)
+    for k in range(16):
+        t = native.tracer_for(small, seed=5, num_rays=RAYS, accel=accel)
+        t.run()
+        t.set_elements(sc.elements)
+        native.debug_fail_allocation(k)
+        try:
+            t.initialize()
+            failed = False
+        except native.CspError as e:
+            assert e.status == -3
+            failed = True
+        finally:
+            native.debug_fail_allocation(-1)
+        if not failed:
+            assert k >= 2
+            break
+        assert t.copy_hits()[0].any()  # the last run's
+        if k < 2:  # the element records' buffers: before the new scene is accepted
+            _expect(t, small, oracle32)
+            t.initialize()
+        else:
+            with pytest.raises(native.CspError) as e:
+                t.run()
+            assert e.value.status == -6
+            t.update()
+        _expect(t, sc, oracle32)
+        t.close()
