@@ -144,8 +144,8 @@ CSP_API int csp_initialize(csp_handle h);
 /* Trace num_rays rays and wait for them (run()).  Fully rewrites the num_rays x 5 hit buffer. */
 CSP_API int csp_run(csp_handle h);
 /* Enqueue the trace on `stream` (a cudaStream_t, NULL = the handle's own stream); no host sync.
- * It writes the handle's hit buffer, so it must not overlap another run or trace of the handle on
- * the GPU (it also shares the handle's work counter with them). */
+ * It writes the handle's hit buffer, so it must not overlap another run of the handle, nor a copy of
+ * its records or its flux map, on the GPU; windows of csp_trace_into may be traced meanwhile. */
 CSP_API int csp_trace_async(csp_handle h, void* stream);
 /* Re-read the element poses given since initialize (same count), refit the acceleration structure
  * in place and recompute the sun plane (update()). */

@@ -112,10 +112,10 @@ void System::release() {
     cap_cells = cap_items = cap_global = 0;
     cudaFree(d_sgrid);
     cudaFree(d_sgjob);
-    cudaFree(d_tile_counter);
+    cudaFree(d_counters);
     d_sgrid = nullptr;
     d_sgjob = nullptr;
-    d_tile_counter = nullptr;
+    d_counters = nullptr;
     cap_sgrid = 0;
     cudaFree(d_cpoints);
     cudaFree(d_ccounts);
@@ -345,6 +345,8 @@ int System::load_scene(const char* not_planar) {
     if ((rc = upload_grid())) return rc;
     if ((rc = prepare_sun())) return rc;
     if ((rc = build_sungrid())) return rc;
+    // zero before the first launch, and every launch leaves its counter so
+    if ((rc = cuda_status(cudaMemsetAsync(d_counters, 0, kCounterBytes, stream), "memset"))) return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "scene set-up"))) return rc;
     records_busy = false;
     loaded = true;
@@ -356,12 +358,8 @@ int System::initialize() {
     const auto t0 = std::chrono::steady_clock::now();
     int rc = ensure_streams();
     if (rc) return rc;
-    if (!d_tile_counter) {
-        if ((rc = cuda_status(dev_alloc((void**)&d_tile_counter, 2 * sizeof(unsigned int)), "cudaMalloc tile counter")))
-            return rc;
-        // zero before the first launch; every launch leaves it so
-        if ((rc = cuda_status(cudaMemsetAsync(d_tile_counter, 0, 2 * sizeof(unsigned int), stream), "memset"))) return rc;
-    }
+    if (!d_counters && (rc = cuda_status(dev_alloc((void**)&d_counters, kCounterBytes), "cudaMalloc tile counters")))
+        return rc;
     h3t12 = halton3_table();
     topology = false;
     if (!d_sun && (rc = cuda_status(dev_alloc((void**)&d_sun, sizeof(SunFrame)), "cudaMalloc sun"))) return rc;
@@ -381,7 +379,22 @@ int System::update() {
     return rc ? rc : ensure_hit_buffers();
 }
 
-TraceArgs System::args(uint64_t begin, uint64_t count) const {
+// Work counter of a launch on `st`.  A launch hands out its tiles by its counter and leaves it zero, so two
+// that overlap on the GPU must not share one, or they and every later launch of it would skip tiles: the
+// launches take turns on kCounters of them, captured ones (whose counter stays with the graph) on as many
+// others.
+unsigned int* System::next_counter(cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st != stream && cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+        cudaGetLastError();  // the launch itself reports what is wrong with the stream
+        capture = cudaStreamCaptureStatusNone;
+    }
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    const unsigned k = (captured ? next_captured : next_eager).fetch_add(1u, std::memory_order_relaxed) % kCounters;
+    return d_counters + 2 * (captured ? kCounters + k : k);
+}
+
+TraceArgs System::args(uint64_t begin, uint64_t count, unsigned int* counter) const {
     TraceArgs a;
     a.nodes = d_nodes;
     a.prims = d_prims;
@@ -397,7 +410,7 @@ TraceArgs System::args(uint64_t begin, uint64_t count) const {
     a.grid = grid.valid ? d_grid : nullptr;
     a.h3t12 = h3t12;
     a.sgrid = n_scene > kFlatListMax && d_sgrid ? sgjob_host.desc : nullptr;
-    a.tile_counter = d_tile_counter;
+    a.tile_counter = counter;
     return a;
 }
 
@@ -405,9 +418,8 @@ int System::trace_async(cudaStream_t st) {
     if (!ready()) return fail(CSP_ERR_STATE, "trace before initialize()");
     int rc = ensure_hit_buffers();
     if (rc) return rc;
-    // it writes the hit buffer: it never overlaps the handle's other launches, so the tile counter
-    // serves it on any stream
-    return cuda_status(launch_trace(args(0, num_rays), st ? st : stream), "trace_kernel");
+    if (!st) st = stream;
+    return cuda_status(launch_trace(args(0, num_rays, next_counter(st)), st), "trace_kernel");
 }
 
 int System::run() {
@@ -416,7 +428,7 @@ int System::run() {
     int rc = ensure_hit_buffers();
     if (rc) return rc;
     if ((rc = cuda_status(cudaEventRecord(ev0, stream), "cudaEventRecord"))) return rc;
-    if ((rc = cuda_status(launch_trace(args(0, num_rays), stream), "trace_kernel"))) return rc;
+    if ((rc = cuda_status(launch_trace(args(0, num_rays, next_counter(stream)), stream), "trace_kernel"))) return rc;
     if ((rc = cuda_status(cudaEventRecord(ev1, stream), "cudaEventRecord"))) return rc;
     if ((rc = cuda_status(cudaEventSynchronize(ev1), "trace"))) return rc;
     float ms = 0.f;
@@ -435,7 +447,7 @@ int System::run_to_host(float* dst, uint32_t* ids_dst) {
     const auto t0 = std::chrono::steady_clock::now();
     for (uint64_t b = 0; b < num_rays; b += chunk) {
         const uint64_t c = std::min(chunk, num_rays - b);
-        if ((rc = cuda_status(launch_trace(args(b, c), stream), "trace_kernel"))) break;
+        if ((rc = cuda_status(launch_trace(args(b, c, next_counter(stream)), stream), "trace_kernel"))) break;
         cudaEvent_t ev;
         if ((rc = cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate"))) break;
         done.push_back(ev);
@@ -514,7 +526,7 @@ int System::run_compact_chunks(float* points, uint8_t* counts, float* records, u
             const int at = (int)(k % kCompactRing);
             unsigned long long* sums = d_csums + (chunk / 256 + 1) * at;
             const float4* rows = d_hits + cur.begin * kMaxDepth;
-            rc = cuda_status(launch_trace(args(cur.begin, cur.count), stream), "trace_kernel");
+            rc = cuda_status(launch_trace(args(cur.begin, cur.count, next_counter(stream)), stream), "trace_kernel");
             if (!rc && k >= kCompactRing)
                 rc = cuda_status(cudaStreamWaitEvent(stream, copied[at], 0), "cudaStreamWaitEvent");
             if (!rc)
@@ -593,7 +605,7 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
             return rc ? rc : timed();
         }
     }
-    if ((rc = cuda_status(launch_trace(args(0, n), stream), "trace_kernel"))) return rc;
+    if ((rc = cuda_status(launch_trace(args(0, n, next_counter(stream)), stream), "trace_kernel"))) return rc;
     if ((rc = cuda_status(launch_compact_count(d_hits, n, d_cpoints, d_ccounts, d_csums, nullptr, stream),
                           "compact_count_kernel")))
         return rc;
@@ -881,13 +893,13 @@ int csp_trace_into(csp_handle h, void* hits, void* ids, uint64_t first, uint64_t
     if (!hits && count) return fail(CSP_ERR_INVALID_ARGUMENT, "null hit buffer");
     if (!csp::valid_ray_window(first, count))
         return fail(CSP_ERR_INVALID_ARGUMENT, "ray window [first_ray, first_ray + count) must stay below 2^56");
-    csp::TraceArgs a = s->args(0, 0);
+    cudaStream_t st = stream ? reinterpret_cast<cudaStream_t>(stream) : s->stream;
+    // off the handle's stream static shares of the tiles
+    csp::TraceArgs a = s->args(0, 0, st == s->stream ? s->next_counter(st) : nullptr);
     a.hits = reinterpret_cast<float4*>(hits);
     a.ids = reinterpret_cast<uint32_t*>(ids);
     a.ray_begin = first;
     a.count = count;
-    cudaStream_t st = stream ? reinterpret_cast<cudaStream_t>(stream) : s->stream;
-    if (st != s->stream) a.tile_counter = nullptr;  // may overlap the launches on the handle's stream
     return csp::cuda_status(csp::launch_trace(a, st), "trace_kernel");
 }
 

@@ -46,8 +46,8 @@ struct TraceArgs {
     const float* h3t12;    // Halton base-3 partial sums after 12 digits (halton3_table), or nullptr
     const SunGrid* sgrid;  // candidate grid of the sun rays (scenes of more than 8 elements)
     // single-scene launches: tiles handed out by this device counter ([0] tiles, [1] CTAs done; zero
-    // between launches, the last CTA sees to that) in guided grabs; nullptr: static shares (launches
-    // that may overlap on the GPU with another of the same counter use that)
+    // between launches, the last CTA sees to that) in guided grabs; launches that overlap on the GPU have
+    // different ones.  nullptr: static shares
     unsigned int* tile_counter;
 };
 

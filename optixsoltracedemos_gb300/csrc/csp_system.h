@@ -1,6 +1,7 @@
 // csp_system.h -- state behind one csp_handle.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -91,7 +92,11 @@ struct System {
     unsigned char* d_sgrid = nullptr;
     size_t cap_sgrid = 0;
     SunGridJob* d_sgjob = nullptr;
-    unsigned int* d_tile_counter = nullptr;  // guided tile grabs of the launches on `stream`
+    // work counters {tiles, CTAs done} of the launches, see next_counter
+    static constexpr unsigned kCounters = 64;
+    static constexpr size_t kCounterBytes = 2 * kCounters * 2 * sizeof(unsigned int);
+    unsigned int* d_counters = nullptr;
+    std::atomic<unsigned> next_eager{0}, next_captured{0};
     SunGridJob sgjob_host{};
     // compact records (csp_run_to_host_compact): points, counts, block offsets, records
     float* d_cpoints = nullptr;
@@ -132,7 +137,8 @@ struct System {
     int ensure_hit_buffers();
     int initialize();
     int update();
-    TraceArgs args(uint64_t begin, uint64_t count) const;
+    unsigned int* next_counter(cudaStream_t st);
+    TraceArgs args(uint64_t begin, uint64_t count, unsigned int* counter) const;
     int trace_async(cudaStream_t st);
     int run();
     int run_to_host(float* dst, uint32_t* ids);
