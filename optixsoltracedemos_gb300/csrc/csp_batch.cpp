@@ -44,9 +44,15 @@
 namespace csp {
 namespace {
 
-// offsets 32-byte aligned: the kernels read records and boxes 32 bytes at a time
-constexpr size_t kPoolElements = 4096;    // elements of a run from which its host builds use the batch's threads
+// Host work of a run goes on the batch's threads where one thread would take longer: waking them costs
+// about 20 us and each instance, one task, about 1.1 us more.  One thread packs an element of own poses in
+// 0.105 us (8 x 200 elements 166 us, 56 on the threads; 64 x 16 130 and 100; 256 x 8 309 and 310) and copies one
+// into the staging image in about 4 ns, of instances with and without poses alike (16 x 2,000 elements 100
+// us, 46 on the threads; 4 x 2,000 25 and 29; 64 x 250 70 and 90).
+bool pack_on_threads(size_t elements, size_t instances) { return instances > 1 && elements >= 512 + 8 * instances; }
+bool copy_on_threads(size_t elements, size_t instances) { return instances > 1 && elements >= 8192 + 256 * instances; }
 constexpr size_t kKeepElements = 400000;  // elements (of ~160 B) of a run whose host records stay allocated
+// offsets 32-byte aligned: the kernels read records and boxes 32 bytes at a time
 size_t align32(size_t x) { return (x + 31) & ~(size_t)31; }
 
 // Tuned launch parameters per (device model, kernel build, kernel group, ray-count class), shared
@@ -763,11 +769,13 @@ int Batch::run_async() {
     // both parallel over instances
     const size_t n = inst.size();
     builds.resize(n);  // the vectors of the last run's are reused
-    size_t total = 0;
-    for (size_t i = 0; i < n; ++i) total += inst[i].poses.empty() ? 0 : count_of(i);
-    const bool pooled = total >= kPoolElements && n > 1;
-    if (pooled && !pool.started()) pool.start(std::min(63u, std::max(2u, std::thread::hardware_concurrency()) - 1));
-    auto parallel = [&](auto&& fn) {
+    size_t own = 0, all = 0;  // elements of the instances with poses of their own, of all instances
+    for (size_t i = 0; i < n; ++i) {
+        all += count_of(i);
+        if (!inst[i].poses.empty()) own += count_of(i);
+    }
+    auto parallel = [&](bool pooled, auto&& fn) {
+        if (pooled && !pool.started()) pool.start(std::min(63u, std::max(2u, std::thread::hardware_concurrency()) - 1));
         std::vector<int> irc(n, CSP_OK);
         std::vector<std::string> ierr(n);
         auto one = [&](size_t i) { irc[i] = fn(i, ierr[i]); };
@@ -778,9 +786,10 @@ int Batch::run_async() {
             if (irc[i]) return set_error(irc[i], "instance " + std::to_string(i) + ": " + ierr[i]);
         return (int)CSP_OK;
     };
-    if ((rc = parallel([&](size_t i, std::string& err) { return build_instance(i, err); }))) return rc;
+    if ((rc = parallel(pack_on_threads(own, n), [&](size_t i, std::string& err) { return build_instance(i, err); })))
+        return rc;
     if ((rc = layout(si))) return rc;
-    if ((rc = parallel([&](size_t i, std::string&) {
+    if ((rc = parallel(copy_on_threads(all, n), [&](size_t i, std::string&) {
              fill_instance(i);
              return (int)CSP_OK;
          })))
@@ -795,7 +804,7 @@ int Batch::run_async() {
     write_descs(desc, tb, h_stage);
     // everything the device needs is in the staging image now; the builds of small batches keep their
     // memory for the next run
-    if (total > kKeepElements) {
+    if (own > kKeepElements) {
         builds.clear();
         builds.shrink_to_fit();
     }

@@ -111,7 +111,7 @@ struct Batch {
     int max_field_cells = 0;  // of the field grids that the device builds
     int n_sg = 0, max_n = 0;  // sun grid build jobs; largest element count of the instances
     std::vector<InstBuild> builds;  // per instance, during a run (instances with poses)
-    HostPool pool;                  // host builds of batches of kPoolElements or more
+    HostPool pool;                  // packing and copies of larger runs
     int n_refit = 0, max_nodes = 0;  // refit jobs and their largest node count
 
     double time_setup = 0.0, time_trace = 0.0;  // of the last completed run
