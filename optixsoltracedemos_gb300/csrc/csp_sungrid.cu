@@ -10,7 +10,7 @@
 // the lower element index on equal t whatever the order of the candidates.
 //
 // Four launches per set of states:
-//   size    a cluster of kStateCluster blocks per state (dependent reductions over the elements: the
+//   size    a block or a cluster of kStateCluster blocks per state (dependent reductions over the elements: the
 //           middle of the field and with it the reference plane; every element's rectangles; the grid
 //           size from the candidate rectangles' mean extent, shrunk until the registered items fit
 //           the capacity), the descriptor, zeroed counts and raster
@@ -38,6 +38,7 @@ constexpr int kMaxAxisCells = 4096;
 constexpr float kCellScale = 0.5f;  // cell width / mean rectangle width
 constexpr int kMaxJobsPerLaunch = 65535;  // gridDim.y limit
 constexpr int kElemBlock = 256;
+constexpr int kWideField = 65536;  // field cells (0.5 MB) from which one block would take long to zero them
 constexpr int kElemLanes = 8;  // lanes that share an element's cells and raster words
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -67,12 +68,13 @@ __device__ __forceinline__ void set_reach(uint32_t* __restrict__ raster, float4 
     }
 }
 
-__global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
+template <int kCluster>
+__global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kCluster)
     sungrid_size_kernel(const SunGridJob* __restrict__ jobs) {
-    const SunGridJob& J = jobs[blockIdx.x / kStateCluster];
+    const SunGridJob& J = jobs[blockIdx.x / kCluster];
     const int n = J.n;
-    constexpr int kThreads = kStateCluster * kStateBlock;
-    const int tid = (int)(blockIdx.x % kStateCluster) * kStateBlock + (int)threadIdx.x;
+    constexpr int kThreads = kCluster * kStateBlock;
+    const int tid = (int)(blockIdx.x % kCluster) * kStateBlock + (int)threadIdx.x;
     __shared__ SunFrame S;
     __shared__ StateSmem sm;
     __shared__ unsigned long long upart[kStateBlock / 32], uslot;
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
             hhi = fmaxf(hhi, h);
         }
     }
-    const float4 mid = state_reduce<kStateCluster>(make_float4(zlo, -zhi, hlo, -hhi), sm.part, &sm.slot, Min4());
+    const float4 mid = state_reduce<kCluster>(make_float4(zlo, -zhi, hlo, -hhi), sm.part, &sm.slot, Min4());
     const float dz = fabsf(S.w.z) - tan_a * sqrtf(fmaxf(0.0f, 1.0f - S.w.z * S.w.z));
     const bool level = dz > 0.02f && (-mid.y - mid.x) < dz * (-mid.w - mid.z);
     const float4 plane = level ? make_float4(0.0f, 0.0f, 1.0f, 0.5f * (mid.x - mid.y))
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
         const float wu = __saturatef(r.y) - __saturatef(r.x), wv = __saturatef(r.w) - __saturatef(r.z);
         if (wu < 0.25f && wv < 0.25f) ext = Sum()(ext, make_float4(wu, wv, 1.0f, 0.0f));
     }
-    ext = state_reduce<kStateCluster>(ext, sm.part, &sm.slot, Sum());
+    ext = state_reduce<kCluster>(ext, sm.part, &sm.slot, Sum());
     // cells half as wide as the mean rectangle: a rectangle covers about 3 x 3 cells
     int nu = 1, nv = 1;
     if (ext.z > 0.0f) {
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
             const long long cells = (long long)(iu1 - iu0 + 1) * (iv1 - iv0 + 1);
             if (cells <= kSunGridMaxCells) items += (unsigned long long)cells;
         }
-        total = state_reduce<kStateCluster>(items, upart, &uslot, Sum());
+        total = state_reduce<kCluster>(items, upart, &uslot, Sum());
         if (total <= J.cap_items || (nu == 1 && nv == 1)) break;
         nu = max(1, nu * 3 / 4);
         nv = max(1, nv * 3 / 4);
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kStateBlock) __cluster_dims__(kStateCluster)
         d.aabbs = J.aabbs;
         *J.desc = d;
     }
-    cooperative_groups::this_cluster().sync();  // the slots are read
+    if constexpr (kCluster > 1) cooperative_groups::this_cluster().sync();  // the slots are read
 }
 
 // Cells of element e's candidate rectangle, k-th of `cells`.
@@ -358,7 +360,12 @@ cudaError_t launch_sungrid_build(const SunGridJob* jobs, int n_jobs, int max_n, 
     for (int j0 = 0; j0 < n_jobs; j0 += kMaxJobsPerLaunch) {
         const unsigned nj = (unsigned)std::min(kMaxJobsPerLaunch, n_jobs - j0);
         const SunGridJob* J = jobs + j0;
-        sungrid_size_kernel<<<nj * kStateCluster, kStateBlock, 0, stream>>>(J);
+        // A block does for few elements and field cells to zero: a cluster for each of 64 states of 101
+        // elements is 512 CTAs in two waves, 25.6 us against 9 (one state alone 4.5 against 5).
+        if (max_n >= kStateClusterMin || max_field_cells >= kWideField)
+            sungrid_size_kernel<kStateCluster><<<nj * kStateCluster, kStateBlock, 0, stream>>>(J);
+        else
+            sungrid_size_kernel<1><<<nj, kStateBlock, 0, stream>>>(J);
         sungrid_count_kernel<<<dim3(elem_blocks, nj, parts), kElemBlock, 0, stream>>>(J);
         sungrid_ranges_kernel<<<dim3(cell_blocks, nj, parts), kElemBlock, 0, stream>>>(J);
         sungrid_fill_kernel<<<dim3(elem_blocks, nj, parts), kElemBlock, 0, stream>>>(J);

@@ -111,8 +111,9 @@ struct Cfg {
 // walk the same grid cells.  A launch is cut into whole blocks of S1 = 2^8 3^5 first, then over what is
 // left of S2 = 2^7 3^4 and of S3 = 2^6 3^3 (55,296 rays), then the identity order for the tail: a
 // bijection on [0, count).  Without S3 up to 331,775 rays went in identity order (1.2M rays of a
-// hillside of 600: 91.5 us, 87.3 with it).  Launches without dense records (kFine) take blocks of
-// S0 = 2^9 3^6 (11,943,936 rays) before S1 and none of S3: they gain from the smaller patches, while in
+// hillside of 600: 91.5 us, 87.3 with it; 64 instances of 65,536 rays over 100 heliostats 239 us, 170 with
+// it; 16 of 400,000 over 10,000 864 and 833).  Launches without dense records (kFine) take blocks of
+// S0 = 2^9 3^6 (11,943,936 rays) before S1: they gain from the smaller patches, while in
 // dense launches a warp's 32 rows would span ~1 GB of the hit buffer (64M rays of 10,000 heliostats:
 // 5349 us against 4861).
 // With G > 1 groups of G consecutive warps (of one tile, i.e. CTA) take neighbouring patches: warp k of
@@ -145,7 +146,7 @@ __device__ __forceinline__ U coherent_order_t(U kk, U count) {
     if (kFine && coherent_level<kCoherentS0, G>(kk, count, first)) return first + kk;
     if (coherent_level<kCoherentS1, G>(kk, count, first)) return first + kk;
     if (coherent_level<kCoherentS2, G>(kk, count, first)) return first + kk;
-    if (!kFine) coherent_level<kCoherentS3, G>(kk, count, first);
+    coherent_level<kCoherentS3, G>(kk, count, first);
     return first + kk;
 }
 
