@@ -775,7 +775,8 @@ int Batch::run_async() {
         if (!inst[i].poses.empty()) own += count_of(i);
     }
     auto parallel = [&](bool pooled, auto&& fn) {
-        if (pooled && !pool.started()) pool.start(std::min(63u, std::max(2u, std::thread::hardware_concurrency()) - 1));
+        if (pooled)
+            pool.start(std::min({63u, std::max(2u, std::thread::hardware_concurrency()) - 1, (unsigned)n - 1}));
         std::vector<int> irc(n, CSP_OK);
         std::vector<std::string> ierr(n);
         auto one = [&](size_t i) { irc[i] = fn(i, ierr[i]); };

@@ -166,8 +166,9 @@ int System::ensure_streams() {
     return cuda_status(cudaEventCreate(&ev1), "cudaEventCreate");
 }
 
-// Element count from which a scene's records are packed on the handle's host threads (10,001 elements
-// take 904 us on one thread of a 16-core host; a whole update() takes 323 us on sixteen).
+// Element count from which a scene's records are packed on the handle's host threads.  With the threads
+// up, a whole update() is as fast with as without them at 700 elements (129 and 134 us; 2,000: 271 and 174,
+// 4,000: 495 and 276 on a 16-core host), but they have to pay for their start first.
 constexpr uint32_t kPoolElements = 2048;
 
 // Element records of the current elements, packed and put on the device, and the plan of their field
@@ -205,7 +206,7 @@ int System::build_scene(const char* not_planar) {
     std::string err;
     GridStats stats;
     if (n >= kPoolElements) {
-        if (!pool.started()) pool.start(std::min(15u, std::max(2u, std::thread::hardware_concurrency()) - 1));
+        pool.start(std::min({15u, std::max(2u, std::thread::hardware_concurrency()) - 1, build_ranges(n) - 1}));
         rc = build_elements(
             elements.data(), n, scene, err,
             [this](size_t tasks, const std::function<void(size_t)>& body) { pool.run(tasks, body); }, &stats, stage);

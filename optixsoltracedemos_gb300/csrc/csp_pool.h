@@ -4,6 +4,7 @@
 #include <condition_variable>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <thread>
@@ -11,16 +12,20 @@
 
 namespace csp {
 
-// Fixed set of host threads for the parallel part of a scene's set-up (element records in ranges),
-// owned by one handle, batch or server and joined with it.  run() executes body(k) for k in [0, tasks) on the pool and the calling thread and returns when all
-// are done; concurrent callers take turns.
+// Host threads for the parallel part of a scene's set-up (element records in ranges), owned by one
+// handle, batch or server and joined with it.  run() executes body(k) for k in [0, tasks) on the pool and
+// the calling thread and returns when all are done; concurrent callers take turns.  body must not throw.
 class HostPool {
 public:
     ~HostPool() { stop(); }
-    bool started() const { return !th_.empty(); }
+    // At least `threads` threads, or as many as the system gives: run() does without any.  One costs about
+    // 55 us, so callers ask for what their tasks can use.
     void start(unsigned threads) {
-        quit_ = false;
-        for (unsigned t = 0; t < threads; ++t) th_.emplace_back([this] { loop(); });
+        try {
+            th_.reserve(threads);
+            while (th_.size() < threads) th_.emplace_back([this] { loop(); });
+        } catch (const std::exception&) {  // no thread, or no memory for one
+        }
     }
     void stop() {
         {
@@ -30,6 +35,7 @@ public:
         cv_.notify_all();
         for (auto& t : th_) t.join();
         th_.clear();
+        quit_ = false;
     }
     void run(size_t tasks, const std::function<void(size_t)>& body) {
         std::lock_guard<std::mutex> turn(run_mu_);

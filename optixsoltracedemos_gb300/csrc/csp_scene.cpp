@@ -350,7 +350,7 @@ int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string&
     if (rc) return rc;
     size_scene(n, s);
     constexpr uint32_t kRange = kBuildChunk / 2;
-    const size_t chunks = (n + kRange - 1) / kRange;
+    const size_t chunks = build_ranges(n);
     std::vector<uint32_t> bad(chunks);
     std::vector<int> status(chunks, CSP_OK);
     std::vector<const char*> whys(chunks, "");

@@ -48,6 +48,7 @@ using ParallelFor = std::function<void(size_t tasks, const std::function<void(si
 // (each element's packing reads only that element), and the same error (the lowest failing element).
 // `packed(begin, end)` is called on the thread that packed the range, if given.
 constexpr uint32_t kBuildChunk = 1024;
+inline uint32_t build_ranges(uint32_t n) { return (n + kBuildChunk / 2 - 1) / (kBuildChunk / 2); }
 int build_elements(const csp_element* el, uint32_t n, HostScene& s, std::string& err, const ParallelFor& pf,
                    GridStats* stats = nullptr, const std::function<void(uint32_t, uint32_t)>& packed = nullptr);
 

@@ -90,3 +90,16 @@ def test_rsqrt_near_1_equals_square_root_and_division(tmp_path):
                     os.path.join(root, "tests", "cpp", "rsqrt_near_1_check.cpp"), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "0 mismatches", r.stdout
+
+
+def test_host_pool_without_threads(tmp_path):
+    """Threads that the system refuses leave the pool with fewer, not the process with an exception."""
+    import shutil
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = str(tmp_path / "host_pool_check")
+    subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-O2", "-pthread", "-I",
+                    os.path.join(root, "optixsoltracedemos_gb300", "csrc"),
+                    os.path.join(root, "tests", "cpp", "host_pool_check.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "OK", r.stdout + r.stderr
