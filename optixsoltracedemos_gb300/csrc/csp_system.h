@@ -128,7 +128,7 @@ struct System {
     int ensure_streams();
     bool ready() const { return initialized && loaded; }
     int build_scene(const char* not_planar);
-    int load_scene(const char* not_planar);
+    int load_scene(const char* not_planar, bool first);
     int upload_nodes();
     int upload_grid();
     int prepare_sun();
