@@ -476,13 +476,17 @@ int System::run_to_host(float* dst, uint32_t* ids_dst) {
 }
 
 // Chunks of a compact run: traced and compacted on `stream` while the chunk before is copied on
-// `copy_stream`, a quarter of the run each, at most 2^20 rays (84 MB of rows, still in L2 when they are
-// compacted) and at least 2^17 (below, a chunk's kernels are shorter than its launches).  A copy costs
-// about 2 us besides its bytes (16 B per ray of the single parabolic heliostat at the host link's ~190
-// GB/s), so the counts follow in one copy at the end.  4M rays of that heliostat: 577 us in one piece,
-// 445 in eight chunks, 436 in four, 444 to 464 with chunks that start at 2^18 or 2^17 and double; the
-// copies alone 349 us.
-constexpr uint64_t kCompactChunkMin = 1u << 17, kCompactChunkMax = 1u << 20;
+// `copy_stream`: up to four parts of the run, of at most 2^20 rays (84 MB of rows, still in L2 when they are
+// compacted) and at least 327,680.  A copy costs about 2 us besides its bytes (16 B per ray of the single
+// parabolic heliostat at the host link's ~190 GB/s), so the counts follow in one copy at the end.  4M rays
+// of that heliostat: 577 us in one piece, 445 in eight chunks, 436 in four, 444 to 464 with chunks that
+// start at 2^18 or 2^17 and double; the copies alone 349 us.  A part's launches and waits cost about 15 us, and
+// field launches gain least from an early copy.  Times in 1 / 2 / 3 / 4 parts, us, of a hillside of 600, the
+// parabolic heliostat, and a corridor of 1.5 records a ray: 300,000 rays 103 / 120 / 148 / 183, 87 / 91 / 106 / 125,
+// 141 / 129 / 143 / 154; 600,000 154 / 150 / 184 / 205, 123 / 113 / 127 / 142, 230 / 196 / 202 / 208; 2^20 211 / 199 / 217 /
+// 242, 173 / 155 / 165 / 173, 369 / 308 / 294 / 289; 2^21 350 / 306 / 314 / 334, 309 / 259 / 251 / 253, 684 / 570 / 535 / 523
+// (into pageable memory 20 to 40 us more, alike).
+constexpr uint64_t kCompactChunkMin = 327680, kCompactChunkMax = 1u << 20, kCompactParts = 4;
 constexpr int kCompactRing = 2;  // chunks whose records wait on the device for their copy
 
 int System::ensure_compact_buffers(uint64_t n) {
@@ -585,8 +589,9 @@ int System::run_to_host_compact(float* points, uint8_t* counts, float* records, 
         return CSP_OK;
     };
     // in chunks when no number of records can exceed the capacity (else it is known only after the
-    // whole trace, and nothing may be copied before) and the run is longer than the first one
-    const uint64_t chunk = std::min(kCompactChunkMax, std::max(kCompactChunkMin, (n / 4 + 255) / 256 * 256));
+    // whole trace, and nothing may be copied before) and the run has more than one
+    const uint64_t parts = std::max<uint64_t>(1, std::min(kCompactParts, n / kCompactChunkMin));
+    const uint64_t chunk = std::min(kCompactChunkMax, ((n + parts - 1) / parts + 255) / 256 * 256);
     if (n > chunk && capacity / 4 >= n) {
         const uint64_t need = 4 * chunk * kCompactRing;
         if (need > cap_cring) {

@@ -31,3 +31,16 @@ def test_compact_chunks(gpu, n):
             t.run_to_host_compact(points=sentinel, records=np.empty((len(r) - 1, 4), np.float32))
         assert (sentinel == -7.0).all()
     t.close()
+
+
+@pytest.mark.parametrize("n", [655_359, 655_360, 983_039, 983_041, 1_310_720, (1 << 22) + 257])
+def test_compact_parts(gpu, n):
+    """Runs around the sizes at which they get another part, and past four parts of 2^20 rays."""
+    sc = scenes.corridor(slope_error=1e-3)
+    t = native.tracer_for(sc, seed=6, num_rays=n, record_ids=False)
+    points, counts, records = t.run_to_host_compact(records=np.empty((4 * n, 4), np.float32))
+    p, c, r = _dense(t)
+    np.testing.assert_array_equal(points, p)
+    np.testing.assert_array_equal(counts, c)
+    np.testing.assert_array_equal(records, r)
+    t.close()
