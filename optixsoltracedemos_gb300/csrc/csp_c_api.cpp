@@ -134,7 +134,7 @@ void System::release() {
     cudaFree(d_flux);
     if (h_flux) cudaFreeHost(h_flux);
     d_flux = h_flux = nullptr;
-    cap_flux = 0;
+    cap_flux = cap_hflux = 0;
     d_nodes = nullptr;
     d_prims = nullptr;
     d_optics = nullptr;
@@ -664,23 +664,27 @@ int System::flux_map(uint32_t nx, uint32_t ny, uint32_t* counts, double dni, dou
     if (!initialized || !d_hits) return fail(CSP_ERR_STATE, "flux map before initialize()/run()");
     if (nx == 0 || ny == 0 || (uint64_t)nx * ny > (1u << 26)) return fail(CSP_ERR_INVALID_ARGUMENT, "bad flux grid");
     const size_t nb = (size_t)nx * ny;
-    // device: counters and map, zeroed in one go; pinned host memory: the map and the sun frame
+    // device: counters and map, zeroed in one go; host, pinned where there is memory for it: the sun frame
+    // and the map
     constexpr size_t kStats = 4 * sizeof(unsigned long long);
-    const size_t map_bytes = nb * sizeof(uint32_t);
+    const size_t map_bytes = nb * sizeof(uint32_t), host_bytes = sizeof(SunFrame) + map_bytes;
     int rc;
     if (nb > cap_flux) {
         cudaFree(d_flux);
-        if (h_flux) cudaFreeHost(h_flux);
-        d_flux = h_flux = nullptr;
+        d_flux = nullptr;
         cap_flux = 0;
         if ((rc = cuda_status(dev_alloc((void**)&d_flux, kStats + map_bytes), "cudaMalloc flux map"))) return rc;
-        if ((rc = cuda_status(host_alloc((void**)&h_flux, sizeof(SunFrame) + map_bytes), "cudaHostAlloc flux map"))) {
-            cudaFree(d_flux);
-            d_flux = h_flux = nullptr;
-            return rc;
-        }
         cap_flux = nb;
     }
+    if (nb > cap_hflux) {
+        if (h_flux) cudaFreeHost(h_flux);
+        h_flux = nullptr;
+        cap_hflux = 0;
+        if (host_alloc((void**)&h_flux, host_bytes) == cudaSuccess) cap_hflux = nb;
+        else cudaGetLastError();  // a slower copy
+    }
+    std::vector<float4> pageable(nb > cap_hflux ? (host_bytes + sizeof(float4) - 1) / sizeof(float4) : 0);
+    unsigned char* const block = nb > cap_hflux ? reinterpret_cast<unsigned char*>(pageable.data()) : h_flux;
     FluxTarget F;
     flux_target(elements.back(), nx, ny, F);
     F.stats = reinterpret_cast<unsigned long long*>(d_flux);
@@ -689,15 +693,15 @@ int System::flux_map(uint32_t nx, uint32_t ny, uint32_t* counts, double dni, dou
     if ((rc = cuda_status(cudaMemsetAsync(d_flux, 0, kStats + map_bytes, stream), "memset flux"))) return rc;
     if ((rc = cuda_status(launch_flux_records(d_hits, num_rays * kMaxDepth, F, stream), "flux_records_kernel")))
         return rc;
-    if ((rc = cuda_status(cudaMemcpyAsync(h_flux + sizeof(SunFrame), F.counts, map_bytes, cudaMemcpyDeviceToHost, stream),
+    if ((rc = cuda_status(cudaMemcpyAsync(block + sizeof(SunFrame), F.counts, map_bytes, cudaMemcpyDeviceToHost, stream),
                           "D2H flux map")))
         return rc;
-    if ((rc = cuda_status(cudaMemcpyAsync(h_flux, d_sun, sizeof(SunFrame), cudaMemcpyDeviceToHost, stream),
+    if ((rc = cuda_status(cudaMemcpyAsync(block, d_sun, sizeof(SunFrame), cudaMemcpyDeviceToHost, stream),
                           "D2H sun frame")))
         return rc;
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "flux map"))) return rc;
-    const SunFrame& f = *reinterpret_cast<const SunFrame*>(h_flux);
-    const uint32_t* host = reinterpret_cast<const uint32_t*>(h_flux + sizeof(SunFrame));
+    const SunFrame& f = *reinterpret_cast<const SunFrame*>(block);
+    const uint32_t* host = reinterpret_cast<const uint32_t*>(block + sizeof(SunFrame));
     if (counts) std::copy(host, host + nb, counts);
     if (flux)
         counts_to_flux(host, nb, dni, sun_plane_area(f), num_rays, flux_bin_area(elements.back(), nx, ny), flux);

@@ -111,7 +111,7 @@ struct System {
     unsigned long long* h_ctotal = nullptr;
     unsigned char* d_flux = nullptr;  // csp_flux_map: counters [4], then the map
     unsigned char* h_flux = nullptr;  // pinned: the sun frame, then the map
-    size_t cap_flux = 0;
+    size_t cap_flux = 0, cap_hflux = 0;  // bins of the two
     size_t cap_nodes = 0;
     uint64_t cap_rays = 0;
     bool ids_allocated = false;

@@ -47,3 +47,25 @@ def test_batch_record_counters(gpu, oracle32, name, tuning):
         want = [n, (oh[..., 0] == 1.0).sum(), (oh[..., 0] == 2.0).sum(), counts.sum()]
         assert [int(v) for v in b.stats(k)] == [int(v) for v in want]
     b.close()
+
+
+@pytest.mark.parametrize("bins", [100, 700])
+def test_map_without_pinned_memory(gpu, bins):
+    """Where no pinned memory is to be had the map is the same."""
+    sc = scenes.large_field(n_heliostats=50, sun=scenes.sun_vector(45.0, 10.0))
+    maps = []
+    for fail in (False, True):
+        t = native.tracer_for(sc, seed=1, num_rays=200_000)
+        t.run()
+        t.flux_map(2, 2)  # the map on the device and its pinned copy are to grow
+        for k in range(3):
+            if fail:
+                native.debug_fail_allocation(1 if k == 0 else 0)  # the second allocation of the first call
+            try:
+                maps.append(t.flux_map(bins, bins)[0])
+            finally:
+                native.debug_fail_allocation(-1)
+        t.close()
+    assert maps[0].any()
+    for m in maps[1:]:
+        np.testing.assert_array_equal(m, maps[0])
