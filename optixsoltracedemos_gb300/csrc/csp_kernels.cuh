@@ -81,7 +81,7 @@ struct SunGridJob {
     uint2* cells;             // [cap_cells]
     uint32_t* alloc;          // items handed out to cells so far
     float4* rect;             // [n] candidate rectangles
-    float4* reach_rect;       // [n] reach rectangles
+    float4* reach_rect;       // [n] reach rectangles (in the space of item_rect)
     uint32_t* reach;          // [kReachRaster^2 / 32]
     // the state's field grid, when the device builds it (cells null: not)
     const Aabb* prune;        // [n] pruning boxes
@@ -97,16 +97,18 @@ struct SunGridJob {
 };
 
 // Capacities of the sun grid of an n-element scene and the device bytes of its arrays (each array
-// 256-byte aligned, in the order of sungrid_place), descriptor included.
+// 256-byte aligned, in the order of sungrid_place), descriptor included, the raster too or not.
 struct SunGridCaps {
     int cap_cells;
     uint32_t cap_items;
 };
 SunGridCaps sungrid_caps(uint32_t n);
-size_t sungrid_bytes(uint32_t n);
-// Carve the arrays of an n-element scene's sun grid out of `base` (sungrid_bytes(n) bytes, 256-byte
-// aligned); fills every SunGridJob field except sun and aabbs.
-void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job);
+constexpr size_t kReachBytes = kReachRaster * kReachRaster / 8;
+size_t sungrid_bytes(uint32_t n, bool raster = true);
+// Carve the arrays of an n-element scene's sun grid out of `base` (sungrid_bytes(n, !raster) bytes, 256-byte
+// aligned), the reach raster out of `raster` (kReachBytes) if given; fills every SunGridJob field except
+// sun and aabbs.
+void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job, unsigned char* raster = nullptr);
 
 // Build the sun grids (and field grids, where the jobs have them) of n_jobs scene states (jobs: device
 // array) on `stream`; max_n, max_field_cells = the largest element count and field_nx * field_ny

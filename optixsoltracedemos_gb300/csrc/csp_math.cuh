@@ -92,6 +92,11 @@ CSP_HD float4 grid_box(float4 lo, float4 hi) {
     return make_float4(lo.x - m, lo.y - m, hi.x + m, hi.y + m);
 }
 
+// Cell of coordinate x along an axis of n cells of that grid, from x0 on, 1 / inv wide.
+CSP_HD int field_index(float x, float x0, float inv, int n) {
+    return (int)fminf(fmaxf(floorf((x - x0) * inv), 0.0f), (float)(n - 1));
+}
+
 // ------------------------------------------------------------------------------------ Philox ---
 struct u32x4 {
     uint32_t x, y, z, w;

@@ -621,6 +621,17 @@ void plan_grid(const HostScene& s, const GridStats& st, HostGrid& g) {
     g.valid = true;
 }
 
+uint32_t field_items(const HostScene& s, const HostGrid& g) {
+    uint64_t items = 0;
+    for (size_t i = 0; i + 1 < s.prune.size(); ++i) {
+        const float4 b = grid_box(s.prune[i].lo, s.prune[i].hi);
+        const int nx = field_index(b.z, g.x0, g.inv_cell, g.nx) - field_index(b.x, g.x0, g.inv_cell, g.nx) + 1;
+        const int ny = field_index(b.w, g.y0, g.inv_cell, g.ny) - field_index(b.y, g.y0, g.inv_cell, g.ny) + 1;
+        items += (uint64_t)nx * ny;
+    }
+    return (uint32_t)std::min<uint64_t>(items, g.cap_items);
+}
+
 void build_grid(const HostScene& s, HostGrid& g) {
     g = HostGrid{};
     const uint32_t n = (uint32_t)s.prims.size();

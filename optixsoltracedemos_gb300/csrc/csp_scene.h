@@ -100,6 +100,10 @@ void build_grid(const HostScene& s, HostGrid& g);
 // hence the median) -- any ordinary field; others take build_grid.
 void plan_grid(const HostScene& s, const GridStats& stats, HostGrid& g);
 
+// Items of a grid that the device builds for the scene: at most the plan's cap_items, which is a bound
+// from the largest box.
+uint32_t field_items(const HostScene& s, const HostGrid& g);
+
 // Device descriptor of a grid whose arrays live at the given device addresses.
 GridDesc grid_desc(const HostGrid& g, const uint2* cells, const Aabb* items, const Aabb* global);
 

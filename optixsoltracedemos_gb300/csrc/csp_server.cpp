@@ -20,8 +20,9 @@
 // rays are traced with the same (seed, instance, ray index) and its flux map is an integer sum.
 //
 // Device memory: one arena of the configured budget, first-fit blocks per request (element
-// records when the request has its own poses, refitted nodes, sun frame, sun grid, flux map).  A request is
-// admitted when its block fits; requests larger than the whole budget fail.
+// records when the request has its own poses, refitted nodes, sun frame, sun grid, flux map); of fixed
+// size outside it, per active request, the reach raster of the sun grid, job tables and results.  A request
+// is admitted when its block fits; requests larger than the whole budget fail.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -174,6 +175,7 @@ struct Server {
 
     unsigned char* d_arena = nullptr;
     Arena arena;
+    unsigned char* d_reach = nullptr;  // reach rasters of the active requests' sun grids, by result slot
     // per-step device tables and their pinned staging
     unsigned char* d_step[2] = {nullptr, nullptr};
     unsigned char* h_step[2] = {nullptr, nullptr};
@@ -252,6 +254,7 @@ void Server::stop() {
     }
     scenes.clear();
     cudaFree(d_arena);
+    cudaFree(d_reach);
     for (int p = 0; p < 2; ++p) {
         cudaFree(d_step[p]);
         cudaFree(d_counter[p]);
@@ -263,7 +266,7 @@ void Server::stop() {
     d_jobs = nullptr;
     if (h_adm) cudaFreeHost(h_adm);
     if (h_res) cudaFreeHost(h_res);
-    d_arena = nullptr;
+    d_arena = d_reach = nullptr;
     h_adm = h_res = nullptr;
     if (adm_done) cudaEventDestroy(adm_done);
     adm_done = nullptr;
@@ -299,6 +302,8 @@ int Server::start(int dev, size_t budget_bytes, int max_act, uint64_t step_targe
     if (budget > free_b) return set_error(CSP_ERR_OUT_OF_MEMORY, "server memory budget exceeds free device memory");
     if ((rc = cuda_status(dev_alloc((void**)&d_arena, budget), "cudaMalloc server arena"))) return rc;
     arena.reset(budget);
+    if ((rc = cuda_status(dev_alloc((void**)&d_reach, (size_t)max_active * kReachBytes), "cudaMalloc reach rasters")))
+        return rc;
     step_bytes = align256((size_t)max_active * sizeof(InstanceDesc)) * kBatchGroups +
                  align256((size_t)(max_active + 1) * sizeof(uint64_t)) * kBatchGroups;
     for (int p = 0; p < 2; ++p) {
@@ -369,9 +374,9 @@ static BlockLayout block_layout(const SRequest& r, uint32_t nx, uint32_t ny) {
         at = o;
         o += align256(bytes);
     };
-    take(L.grid, sizeof(GridDesc));
+    take(L.grid, sizeof(GridDesc) + 4 * sizeof(unsigned long long));
+    L.stats = L.grid + sizeof(GridDesc);
     take(L.counts, (size_t)nx * ny * sizeof(uint32_t));
-    take(L.stats, 4 * sizeof(unsigned long long));
     if (!r.poses.empty()) {
         take(L.prims, n * sizeof(Prim));
         take(L.optics, n * sizeof(Optics));
@@ -386,7 +391,7 @@ static BlockLayout block_layout(const SRequest& r, uint32_t nx, uint32_t ny) {
     L.upload = o;
     take(L.sun, sizeof(SunFrame));
     if (!r.poses.empty() && r.group != kAccelGrid) take(L.nodes, s.base.nodes.size() * sizeof(Node));
-    if (r.group != kAccelFlat) take(L.sgrid, sungrid_bytes((uint32_t)n));
+    if (r.group != kAccelFlat) take(L.sgrid, sungrid_bytes((uint32_t)n, false));
     if (!r.poses.empty() && r.group == kAccelGrid && r.grid.on_device)
         take(L.field, field_bytes(r.grid.nx, r.grid.ny, r.grid.cap_items));
     L.total = o;
@@ -438,6 +443,17 @@ int Server::submit(SRequest&& request, uint64_t* id) {
     r->group = s.group;
     if (r->group != kAccelFlat && !r->poses.empty()) r->group = r->grid.valid ? kAccelGrid : kAccelBvh;
     r->bytes = request_bytes(*r);
+    // where the budget is short: the grid with room for its exact items, then no grid but the BVH (the
+    // same records, traced slower)
+    if (r->bytes > budget && r->group == kAccelGrid && r->grid.on_device) {
+        r->grid.cap_items = field_items(r->hs, r->grid);
+        r->bytes = request_bytes(*r);
+    }
+    if (r->bytes > budget && r->group == kAccelGrid && !r->poses.empty()) {
+        r->grid = HostGrid{};
+        r->group = kAccelBvh;
+        r->bytes = request_bytes(*r);
+    }
     if (r->bytes > budget) return set_error(CSP_ERR_OUT_OF_MEMORY, "request larger than the server memory budget");
     r->t_submit = Clock::now();
     if (!have_first) {
@@ -590,7 +606,7 @@ int Server::admit(std::vector<SRequest*>& admitted, std::string& err) {
         sj.out = reinterpret_cast<SunFrame*>(d_arena + r.o_sun);
         if (r.group != kAccelFlat) {
             SunGridJob& gj = sgs[n_sg++];
-            sungrid_place(d_arena + r.o_sgrid, n, gj);
+            sungrid_place(d_arena + r.o_sgrid, n, gj, d_reach + (size_t)r.result_slot * kReachBytes);
             gj.sun = sj.out;
             gj.aabbs = d_aabbs;
             if (r.own_records && r.group == kAccelGrid && r.grid.on_device) {

@@ -196,11 +196,10 @@ __device__ __forceinline__ void field_cells_of(const SunGridJob& J, int e, F&& f
     if (!J.field_cells || e + 1 >= J.n) return;
     const Aabb p = J.prune[e];
     const float4 b = grid_box(p.lo, p.hi);
-    auto index = [](float x, float x0, float inv, int n) {
-        return (int)fminf(fmaxf(floorf((x - x0) * inv), 0.0f), (float)(n - 1));
-    };
-    const int ax = index(b.x, J.field_x0, J.field_inv, J.field_nx), bx = index(b.z, J.field_x0, J.field_inv, J.field_nx);
-    const int ay = index(b.y, J.field_y0, J.field_inv, J.field_ny), by = index(b.w, J.field_y0, J.field_inv, J.field_ny);
+    const int ax = field_index(b.x, J.field_x0, J.field_inv, J.field_nx);
+    const int bx = field_index(b.z, J.field_x0, J.field_inv, J.field_nx);
+    const int ay = field_index(b.y, J.field_y0, J.field_inv, J.field_ny);
+    const int by = field_index(b.w, J.field_y0, J.field_inv, J.field_ny);
     for (int y = ay; y <= by; ++y)
         for (int x = ax; x <= bx; ++x) f(J.field_cells + y * J.field_nx + x);
 }
@@ -293,15 +292,14 @@ SunGridCaps sungrid_caps(uint32_t n) {
     return c;
 }
 
-size_t sungrid_bytes(uint32_t n) {
+size_t sungrid_bytes(uint32_t n, bool raster) {
     const SunGridCaps c = sungrid_caps(n);
-    return a256(sizeof(SunGrid)) + a256((size_t)c.cap_cells * sizeof(uint2)) + a256(sizeof(uint32_t)) +
-           2 * a256((size_t)n * sizeof(float4)) + a256(kReachRaster * kReachRaster / 8) +
-           a256((size_t)c.cap_items * sizeof(float4)) + a256((size_t)c.cap_items * sizeof(Aabb)) +
-           a256((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t));
+    return a256(sizeof(SunGrid) + sizeof(uint32_t)) + a256((size_t)c.cap_cells * sizeof(uint2)) +
+           a256((size_t)n * sizeof(float4)) + (raster ? kReachBytes : 0) + a256((size_t)c.cap_items * sizeof(float4)) +
+           a256((size_t)c.cap_items * sizeof(Aabb)) + a256((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t));
 }
 
-void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job) {
+void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job, unsigned char* raster) {
     const SunGridCaps c = sungrid_caps(n);
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -309,13 +307,13 @@ void sungrid_place(unsigned char* base, uint32_t n, SunGridJob& job) {
         o += a256(bytes);
         return p;
     };
-    job.desc = reinterpret_cast<SunGrid*>(take(sizeof(SunGrid)));
+    job.desc = reinterpret_cast<SunGrid*>(take(sizeof(SunGrid) + sizeof(uint32_t)));
+    job.alloc = reinterpret_cast<uint32_t*>(job.desc + 1);
     job.cells = reinterpret_cast<uint2*>(take((size_t)c.cap_cells * sizeof(uint2)));
-    job.alloc = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t)));
     job.rect = reinterpret_cast<float4*>(take((size_t)n * sizeof(float4)));
-    job.reach_rect = reinterpret_cast<float4*>(take((size_t)n * sizeof(float4)));
-    job.reach = reinterpret_cast<uint32_t*>(take(kReachRaster * kReachRaster / 8));
+    job.reach = reinterpret_cast<uint32_t*>(raster ? raster : take(kReachBytes));
     job.item_rect = reinterpret_cast<float4*>(take((size_t)c.cap_items * sizeof(float4)));
+    job.reach_rect = job.item_rect;  // read by the count pass, before the fill pass writes items (n <= cap_items)
     job.item_box = reinterpret_cast<Aabb*>(take((size_t)c.cap_items * sizeof(Aabb)));
     job.global_id = reinterpret_cast<uint32_t*>(take((size_t)std::max<uint32_t>(n, 1) * sizeof(uint32_t)));
     job.prune = nullptr;
