@@ -616,7 +616,12 @@ void plan_grid(const HostScene& s, const GridStats& st, HostGrid& g) {
     // a box of side w touches at most floor(w / cell) + 2 cells along an axis (the hundredth covers the
     // rounding of the cell index)
     const uint32_t k = (uint32_t)(st.max / cell + 0.01) + 2;
-    g.cap_items = st.n * k * k;
+    const uint64_t items = (uint64_t)st.n * k * k;
+    if (items > 0xFFFFFFFFull) {  // item positions are 32-bit: the exact number, which is far smaller
+        build_grid(s, g);
+        return;
+    }
+    g.cap_items = (uint32_t)items;
     g.on_device = true;
     g.valid = true;
 }

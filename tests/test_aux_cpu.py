@@ -103,3 +103,19 @@ def test_host_pool_without_threads(tmp_path):
                     os.path.join(root, "tests", "cpp", "host_pool_check.cpp"), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "OK", r.stdout + r.stderr
+
+
+def test_field_grid_plan_of_very_many_elements(tmp_path):
+    """The item bound of a device-built field grid stays within 32 bits."""
+    import shutil
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    csrc = os.path.join(root, "optixsoltracedemos_gb300", "csrc")
+    cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    exe = str(tmp_path / "plan_grid_check")
+    subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", csrc, "-I",
+                    os.path.join(root, "include"), "-I", cuda_inc,
+                    os.path.join(root, "tests", "cpp", "plan_grid_check.cpp"), os.path.join(csrc, "csp_scene.cpp"),
+                    "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip().endswith("OK"), r.stdout + r.stderr
