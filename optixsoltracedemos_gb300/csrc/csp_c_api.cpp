@@ -336,9 +336,9 @@ int System::ensure_hit_buffers() {
     return CSP_OK;
 }
 
-// The current elements and sun on the device, complete when it returns.  After a failure past
-// build_scene's checks (device memory) the handle traces nothing until a later update() or initialize()
-// gets through; the records and the flux map of its last run stay readable.
+// The current elements and sun on the device, complete when it returns, and room for the records.  After a
+// failure past build_scene's checks (device memory) the handle traces nothing until a later update() or
+// initialize() gets through; the records and the flux map of its last run stay readable.
 int System::load_scene(const char* not_planar, bool first) {
     int rc;
     if ((rc = build_scene(not_planar))) return rc;
@@ -348,10 +348,11 @@ int System::load_scene(const char* not_planar, bool first) {
     if ((rc = build_sungrid())) return rc;
     // the counters are zero before the first launch, and every launch leaves its own so
     if (first && (rc = cuda_status(cudaMemsetAsync(d_counters, 0, kCounterBytes, stream), "memset"))) return rc;
+    const int no_hits = ensure_hit_buffers();  // while the device works; the scene is complete without
     if ((rc = cuda_status(cudaStreamSynchronize(stream), "scene set-up"))) return rc;
     records_busy = false;
     loaded = true;
-    return CSP_OK;
+    return no_hits;
 }
 
 int System::initialize() {
@@ -365,7 +366,6 @@ int System::initialize() {
     topology = false;
     if (!d_sun && (rc = cuda_status(dev_alloc((void**)&d_sun, sizeof(SunFrame)), "cudaMalloc sun"))) return rc;
     if ((rc = load_scene("the scene is not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)", true))) return rc;
-    if ((rc = ensure_hit_buffers())) return rc;
     initialized = true;
     time_setup = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return CSP_OK;
@@ -376,8 +376,7 @@ int System::update() {
     if (!initialized) return fail(CSP_ERR_STATE, "update() before initialize()");
     if (elements.size() != n_scene)
         return fail(CSP_ERR_STATE, "update() needs the element count of initialize(); call initialize() again");
-    const int rc = load_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)", false);
-    return rc ? rc : ensure_hit_buffers();
+    return load_scene("the new poses are not a planar field: no grid (use CSP_ACCEL_AUTO or _BVH)", false);
 }
 
 // Work counter of a launch on `st`.  A launch hands out its tiles by its counter and leaves it zero, so two
