@@ -49,10 +49,7 @@ struct TraceSmem {
 // of the candidate and cell lists of the others.  64M rays over 10,000 heliostats: seven / eight / nine 4905 /
 // 4656 / 4726 us, four of 256 threads (a tile's barriers over twice the warps) 4691; the single
 // parabolic heliostat, 16M rays: four of 256 302 against 287 us, ten of 128 (48 registers, spills) 299, two of 512 322.
-template <int kAccel>
-constexpr int trace_min_blocks() {
-    return 1024 / kTraceBlock;
-}
+constexpr int kTraceBlocksPerSM = 1024 / kTraceBlock;
 
 // Persistent kernel over the tiles of one launch; dense records out.  With a tile counter every CTA
 // starts on a share of its own (half of an even share for element lists, a quarter for fields, whose
@@ -68,7 +65,7 @@ constexpr int trace_min_blocks() {
 constexpr uint32_t kTraceGrab = 8;
 
 template <int kAccel, bool kIds>
-__global__ void __launch_bounds__(kTraceBlock, trace_min_blocks<kAccel>()) trace_kernel(
+__global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM) trace_kernel(
     const typename PlainCfg<kAccel, kIds>::Args A) {
     using C = PlainCfg<kAccel, kIds>;
     extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -736,7 +736,6 @@ GridDesc grid_desc(const HostGrid& g, const uint2* cells, const Aabb* items, con
     d.cells = cells;
     d.items = items;
     d.global = global;
-    d.reserved = nullptr;
     return d;
 }
 

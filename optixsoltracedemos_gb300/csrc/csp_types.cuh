@@ -91,7 +91,6 @@ struct alignas(16) GridDesc {
     const uint2* cells;
     const Aabb* items;
     const Aabb* global;
-    const void* reserved;
 };
 
 // Candidate grid of the sun rays of one scene state and sun frame (scenes of more than 8
