@@ -70,10 +70,10 @@ NCU_TRAFFIC_PER_LAUNCH_FIELD = 64 * (38493696 + 304543232)
 # Batch kernel (field grid) on the batched workload: warp instructions and DRAM bytes per traced ray,
 # from `ncu -k regex:^batch_kernel -s 2 -c 1` of `python bench.py --workload batched
 # --instances 8 --tuning 256,4,256 --steps 1 --warmup 3 --no-systems --no-cpu-baseline
-# --plain-instances 1` (one launch over 42,028,566 rays): smsp__inst_executed.sum = 2,694,909,092
-# and dram__bytes_read.sum + dram__bytes_write.sum = 53,576,448 + 1,150,208 bytes, per ray.
-BATCH_WARP_INST_PER_RAY = 2694909092 / 42028566
-BATCH_DRAM_BYTES_PER_RAY = (53576448 + 1150208) / 42028566
+# --plain-instances 1` (one launch over 42,028,566 rays): smsp__inst_executed.sum = 2,632,170,872
+# and dram__bytes_read.sum + dram__bytes_write.sum = 54,744,576 + 1,460,992 bytes, per ray.
+BATCH_WARP_INST_PER_RAY = 2632170872 / 42028566
+BATCH_DRAM_BYTES_PER_RAY = (54744576 + 1460992) / 42028566
 ISSUE_PER_SM_PER_CYCLE = 4  # one warp instruction per cycle per scheduler, 4 schedulers per SM
 
 

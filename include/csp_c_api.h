@@ -147,8 +147,10 @@ CSP_API int csp_run(csp_handle h);
  * It writes the handle's hit buffer, so it must not overlap another run of the handle, nor a copy of
  * its records or its flux map, on the GPU; windows of csp_trace_into may be traced meanwhile. */
 CSP_API int csp_trace_async(csp_handle h, void* stream);
-/* Re-read the element poses given since initialize (same count), refit the acceleration structure
- * in place and recompute the sun plane (update()). */
+/* Re-read the element poses given since initialize (same count), rebuild or refit what finds the
+ * closest hit (the field grid of a planar field, else the BVH) and recompute the sun plane (update()).
+ * Poses that are refused (CSP_ERR_BAD_SCENE) leave the scene of the last set-up as it was, and so does
+ * a refused csp_initialize; after CSP_ERR_OUT_OF_MEMORY another csp_update may complete it. */
 CSP_API int csp_update(csp_handle h);
 
 /* Copy hit records of rays [first_ray, first_ray + count) to host memory: dst holds count * 5 * 4
@@ -248,7 +250,8 @@ CSP_API int csp_flux_target(const csp_element* receiver, uint32_t nx, uint32_t n
  * A batch holds scenes (element lists; a scene's BVH topology is built once) and instances (a
  * scene with optional per-instance element poses -- same count and surfaces, new origins, aim
  * points or rotations -- a sun vector and shape, a ray count, a seed and a Philox instance id).
- * csp_batch_run uploads the instances, refits each instance's BVH on the device, computes every
+ * csp_batch_run uploads the instances, builds each instance's field grid (or refits its BVH, where it
+ * is not a planar field) on the device, computes every
  * instance's sun plane and traces all instances in one persistent launch per scene class
  * (<= 8 elements / larger), binning receiver records into per-instance flux maps on the fly; no
  * per-ray records are kept.  The device work of a run is one CUDA graph, re-launched while the
@@ -307,7 +310,7 @@ CSP_API int csp_batch_get_transfer(csp_batch b, uint64_t* h2d_bytes, uint64_t* d
  * bytes (0 = half the free device memory, at most 8 GiB).  Scenes are added once and stay resident
  * (element records, BVH topology, field grid).  csp_server_submit (any thread, non-blocking)
  * queues a trace request: a scene, optional per-request poses (same count and surfaces: heliostat
- * tracking, refitted in place on the device), a sun, a ray count, seed and Philox instance id.
+ * tracking; its field grid built, or its BVH refitted, on the device), a sun, a ray count, seed and Philox instance id.
  * The worker admits requests as slots (max_active) and arena memory free up and traces every active
  * request's next slice of rays (step_rays across all active requests per step, 0 = 64M, but at
  * least 2^24 rays per request, or its remaining rays) in one persistent launch per kernel group,

@@ -186,7 +186,7 @@ cudaError_t launch_trace_t(const TraceArgs& args, cudaStream_t stream) {
     }
     const uint64_t slots = args.ids ? both >> 32 : (uint32_t)both;
     const uint64_t tiles = (args.count + kTraceBlock - 1) / kTraceBlock;  // CTAs that have work
-    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // 44 TB of records
+    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // 22 TB of records
     const unsigned grid = (unsigned)std::min(tiles, slots);
     return args.ids ? launch_trace_ids<kAccel, true>(args, grid, stream)
                     : launch_trace_ids<kAccel, false>(args, grid, stream);

@@ -64,7 +64,8 @@ struct TraceArgsK : TraceArgs {
 const float* halton3_table();
 
 // Sun-plane distance and parallelogram (lib/geometry_manager.cpp:97-148 with the reductions of
-// lib/sun_utils.cu:53-179) plus the per-launch cone frame (cuda/sun.cu:76-79), one block.
+// lib/sun_utils.cu:53-179) plus the per-launch cone frame (cuda/sun.cu:76-79): one block, a cluster of
+// eight from 1,024 elements.
 cudaError_t launch_prepare_sun(const Aabb* aabbs, int n, float sx, float sy, float sz, float tan_pad, int shape,
                                float param, SunFrame* out, cudaStream_t stream);
 

@@ -40,7 +40,8 @@ constexpr size_t kOffAabbs = kOffOptics + kNoAllocMaxElements * sizeof(Optics);
 constexpr size_t kOffSun = kOffAabbs + kNoAllocMaxElements * sizeof(Aabb);
 constexpr size_t kNoAllocScratchBytes = 4096;
 static_assert(kOffSun + sizeof(SunFrame) <= kNoAllocScratchBytes, "scratch layout exceeds the array");
-static_assert(kOffSun % 16 == 0, "records must stay 16-byte aligned");
+static_assert(kOffNodes % 32 == 0 && kOffPrims % 32 == 0 && kOffAabbs % 32 == 0, "Node, Prim and Aabb are 32-byte aligned");
+static_assert(kOffOptics % 16 == 0 && kOffSun % 16 == 0, "Optics and SunFrame are 16-byte aligned");
 
 // The only intermediate storage of csp_trace_noalloc (see the file comment).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];

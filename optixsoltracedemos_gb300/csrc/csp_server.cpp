@@ -49,6 +49,11 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// Elements from which a submission's records are packed on the server's threads.  One submission alone gains
+// from fewer on (1,000 elements 121 us on the caller's thread, 89 with the pool; 4,000 457 and 229), but the
+// callers take turns on the pool, and without it they pack side by side.
+constexpr uint32_t kPoolElements = 4096;
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct SScene {
@@ -421,7 +426,7 @@ int Server::submit(SRequest&& request, uint64_t* id) {
         std::string err;
         const uint32_t n = (uint32_t)r->poses.size();
         GridStats stats;
-        const int rc = n >= 4096 ? build_elements(
+        const int rc = n >= kPoolElements ? build_elements(
                                        r->poses.data(), n, r->hs, err,
                                        [this](size_t tasks, const std::function<void(size_t)>& body) {
                                            pool.run(tasks, body);

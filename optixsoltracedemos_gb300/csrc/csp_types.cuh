@@ -3,7 +3,8 @@
 // Layout in HBM (records and boxes 32-byte aligned, read through the read-only path):
 //   Prim   [n]      64 B  geometry of one element in the form its intersection test consumes
 //   Optics [n]      16 B  reflectivity, slope error, specularity error (extension)
-//   Aabb   [n]      32 B  element AABB exactly as the reference hands it to OptiX (float)
+//   Aabb   [n]      32 B  element AABB exactly as the reference hands it to OptiX (float), and its element and
+//                         type in lo.w
 //   Node   [m]      32 B  stackless BVH node: box + hit link + miss link
 //   SunFrame        sun-plane parallelogram and cone frame, written on device by the prepare kernel
 //   hits   [N*5]    80 B/ray  float4 {stage, x, y, z}, the reference's hit_point_buffer
@@ -47,8 +48,8 @@ struct alignas(16) Optics {
 };
 
 struct alignas(32) Aabb {
-    float4 lo;  // xyz, w unused
-    float4 hi;
+    float4 lo;  // xyz; w of an element's exact box: element | type << kTypeShift (bits)
+    float4 hi;  // xyz, w unused
 };
 
 // Stackless BVH node.  lo.w / hi.w carry int32 links (bit patterns):
