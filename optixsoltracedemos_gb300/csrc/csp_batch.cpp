@@ -779,7 +779,13 @@ int Batch::run_async() {
             pool.start(std::min({63u, std::max(2u, std::thread::hardware_concurrency()) - 1, (unsigned)n - 1}));
         std::vector<int> irc(n, CSP_OK);
         std::vector<std::string> ierr(n);
-        auto one = [&](size_t i) { irc[i] = fn(i, ierr[i]); };
+        auto one = [&](size_t i) {
+            try {
+                irc[i] = fn(i, ierr[i]);
+            } catch (const std::bad_alloc&) {  // on one of the pool's threads it would end the process
+                irc[i] = CSP_ERR_OUT_OF_MEMORY;
+            }
+        };
         if (pooled) pool.run(n, one);
         else
             for (size_t i = 0; i < n; ++i) one(i);
